@@ -9,15 +9,34 @@ namespace granite_b200 {
 using AdvanceFn = void (*)(const KParams);
 
 // The feature set (FT_* in granite_kernels.cuh) a launch with parameters P may use: a lean
-// variant when every option it leaves out is off in P (window-pair layouts only), else generic.
+// variant when every option it leaves out is off in P, else generic.
 // defer: the caller runs deferred_extras_kernel after every launch, which ends at each record.
-inline int kernel_features(const KParams &P, bool pair, bool defer = false) {
-    if (!pair || P.uplift_mode != 0 || P.abort_mode != 0 || P.topography || P.sphere || P.border_mode != 0 ||
-        P.alive_at != nullptr || P.filter_weights || (P.curvature_mode != 0 && P.curvature_mode != 1))
+inline int kernel_features(const KParams &P, bool defer = false) {
+    if (P.uplift_mode != 0 || P.abort_mode != 0 || P.topography || P.alive_at != nullptr || !P.wind_dynamic ||
+        (P.curvature_mode != 0 && P.curvature_mode != 1))
         return FT_GENERIC;
     const bool extras = (P.volume_mode != 0 && P.nvol > 0) || P.nexpr > 0;
+    if (P.sphere || P.border_mode != 0 || P.filter_weights || P.wide)
+        return extras || P.compensated || P.curvature_mode != 0 ? FT_GENERIC : (FT_LEAN | FT_BORDER);
     if (P.compensated) return extras ? FT_GENERIC : (FT_LEAN | FT_COMP | (P.curvature_mode == 1 ? FT_CURV : 0));
     return FT_LEAN | (P.curvature_mode == 1 ? FT_CURV : 0) | (extras ? (defer ? FT_DEFER : FT_EXTRAS) : 0);
+}
+
+// Where samples of a grid are clamped to (KParams::flo, fn): every corner of the cell beyond is
+// outside the grid.  Window pairs carry one border node below and two above, so their cells are
+// clamped to [-1, n]; 3D ring slots read as such to [-2, n + 1].  Both give the border's zeros; they
+// differ where a sample lies a cell outside beside an edge node that is not finite, which [-1, n]
+// multiplies by a weight of zero.
+inline void clamp_cells(KParams &P, bool as_pair) {
+    const bool one = as_pair || P.dim == 2;
+    P.flo = one ? -1.f : -2.f;
+    const int32_t n[3] = {P.nx, P.ny, P.nz};
+    for (int d = 0; d < 3; ++d) P.fn[d] = one ? (float)n[d] : (float)(n[d] + 1);
+}
+
+// Grids that the fast cell arithmetic does not cover (pcell1 needs coordinates below 2^22).
+inline bool wide_grid(int64_t nx, int64_t ny, int64_t nz) {
+    return nx >= (1 << 22) - 2 || ny >= (1 << 22) - 2 || nz >= (1 << 22) - 2;
 }
 
 // Step kernel for a dimension, integrator, wind layout (pair = window-pair buffer) and feature

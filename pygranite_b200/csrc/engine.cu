@@ -1172,7 +1172,7 @@ int run_prepare(gr_engine *e, RunPlan &R, bool graph) {
 
     // window-pair layout: one load per corner returns both snapshots; launches never cross a
     // window boundary then
-    e->use_pair = e->wind_dynamic && s.layout == 0;
+    e->use_pair = e->wind_dynamic && s.layout == 0 && !wide_grid(e->nx, e->ny, e->nz);
     {
         const int rc = settle_pairs(e);
         if (rc) return rc;
@@ -1208,11 +1208,13 @@ KParams make_params(gr_engine *e) {
     for (int d = 0; d < 3; ++d) {
         P.inv_scale[d] = e->inv_scale[d];
         P.off[d] = e->off[d];
+        P.noff[d] = -e->off[d];
         P.dom[d] = e->dom[d];
         P.scale[d] = e->scale[d];
     }
     P.nx = (int32_t)e->nx; P.ny = (int32_t)e->ny; P.nz = (int32_t)e->nz; P.dim = e->dim;
-    P.fn[0] = (float)e->nx; P.fn[1] = (float)e->ny; P.fn[2] = (float)e->nz;
+    P.wide = wide_grid(e->nx, e->ny, e->nz);
+    clamp_cells(P, e->use_pair);
     P.pnx = (int32_t)(e->nx + 3); P.pnxy = (int32_t)((e->nx + 3) * (e->ny + 3));
     P.wind = e->wind.p; P.wind_stride = e->wind_stride;
     P.vol = e->vol.p; P.vol_plane = e->nodes;
@@ -1333,7 +1335,7 @@ using KernelFn = void (*)(const KParams);
 KernelFn pick_kernel(const gr_engine *e, const KParams &P, bool defer) {
     const bool rk4 = e->s.integrator == 1;
     const int st = e->s.storage;
-    const int ft = kernel_features(P, e->use_pair, defer);
+    const int ft = kernel_features(P, defer);
     return st == GR_STORE_BF16 ? advance_bf16(e->dim, rk4, e->use_pair, ft)
          : st == GR_STORE_F16 ? advance_f16(e->dim, rk4, e->use_pair, ft) : advance_f32(e->dim, rk4, e->use_pair, ft);
 }
@@ -1453,7 +1455,7 @@ int make_ctx(gr_engine *e, RunPlan &R, RunCtx &r) {
     r.P = make_params(e);
     // deferred volume / expression values: not in graph runs (fixed launch shapes) and only
     // where a lean variant applies
-    r.defer = !R.graph && r.P.vlast != nullptr && (kernel_features(r.P, e->use_pair, true) & FT_DEFER) != 0;
+    r.defer = !R.graph && r.P.vlast != nullptr && (kernel_features(r.P, true) & FT_DEFER) != 0;
     // resolved per run (a cache lookup after the first compile): expressions and settings may
     // change between runs
     e->jit_extras = nullptr;

@@ -52,7 +52,9 @@ constexpr int GR_MAX_CON = 4;
 // values to deferred_extras_kernel after the launch: the step kernel only stores each moved step's
 // stage-averaged velocity and step index, and hands them to the record at a save step.  The lean
 // variants drop the dead state from registers; their arithmetic is the generic variant's.
-constexpr int FT_GENERIC = 0, FT_LEAN = 1, FT_CURV = 2, FT_EXTRAS = 4, FT_COMP = 8, FT_DEFER = 16;
+// FT_BORDER (with FT_LEAN alone) keeps the loop borders, sphere coordinates, 1/256 filter weights and
+// wide grids as runtime options: positions on a sphere or in a periodic domain.
+constexpr int FT_GENERIC = 0, FT_LEAN = 1, FT_CURV = 2, FT_EXTRAS = 4, FT_COMP = 8, FT_DEFER = 16, FT_BORDER = 32;
 
 // Step-schedule flags.
 constexpr int SF_SAVE = 1;       // position / info record after this step
@@ -71,7 +73,9 @@ struct KParams {
     // geometry (TrajectoryIntegrator.tpp:521-574)
     float inv_scale[3], off[3], dom[3], scale[3];
     int32_t nx, ny, nz, dim;
-    float fn[3];                  // nx, ny, nz as floats (the upper clamp of the window pair's cells)
+    float fn[3], flo;             // clamp of a sample's grid coordinates: [flo, fn] (clamp_cells)
+    int32_t wide;                 // 1: a grid too large for pcell1 or the cell index (ring layouts only)
+    float noff[3];                // -off: world position -> grid is (p + noff) * inv_scale
     // ring buffers: slot s of quantity q starts at base + s * stride
     const void *wind;
     int64_t wind_stride;          // bytes per slot
@@ -133,6 +137,15 @@ struct KParams {
 
 __device__ __forceinline__ float lerp_(float a, float b, float t) { return __fmaf_rn(t, b - a, a); }
 
+// Paired float32 operations (one instruction for two values); each half rounds like the scalar
+// operation.  a - b is formed as fma(b, -1, a): the product is exact, so it rounds like the
+// subtraction.
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
 // Texture coordinate -> cell index and fraction.  Coordinates are clamped to [-2, n+1]
 // first; every corner outside the grid is border (3D) or clamped (2D), so the clamp never
 // changes a value and keeps the integer conversion in range.
@@ -146,73 +159,56 @@ __device__ __forceinline__ void cell(float a, int n, int fw, int &i, float &f) {
     if (fw) f = floorf(f * 256.0f + 0.5f) * (1.0f / 256.0f);
 }
 
-template <typename W> struct Store;
+template <typename H> __device__ __forceinline__ float2 cvt16(unsigned q) {
+    if constexpr (std::is_same<H, __half>::value)
+        return __half22float2(*reinterpret_cast<const __half2 *>(&q));
+    else
+        return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&q));
+}
+
+// Ring nodes, (u, v) and w of one snapshot: 16-bit types, and float32 below.
+template <typename H> struct Store {
+    static __device__ __forceinline__ void load3(const void *node, float2 &uv, float &w) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(node));
+        uv = cvt16<H>(q.x); w = cvt16<H>(q.y).x;
+    }
+    static __device__ __forceinline__ float2 load2(const void *node) { return cvt16<H>(__ldg(reinterpret_cast<const unsigned *>(node))); }
+    static constexpr int bytes3 = 8, bytes2 = 4;
+};
 
 template <> struct Store<float> {
     // 3D node {u, v, w, 0}
-    static __device__ __forceinline__ void load3(const void *base, int32_t idx, float &u, float &v, float &w) {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(base) + idx);
-        u = q.x; v = q.y; w = q.z;
+    static __device__ __forceinline__ void load3(const void *node, float2 &uv, float &w) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(node));
+        uv = make_float2(q.x, q.y); w = q.z;
     }
-    static __device__ __forceinline__ void load2(const void *base, int32_t idx, float &u, float &v) {
-        const float2 q = __ldg(reinterpret_cast<const float2 *>(base) + idx);
-        u = q.x; v = q.y;
-    }
+    static __device__ __forceinline__ float2 load2(const void *node) { return __ldg(reinterpret_cast<const float2 *>(node)); }
     static constexpr int bytes3 = 16, bytes2 = 8;
 };
 
-template <> struct Store<__nv_bfloat16> {
-    static __device__ __forceinline__ void load3(const void *base, int32_t idx, float &u, float &v, float &w) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(base) + idx);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&q.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&q.y));
-        u = a.x; v = a.y; w = b.x;
-    }
-    static __device__ __forceinline__ void load2(const void *base, int32_t idx, float &u, float &v) {
-        const unsigned q = __ldg(reinterpret_cast<const unsigned *>(base) + idx);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&q));
-        u = a.x; v = a.y;
-    }
-    static constexpr int bytes3 = 8, bytes2 = 4;
-};
-
-template <> struct Store<__half> {
-    static __device__ __forceinline__ void load3(const void *base, int32_t idx, float &u, float &v, float &w) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(base) + idx);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&q.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&q.y));
-        u = a.x; v = a.y; w = b.x;
-    }
-    static __device__ __forceinline__ void load2(const void *base, int32_t idx, float &u, float &v) {
-        const unsigned q = __ldg(reinterpret_cast<const unsigned *>(base) + idx);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&q));
-        u = a.x; v = a.y;
-    }
-    static constexpr int bytes3 = 8, bytes2 = 4;
-};
-
-// Window-pair layouts: node n holds, component by component, the back snapshot's value followed
-// by the front snapshot's: {u_b, u_f, v_b, v_f, w_b, w_f, 0, 0} in 3D (32 bytes float32, 16 bytes
-// 16-bit), {u_b, u_f, v_b, v_f} in 2D (16 / 8 bytes).  One load returns both snapshots, and each
-// component arrives as a (back, front) pair that the paired float32 instructions of sm_100
-// (__ffma2_rn) interpolate in space at once.  Built per window from the ring (pack_kernels.cuh),
-// with a border (make_pcell, bil2p_padded).
+// Window-pair layouts: node n holds the back snapshot's (u, v), the front snapshot's (u, v) and
+// the two w: {u_b, v_b, u_f, v_f, w_b, w_f, 0, 0} in 3D (32 bytes float32, 16 bytes 16-bit),
+// {u_b, v_b, u_f, v_f} in 2D (16 / 8 bytes).  One load returns both snapshots, as the operand pairs
+// of sm_100's paired float32 instructions (__ffma2_rn): (u, v) of a snapshot is interpolated in space
+// at once and (w_b, w_f) likewise, and the horizontal wind leaves the sample as a pair, so the time
+// interpolation, the stage positions, the coordinates and the curvature differences are paired
+// operations on (x, y) too.  Built per window from the ring (pack_kernels.cuh), with a border
+// (make_pcell, bil2p_padded).
 template <typename W> struct Pair {};
 
 template <typename W> struct IsPair { static constexpr bool value = false; };
 template <typename W> struct IsPair<Pair<W>> { static constexpr bool value = true; };
 
 template <> struct Store<Pair<float>> {
-    // 3D node: (u_b, u_f), (v_b, v_f), (w_b, w_f), one 256-bit load
-    static __device__ __forceinline__ void load3p(const void *base, int32_t idx, float2 (&c)[3]) {
+    // 3D node: (u_b, v_b), (u_f, v_f), (w_b, w_f), one 256-bit load
+    static __device__ __forceinline__ void load3p(const void *node, float2 (&c)[3]) {
         float r[8];
-        const float *p = reinterpret_cast<const float *>(base) + (int64_t)idx * 8;
         asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
-                     : "l"(p));
+                     : "l"(node));
         c[0] = make_float2(r[0], r[1]); c[1] = make_float2(r[2], r[3]); c[2] = make_float2(r[4], r[5]);
     }
-    // 2D node: (u_b, u_f), (v_b, v_f)
+    // 2D node: (u_b, v_b), (u_f, v_f)
     static __device__ __forceinline__ void load2p(const void *base, int32_t idx, float2 (&c)[2]) {
         const float4 q = __ldg(reinterpret_cast<const float4 *>(base) + idx);
         c[0] = make_float2(q.x, q.y); c[1] = make_float2(q.z, q.w);
@@ -221,16 +217,13 @@ template <> struct Store<Pair<float>> {
 };
 
 template <typename H> struct Store<Pair<H>> {
-    // one 32-bit word = (back, front) of one component, converted to a float pair
-    static __device__ __forceinline__ float2 cvt(unsigned q) {
-        if constexpr (sizeof(H) == 2 && std::is_same<H, __half>::value)
-            return __half22float2(*reinterpret_cast<const __half2 *>(&q));
-        else
-            return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&q));
+    static __device__ __forceinline__ void load3p(const void *node, float2 (&c)[3]) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(node));
+        c[0] = cvt16<H>(q.x); c[1] = cvt16<H>(q.y); c[2] = cvt16<H>(q.z);
     }
     static __device__ __forceinline__ void load2p(const void *base, int32_t idx, float2 (&c)[2]) {
         const uint2 q = __ldg(reinterpret_cast<const uint2 *>(base) + idx);
-        c[0] = cvt(q.x); c[1] = cvt(q.y);
+        c[0] = cvt16<H>(q.x); c[1] = cvt16<H>(q.y);
     }
     static constexpr int bytes3 = 16, bytes2 = 8;
 };
@@ -265,44 +258,28 @@ __device__ __forceinline__ Cell3 make_cell3(const KParams &P, float ax, float ay
     return c;
 }
 
-// Trilinear interpolation of the three wind components of one snapshot (border = 0).
-template <typename W>
-__device__ __forceinline__ void tri3(const void *slot, const Cell3 &c, float &ou, float &ov, float &ow) {
-    float u[8], v[8], w[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
-        const int32_t idx = c.base + (dx ? c.sx : 0) + (dy ? c.sy : 0) + (dz ? c.sz : 0);
-        u[k] = 0.f; v[k] = 0.f; w[k] = 0.f;
-        if (c.valid & (1u << k)) Store<W>::load3(slot, idx, u[k], v[k], w[k]);
-    }
-    float a00 = lerp_(u[0], u[1], c.fx), a10 = lerp_(u[2], u[3], c.fx);
-    float a01 = lerp_(u[4], u[5], c.fx), a11 = lerp_(u[6], u[7], c.fx);
-    ou = lerp_(lerp_(a00, a10, c.fy), lerp_(a01, a11, c.fy), c.fz);
-    a00 = lerp_(v[0], v[1], c.fx); a10 = lerp_(v[2], v[3], c.fx);
-    a01 = lerp_(v[4], v[5], c.fx); a11 = lerp_(v[6], v[7], c.fx);
-    ov = lerp_(lerp_(a00, a10, c.fy), lerp_(a01, a11, c.fy), c.fz);
-    a00 = lerp_(w[0], w[1], c.fx); a10 = lerp_(w[2], w[3], c.fx);
-    a01 = lerp_(w[4], w[5], c.fx); a11 = lerp_(w[6], w[7], c.fx);
-    ow = lerp_(lerp_(a00, a10, c.fy), lerp_(a01, a11, c.fy), c.fz);
-}
-
-// Pair nodes of the last cell a particle sampled (window-pair layouts).  Consecutive samples of
-// one particle (its RK4 stages, its next step) mostly fall in the same cell, whose nodes then
-// need no new gathers; the values and the arithmetic are the same either way.  The cell is
-// identified by its first corner's index in the padded pair buffer (`base`); 3D keeps 24 (back,
-// front) float pairs (48 registers; 16-bit nodes converted when loaded; AdvBounds gives the
-// launch shape), 2D 8 pairs (16 registers).
+// Nodes of the last cell a particle sampled.  Consecutive samples of one particle (its RK4 stages,
+// its next step) mostly fall in the same cell, whose nodes then need no new gathers; the values and
+// the arithmetic are the same either way.  The cell is identified by its first corner's index in a
+// padded grid (`base`, the node index of the pair buffer); 3D keeps 24 float
+// pairs (48 registers; 16-bit nodes converted when loaded; AdvBounds gives the launch shape), 2D 8
+// pairs (16 registers).
 // Corner k + 1 of each x pair (k even) is kept as its difference from corner k, formed once when
 // the cell is loaded: the x lerps of every later sample are then one paired FMA each, with the
 // difference lerp2_ would form (same instruction, same rounding).
 struct SampleCache {
     int32_t base;
-    float2 c2d[2][4];  // 2D: (back, front) of u and v at corners 0, 2 and differences 1 - 0, 3 - 2
-    float2 c2[3][8];   // 3D: (back, front) of u, v, w at even corners, differences at odd ones
-    __device__ __forceinline__ void reset() { base = -1; }
+    float2 c2d[2][4];  // 2D: (u, v) of the back and of the front snapshot at corners 0, 2; differences 1 - 0, 3 - 2
+    float2 c2[3][8];   // 3D: (u, v) back, (u, v) front, (w_b, w_f) at even corners, differences at odd ones
+    __device__ __forceinline__ void reset() { base = (int32_t)0x80000000; }   // no cell's index
 };
 
+// 2D window pair with replicated edges: padded node (x, y), x in [-1, nx + 1] and y in
+// [-1, ny + 1], of a (nx + 3) x (ny + 3) buffer holds node (clamp(x), clamp(y)), so a coordinate
+// clamped to [-1, n] reads the clamp-addressed corners of make_cell2 without index clamps.  Same
+// values: inside [-1, n] cell, fraction and corners are unchanged; outside it both corners of the
+// axis are the same edge node, interpolated with any fraction to that node's value exactly.
+//
 // 3D window pair with a zero border (one node below, two above the grid on every axis): the
 // coordinate is clamped to [-1, n], so every corner of the footprint is a node of the padded
 // buffer and needs no validity test, and the footprint's first corner alone identifies the cell.
@@ -318,98 +295,194 @@ inline int64_t padded_pair_nodes(int dim, int64_t nx, int64_t ny, int64_t nz) {
 #endif
 
 struct PCell {
-    int32_t base;        // padded node index of corner (ix, iy, iz)
+    int32_t base;            // padded node index of corner (ix, iy, iz)
+    uint32_t bx, by, bz;     // PCELL_BITS + cell
     float fx, fy, fz;
 };
 
-// Cell of a padded-axis coordinate without the conversion unit.  a is clamped to [-1, n]
-// (n < 2^22); a + 1.5 * 2^23 rounded toward -infinity lies in [2^23, 2^24), where the floats
+// Cell of a coordinate without the conversion unit.  a is clamped to [lo, n] (n < 2^22, lo >= -2); a + 1.5 * 2^23 rounded toward -infinity lies in [2^23, 2^24), where the floats
 // are the integers, so it is floor(a) + 1.5 * 2^23 exactly and its bit pattern is
 // PCELL_BITS + floor(a).  The fraction a + (1.5 * 2^23 - t) equals a - floorf(a) bit for bit,
 // the sign of a zero fraction included (an exact integer is subtracted either way).
 constexpr uint32_t PCELL_BITS = 0x4B400000u;   // bit pattern of 1.5 * 2^23
-__device__ __forceinline__ uint32_t pcell1(float a, float n, int fw, float &f) {
-    a = fminf(fmaxf(a, -1.0f), n);
+__device__ __forceinline__ float frac256(float f) { return floorf(f * 256.0f + 0.5f) * (1.0f / 256.0f); }
+
+__device__ __forceinline__ uint32_t pcell1(float a, float lo, float n, int fw, float &f) {
+    a = fminf(fmaxf(a, lo), n);
     const float t = __fadd_rd(a, 12582912.0f);
     f = a + (12582912.0f - t);
-    if (fw) f = floorf(f * 256.0f + 0.5f) * (1.0f / 256.0f);
+    if (fw) f = frac256(f);
     return __float_as_uint(t);   // PCELL_BITS + floor(a)
 }
 
-// fw: the launch's filter_weights (0 where the variant has it off at compile time).  The
-// index (iz + 1) pnxy + (iy + 1) pnx + (ix + 1) is formed from the bit patterns of pcell1 in
-// wrapping 32-bit arithmetic, with the patterns' offset removed by one loop-invariant term.
-__device__ __forceinline__ PCell make_pcell(const KParams &P, float ax, float ay, float az, int fw) {
+// pcell1 of x and y at once (one paired operation for each of its additions).
+__device__ __forceinline__ void pcell2(float2 a, float lo, float nx, float ny, int fw, uint32_t &bx, uint32_t &by, float2 &f) {
+    a.x = fminf(fmaxf(a.x, lo), nx);
+    a.y = fminf(fmaxf(a.y, lo), ny);
+    const float2 t = __fadd2_rd(a, both(12582912.0f));
+    f = add2(a, sub2(both(12582912.0f), t));
+    if (fw) f = make_float2(frac256(f.x), frac256(f.y));
+    bx = __float_as_uint(t.x);
+    by = __float_as_uint(t.y);
+}
+
+// The same by the conversion unit, for grids of 2^22 nodes and more along an axis.
+__device__ __forceinline__ uint32_t pcell1_wide(float a, float lo, float n, int fw, float &f) {
+    a = fminf(fmaxf(a, lo), n);
+    const float fl = floorf(a);
+    f = a - fl;
+    if (fw) f = frac256(f);
+    return PCELL_BITS + (uint32_t)(int)fl;
+}
+
+// Cell of a sample at grid coordinates (axy, az).  fw: the launch's filter_weights (0 where the
+// variant has it off at compile time).  The index (iz + 1) pnxy + (iy + 1) pnx + (ix + 1) is formed
+// from the bit patterns of pcell1 in wrapping 32-bit arithmetic, with the patterns' offset removed
+// by one loop-invariant term.
+template <int DIM>
+__device__ __forceinline__ PCell make_pcell(const KParams &P, float2 axy, float az, int fw, float lo, int wide) {
     PCell c;
-    const uint32_t bx = pcell1(ax, P.fn[0], fw, c.fx);
-    const uint32_t by = pcell1(ay, P.fn[1], fw, c.fy);
-    const uint32_t bz = pcell1(az, P.fn[2], fw, c.fz);
-    const uint32_t sy = (uint32_t)P.pnx, sz = (uint32_t)P.pnxy;
-    c.base = (int32_t)(bz * sz + by * sy + bx - (PCELL_BITS - 1u) * (sz + sy + 1u));
+    float2 f;
+    c.bz = 0;
+    c.fz = 0.f;
+    if (wide) {
+        c.bx = pcell1_wide(axy.x, lo, P.fn[0], fw, f.x);
+        c.by = pcell1_wide(axy.y, lo, P.fn[1], fw, f.y);
+        if (DIM == 3) c.bz = pcell1_wide(az, lo, P.fn[2], fw, c.fz);
+    } else {
+        pcell2(axy, lo, P.fn[0], P.fn[1], fw, c.bx, c.by, f);
+        if (DIM == 3) c.bz = pcell1(az, lo, P.fn[2], fw, c.fz);
+    }
+    c.fx = f.x;
+    c.fy = f.y;
+    const uint32_t sy = (uint32_t)P.pnx, sz = DIM == 3 ? (uint32_t)P.pnxy : 0u;
+    c.base = (int32_t)(c.bz * sz + c.by * sy + c.bx - (PCELL_BITS - 1u) * (sz + sy + 1u));
     return c;
 }
 
-// lerp_ on a (back, front) pair with one weight, as paired float32 instructions: b - a is formed
-// as fma(a, -1, b) (the product is exact, so it rounds like the subtraction), then fma(t, d, a);
-// each half equals lerp_ on that half bit for bit.
-__device__ __forceinline__ float2 lerp2_(float2 a, float2 b, float t) {
-    const float2 d = __ffma2_rn(a, make_float2(-1.f, -1.f), b);
-    return __ffma2_rn(make_float2(t, t), d, a);
-}
-
-// b - a of lerp2_, formed alone (the sample cache stores it for the x pairs).
-__device__ __forceinline__ float2 diff2_(float2 a, float2 b) { return __ffma2_rn(a, make_float2(-1.f, -1.f), b); }
+// lerp_ on a pair with one weight: each half equals lerp_ on that half bit for bit.
+__device__ __forceinline__ float2 lerp2_(float2 a, float2 b, float t) { return fma2(both(t), sub2(b, a), a); }
 
 // Trilinear interpolation of 8 corner pairs (odd entries: differences, SampleCache): x, then y,
 // then z (the order of tri3).
 __device__ __forceinline__ float2 tri8p(const float2 (&c)[8], float fx, float fy, float fz) {
-    const float2 tx = make_float2(fx, fx);
-    const float2 a00 = __ffma2_rn(tx, c[1], c[0]), a10 = __ffma2_rn(tx, c[3], c[2]);
-    const float2 a01 = __ffma2_rn(tx, c[5], c[4]), a11 = __ffma2_rn(tx, c[7], c[6]);
+    const float2 tx = both(fx);
+    const float2 a00 = fma2(tx, c[1], c[0]), a10 = fma2(tx, c[3], c[2]);
+    const float2 a01 = fma2(tx, c[5], c[4]), a11 = fma2(tx, c[7], c[6]);
     return lerp2_(lerp2_(a00, a10, fy), lerp2_(a01, a11, fy), fz);
 }
 
-// Loads the 8 padded corners of the cell at `base` into the sample cache as 24 (back, front)
-// float pairs (u, v, w per corner); 16-bit nodes are converted once here, not per sample.
+// Loads the 8 padded corners of the cell at `base` into the sample cache as 24 float pairs
+// ((u, v) back and front, w per corner); 16-bit nodes are converted once here, not per sample.
 template <typename H>
 __device__ __forceinline__ void fill_padded(const KParams &P, const void *pairs, int32_t base, SampleCache &cc) {
-    const int32_t sy = P.pnx, sz = P.pnxy;
+    constexpr int64_t bytes = Store<Pair<H>>::bytes3;
+    const char *row = reinterpret_cast<const char *>(pairs) + base * bytes;
+    const int64_t sy = P.pnx * bytes, sz = P.pnxy * bytes;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int32_t idx = base + ((k & 1) ? 1 : 0) + ((k & 2) ? sy : 0) + ((k & 4) ? sz : 0);
-        float2 c[3];
-        if constexpr (std::is_same<H, float>::value) {
-            Store<Pair<float>>::load3p(pairs, idx, c);
-        } else {
-            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(pairs) + idx);
-            c[0] = Store<Pair<H>>::cvt(q.x);
-            c[1] = Store<Pair<H>>::cvt(q.y);
-            c[2] = Store<Pair<H>>::cvt(q.z);
-        }
-        if (k & 1) {
-            cc.c2[0][k] = diff2_(cc.c2[0][k - 1], c[0]);
-            cc.c2[1][k] = diff2_(cc.c2[1][k - 1], c[1]);
-            cc.c2[2][k] = diff2_(cc.c2[2][k - 1], c[2]);
-        } else {
-            cc.c2[0][k] = c[0]; cc.c2[1][k] = c[1]; cc.c2[2][k] = c[2];
+    for (int k = 0; k < 8; k += 2) {
+        const char *r = row + ((k & 2) ? sy : 0) + ((k & 4) ? sz : 0);
+        float2 a[3], b[3];
+        Store<Pair<H>>::load3p(r, a);
+        Store<Pair<H>>::load3p(r + bytes, b);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            cc.c2[q][k] = a[q];
+            cc.c2[q][k + 1] = sub2(b[q], a[q]);
         }
     }
     cc.base = base;
 }
 
-// The cached corner pairs, reloaded when the cell changes; out[c] = (back, front) value of
-// component c at the sample.  H: the pair's element type (float, bf16 or fp16).
+// The four corners of a 2D cell from the window pair.
 template <typename H>
-__device__ __forceinline__ void tri3p_padded(const KParams &P, const void *pairs, const PCell &c, SampleCache &cc,
-                                             float2 (&out)[3]) {
-    if (c.base != cc.base) fill_padded<H>(P, pairs, c.base, cc);
-    out[0] = tri8p(cc.c2[0], c.fx, c.fy, c.fz);
-    out[1] = tri8p(cc.c2[1], c.fx, c.fy, c.fz);
-    out[2] = tri8p(cc.c2[2], c.fx, c.fy, c.fz);
+__device__ __forceinline__ void fill_edge2(const KParams &P, const void *pairs, int32_t base, SampleCache &cc) {
+    const int32_t idx[4] = {base, base + 1, base + P.pnx, base + P.pnx + 1};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float2 c[2];
+        Store<Pair<H>>::load2p(pairs, idx[k], c);
+        cc.c2d[0][k] = (k & 1) ? sub2(c[0], cc.c2d[0][k - 1]) : c[0];
+        cc.c2d[1][k] = (k & 1) ? sub2(c[1], cc.c2d[1][k - 1]) : c[1];
+    }
+    cc.base = base;
 }
 
-template <typename W> struct PairElem { using type = void; };
-template <typename H> struct PairElem<Pair<H>> { using type = H; };
+// The corners of a cell straight from two ring slots (unpadded grids, both snapshots): corner
+// indices are clamped into the grid, which is the 2D addressing; in 3D the corners outside are then
+// set to zero (the border).  16 loads where the window pair needs 8, but no pass over the grid
+// before the launch.  Against loading every sample's 16 nodes: gr_advance_noalloc, 500,001
+// particles x 20 RK4 steps on 192 x 192 x 64 nodes 1.81 -> 0.49 ms, 1,000 particles x 10 steps
+// 85 -> 67 us; the engine on ring slots, 1e6 particles x 300 steps, 28.3 -> 12.1 ms.
+template <int DIM, typename T>
+__device__ __forceinline__ void fill_ring(const KParams &P, const void *wb, const void *wf, const PCell &c, SampleCache &cc) {
+    constexpr int bytes = DIM == 3 ? Store<T>::bytes3 : Store<T>::bytes2;
+    const int ix = (int)(c.bx - PCELL_BITS), iy = (int)(c.by - PCELL_BITS), iz = DIM == 3 ? (int)(c.bz - PCELL_BITS) : 0;
+    const int x0 = min(max(ix, 0), P.nx - 1), x1 = min(max(ix + 1, 0), P.nx - 1);
+    const int y0 = min(max(iy, 0), P.ny - 1), y1 = min(max(iy + 1, 0), P.ny - 1);
+    const int32_t dx = (x1 - x0) * bytes;
+    if constexpr (DIM == 2) {
+        const int32_t row[2] = {y0 * P.nx + x0, y1 * P.nx + x0};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const char *b = reinterpret_cast<const char *>(wb) + (int64_t)row[r] * bytes;
+            const char *f = reinterpret_cast<const char *>(wf) + (int64_t)row[r] * bytes;
+            const float2 b0 = Store<T>::load2(b), b1 = Store<T>::load2(b + dx);
+            const float2 f0 = Store<T>::load2(f), f1 = Store<T>::load2(f + dx);
+            cc.c2d[0][2 * r] = b0; cc.c2d[0][2 * r + 1] = sub2(b1, b0);
+            cc.c2d[1][2 * r] = f0; cc.c2d[1][2 * r + 1] = sub2(f1, f0);
+        }
+    } else {
+        const int z0 = min(max(iz, 0), P.nz - 1), z1 = min(max(iz + 1, 0), P.nz - 1);
+        const int32_t row[4] = {(z0 * P.ny + y0) * P.nx + x0, (z0 * P.ny + y1) * P.nx + x0,
+                                (z1 * P.ny + y0) * P.nx + x0, (z1 * P.ny + y1) * P.nx + x0};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const char *b = reinterpret_cast<const char *>(wb) + (int64_t)row[r] * bytes;
+            const char *f = reinterpret_cast<const char *>(wf) + (int64_t)row[r] * bytes;
+            Store<T>::load3(b, cc.c2[0][2 * r], cc.c2[2][2 * r].x);
+            Store<T>::load3(b + dx, cc.c2[0][2 * r + 1], cc.c2[2][2 * r + 1].x);
+            Store<T>::load3(f, cc.c2[1][2 * r], cc.c2[2][2 * r].y);
+            Store<T>::load3(f + dx, cc.c2[1][2 * r + 1], cc.c2[2][2 * r + 1].y);
+        }
+        if ((unsigned)ix >= (unsigned)(P.nx - 1) || (unsigned)iy >= (unsigned)(P.ny - 1) ||
+            (unsigned)iz >= (unsigned)(P.nz - 1)) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const bool in = (unsigned)(ix + (k & 1)) < (unsigned)P.nx &&
+                                (unsigned)(iy + ((k >> 1) & 1)) < (unsigned)P.ny &&
+                                (unsigned)(iz + (k >> 2)) < (unsigned)P.nz;
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (!in) cc.c2[q][k] = make_float2(0.f, 0.f);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k += 2)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) cc.c2[q][k + 1] = sub2(cc.c2[q][k + 1], cc.c2[q][k]);
+    }
+    cc.base = c.base;
+}
+
+template <typename W> struct Elem { using type = W; };
+template <typename H> struct Elem<Pair<H>> { using type = H; };
+
+// Loads the corners of cell c into the sample cache: from the window pair wb, or from the ring
+// slots wb and wf.
+template <int DIM, typename W>
+__device__ __forceinline__ void fill(const KParams &P, const void *wb, const void *wf, const PCell &c, SampleCache &cc) {
+    using H = typename Elem<W>::type;
+    if constexpr (!IsPair<W>::value) fill_ring<DIM, H>(P, wb, wf, c, cc);
+    else if constexpr (DIM == 3) fill_padded<H>(P, wb, c.base, cc);
+    else fill_edge2<H>(P, wb, c.base, cc);
+}
+
+// Horizontal components as a pair.
+struct V3 {
+    float2 xy;
+    float z;
+};
 
 // Trilinear interpolation of one scalar float32 plane.
 __device__ __forceinline__ float tri1(const float *plane, const Cell3 &c) {
@@ -445,132 +518,62 @@ __device__ __forceinline__ Cell2 make_cell2(int nx, int ny, int fw, float ax, fl
     return c;
 }
 
-template <typename W>
-__device__ __forceinline__ void bil2(const void *slot, const Cell2 &c, float &ou, float &ov) {
-    float u0, v0, u1, v1, u2, v2, u3, v3;
-    Store<W>::load2(slot, c.i00, u0, v0);
-    Store<W>::load2(slot, c.i10, u1, v1);
-    Store<W>::load2(slot, c.i01, u2, v2);
-    Store<W>::load2(slot, c.i11, u3, v3);
-    ou = lerp_(lerp_(u0, u1, c.fx), lerp_(u2, u3, c.fx), c.fy);
-    ov = lerp_(lerp_(v0, v1, c.fx), lerp_(v2, v3, c.fx), c.fy);
-}
-
-// 2D window pair with replicated edges: padded node (x, y), x in [-1, nx + 1] and y in
-// [-1, ny + 1], of a (nx + 3) x (ny + 3) buffer holds node (clamp(x), clamp(y)), so a coordinate
-// clamped to [-1, n] reads the clamp-addressed corners of make_cell2 without index clamps.  Same
-// values: inside [-1, n] cell, fraction and corners are unchanged; outside it both corners of the
-// axis are the same edge node, interpolated with any fraction to that node's value exactly.
-// The cache keeps the 4 corners as floats (16 registers), keyed by the first corner's index.
-template <typename W>
-__device__ __forceinline__ void bil2p_padded(const KParams &P, const void *pairs, float ax, float ay, int fw,
-                                             SampleCache &cc, float2 (&out)[2]) {
-    float fx, fy;
-    const uint32_t bx = pcell1(ax, P.fn[0], fw, fx);
-    const uint32_t by = pcell1(ay, P.fn[1], fw, fy);
-    const uint32_t sy = (uint32_t)P.pnx;
-    const int32_t base = (int32_t)(by * sy + bx - (PCELL_BITS - 1u) * (sy + 1u));   // (iy + 1) pnx + (ix + 1)
-    if (base != cc.base) {
-        const int32_t idx[4] = {base, base + 1, base + P.pnx, base + P.pnx + 1};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float2 c[2];
-            Store<W>::load2p(pairs, idx[k], c);
-            cc.c2d[0][k] = (k & 1) ? diff2_(cc.c2d[0][k - 1], c[0]) : c[0];
-            cc.c2d[1][k] = (k & 1) ? diff2_(cc.c2d[1][k - 1], c[1]) : c[1];
-        }
-        cc.base = base;
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        out[k] = lerp2_(__ffma2_rn(make_float2(fx, fx), cc.c2d[k][1], cc.c2d[k][0]),
-                        __ffma2_rn(make_float2(fx, fx), cc.c2d[k][3], cc.c2d[k][2]), fy);
-}
-
-
 __device__ __forceinline__ float bil1(const float *plane, const Cell2 &c) {
     return lerp_(lerp_(__ldg(plane + c.i00), __ldg(plane + c.i10), c.fx),
                  lerp_(__ldg(plane + c.i01), __ldg(plane + c.i11), c.fx), c.fy);
 }
 
-struct V3 {
-    float x, y, z;
-};
-
 __device__ __forceinline__ float dot3(const V3 &a, const V3 &b, int dim) {
-    float s = a.x * b.x;
-    s = __fmaf_rn(a.y, b.y, s);
+    float s = a.xy.x * b.xy.x;
+    s = __fmaf_rn(a.xy.y, b.xy.y, s);
     if (dim == 3) s = __fmaf_rn(a.z, b.z, s);
     return s;
 }
 
-// Wind at world position p, time weight t: interpolate() of TrajectoryIntegrator.icc:42-110.
-// FT: the step kernel's feature set; lean variants run with filter_weights off (kernel_features).
-template <int DIM, typename W, int FT = FT_GENERIC>
-__device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf,
-                                      SampleCache &cc) {
-    V3 r{0.f, 0.f, 0.f};
-    const int fw = (FT & FT_LEAN) ? 0 : P.filter_weights;
-    const float ax = (p.x - P.off[0]) * P.inv_scale[0];
-    const float ay = (p.y - P.off[1]) * P.inv_scale[1];
-    if constexpr (IsPair<W>::value) {
-        // window-pair layout (dynamic wind only): wb points at the pair buffer
-        if (DIM == 3) {
-            const float az = (p.z - P.off[2]) * P.inv_scale[2];
-            const PCell c = make_pcell(P, ax, ay, az, fw);
-            float2 bf[3];
-            using H = typename PairElem<W>::type;
-            tri3p_padded<H>(P, wb, c, cc, bf);
-            r.x = lerp_(bf[0].x, bf[0].y, t); r.y = lerp_(bf[1].x, bf[1].y, t); r.z = lerp_(bf[2].x, bf[2].y, t);
-        } else {
-            float2 bf[2];
-            bil2p_padded<W>(P, wb, ax, ay, fw, cc, bf);
-            r.x = lerp_(bf[0].x, bf[0].y, t); r.y = lerp_(bf[1].x, bf[1].y, t);
-        }
-        return r;
-    } else {
-    if (DIM == 3) {
-        const float az = (p.z - P.off[2]) * P.inv_scale[2];
-        const Cell3 c = make_cell3(P, ax, ay, az);
-        float bu, bv, bw;
-        tri3<W>(wb, c, bu, bv, bw);
-        if (P.wind_dynamic) {
-            float fu, fv, fw;
-            tri3<W>(wf, c, fu, fv, fw);
-            r.x = lerp_(bu, fu, t); r.y = lerp_(bv, fv, t); r.z = lerp_(bw, fw, t);
-        } else {
-            r.x = bu; r.y = bv; r.z = bw;
-        }
-    } else {
-        const Cell2 c = make_cell2(P.nx, P.ny, P.filter_weights, ax, ay);
-        float bu, bv;
-        bil2<W>(wb, c, bu, bv);
-        if (P.wind_dynamic) {
-            float fu, fv;
-            bil2<W>(wf, c, fu, fv);
-            r.x = lerp_(bu, fu, t); r.y = lerp_(bv, fv, t);
-        } else {
-            r.x = bu; r.y = bv;
-        }
-    }
-    return r;
-    }
+// World position -> grid coordinates.
+__device__ __forceinline__ float2 grid_xy(const KParams &P, float2 p) {
+    return mul2(add2(p, make_float2(P.noff[0], P.noff[1])), make_float2(P.inv_scale[0], P.inv_scale[1]));
+}
+__device__ __forceinline__ float grid_z(const KParams &P, float z) { return (z + P.noff[2]) * P.inv_scale[2]; }
+
+// Cell of a sample at world position p.
+template <int DIM, typename W, int FT>
+__device__ __forceinline__ PCell cell_at(const KParams &P, const V3 &p) {
+    constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
+    const int fw = options ? P.filter_weights : 0;
+    const float lo = IsPair<W>::value || DIM == 2 ? -1.0f : P.flo;
+    const int wide = options && !IsPair<W>::value ? P.wide : 0;
+    return make_pcell<DIM>(P, grid_xy(P, p.xy), DIM == 3 ? grid_z(P, p.z) : 0.f, fw, lo, wide);
 }
 
-template <int DIM, typename W>
-__device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf) {
-    SampleCache cc;
-    cc.reset();
-    return wind_at<DIM, W>(P, p, t, wb, wf, cc);
+// Wind at world position p, time weight t: interpolate() of TrajectoryIntegrator.icc:42-110.  The
+// cell's corners come from the sample cache, reloaded when the cell changes (wb: the window pair; or
+// wb, wf: the ring slots), interpolated in space, then in time.
+// FT: the step kernel's feature set; lean variants run with filter_weights off (kernel_features).
+template <int DIM, typename W, int FT>
+__device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf,
+                                      SampleCache &cc) {
+    const PCell c = cell_at<DIM, W, FT>(P, p);
+    if (!IsPair<W>::value && (!(FT & FT_LEAN) || (FT & FT_BORDER)) && P.wide) cc.reset();
+    if (c.base != cc.base) fill<DIM, W>(P, wb, wf, c, cc);
+    const bool dynamic = IsPair<W>::value || (FT & FT_LEAN) || P.wind_dynamic;
+    if constexpr (DIM == 3) {
+        const float2 b = tri8p(cc.c2[0], c.fx, c.fy, c.fz), f = tri8p(cc.c2[1], c.fx, c.fy, c.fz);
+        const float2 w = tri8p(cc.c2[2], c.fx, c.fy, c.fz);
+        return dynamic ? V3{lerp2_(b, f, t), lerp_(w.x, w.y, t)} : V3{b, w.x};
+    } else {
+        const float2 tx = both(c.fx);
+        const float2 b = lerp2_(fma2(tx, cc.c2d[0][1], cc.c2d[0][0]), fma2(tx, cc.c2d[0][3], cc.c2d[0][2]), c.fy);
+        const float2 f = lerp2_(fma2(tx, cc.c2d[1][1], cc.c2d[1][0]), fma2(tx, cc.c2d[1][3], cc.c2d[1][2]), c.fy);
+        return V3{dynamic ? lerp2_(b, f, t) : b, 0.f};
+    }
 }
 
 // sphere_coordinates (TrajectoryIntegrator.tpp:98-104).
 __device__ __forceinline__ V3 sphere_(const KParams &P, float py, V3 v) {
     const float pi = 3.14159265358979323846f;
-    V3 r{0.f, 0.f, 0.f};
-    r.x = (v.x * 180.f) / (P.sphere_radius * cosf(py * (pi * 2.f) / 360.f) * pi);
-    r.y = (v.y * 180.f) / (pi * P.sphere_radius);
-    return r;
+    return V3{{(v.xy.x * 180.f) / (P.sphere_radius * cosf(py * (pi * 2.f) / 360.f) * pi),
+               (v.xy.y * 180.f) / (pi * P.sphere_radius)}, 0.f};
 }
 
 __device__ __forceinline__ float ref_at(const float (&ref)[19], int i) {
@@ -676,8 +679,8 @@ __device__ __forceinline__ void eval_extras(const KParams &P, const Code &code, 
     const float t0 = GR_OPT(P, dyn_any) ? E.t0 : 0.f;
     if (GR_OPT(P, volume_mode) != 0 && GR_OPT(P, nvol) > 0) {
         const int vb = GR_OPT(P, volume_mode) == 2 ? E.slot_back : 0, vf = GR_OPT(P, volume_mode) == 2 ? E.slot_front : 0;
-        const float ax = (p.x - P.off[0]) * P.inv_scale[0];
-        const float ay = (p.y - P.off[1]) * P.inv_scale[1];
+        const float ax = (p.xy.x - P.off[0]) * P.inv_scale[0];
+        const float ay = (p.xy.y - P.off[1]) * P.inv_scale[1];
         if (DIM == 3) {
             const float az = (p.z - P.off[2]) * P.inv_scale[2];
             const Cell3 c = make_cell3(P, ax, ay, az);
@@ -703,7 +706,7 @@ __device__ __forceinline__ void eval_extras(const KParams &P, const Code &code, 
     }
     if (GR_OPT(P, nexpr) > 0) {
         float ref[19];
-        ref[0] = p.x; ref[1] = p.y; ref[2] = DIM == 3 ? p.z : 0.f;
+        ref[0] = p.xy.x; ref[1] = p.xy.y; ref[2] = DIM == 3 ? p.z : 0.f;
         ref[3] = GR_OPT(P, curvature_mode) == 3 ? cv : 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) ref[4 + k] = k < GR_OPT(P, nvol) ? vol[k] : 0.f;
@@ -722,7 +725,7 @@ __device__ __forceinline__ void eval_extras(const KParams &P, const Code &code, 
             }
             ref[12 + k] = c;
         }
-        ref[16] = vc.x; ref[17] = vc.y; ref[18] = DIM == 3 ? vc.z : 0.f;
+        ref[16] = vc.xy.x; ref[17] = vc.xy.y; ref[18] = DIM == 3 ? vc.z : 0.f;
 #pragma unroll
         for (int e = 0; e < GR_MAX_EXPR; ++e)
             if (e < GR_OPT(P, nexpr)) cmp[e] = code.eval(e, ref);
@@ -805,8 +808,8 @@ __device__ __forceinline__ void deferred_extras(const KParams &P, const Code &co
             const float cv = GR_OPT(P, curvature_mode) == 3 ? P.curv[i] : 0.f;
             const float4 a = P.vrec[2 * i], v = P.vrec[2 * i + 1];
             const int32_t last_s = __float_as_int(v.w);
-            extras_at<DIM>(P, code, i, pid, last_s >= 0, last_s < 0 ? 0 : last_s, V3{a.x, a.y, a.z},
-                           V3{v.x, v.y, v.z}, cv, irec);
+            extras_at<DIM>(P, code, i, pid, last_s >= 0, last_s < 0 ? 0 : last_s, V3{{a.x, a.y}, a.z},
+                           V3{{v.x, v.y}, v.z}, cv, irec);
         } else {
             if (!all && P.status[i] == 0 && !(P.life && P.life[i] <= k_end)) continue;
             const float4 v = P.vlast[i];
@@ -814,8 +817,8 @@ __device__ __forceinline__ void deferred_extras(const KParams &P, const Code &co
             if (last_s < 0) continue;
             const int64_t pid = P.id[i];
             const float cv = GR_OPT(P, curvature_mode) == 3 ? P.curv[i] : 0.f;
-            const V3 p{P.px[i], P.py[i], DIM == 3 ? P.pz[i] : 0.f};
-            extras_at<DIM>(P, code, i, pid, true, last_s, p, V3{v.x, v.y, v.z}, cv, -1);
+            const V3 p{{P.px[i], P.py[i]}, DIM == 3 ? P.pz[i] : 0.f};
+            extras_at<DIM>(P, code, i, pid, true, last_s, p, V3{{v.x, v.y}, v.z}, cv, -1);
             reinterpret_cast<int32_t *>(P.vlast + i)[3] = -1;
         }
     }
@@ -831,9 +834,7 @@ __global__ void __launch_bounds__(256, 3) deferred_extras_kernel(const __grid_co
         deferred_extras<DIM>(P, GlobalCode{P.prog}, rec, irec, k_end, all);
 }
 
-#ifndef GR_ADV_MIN_BLOCKS
-#define GR_ADV_MIN_BLOCKS 2
-#endif
+constexpr int GR_ADV_MIN_BLOCKS = 2, GR_F32_BLOCKS = 4, GR_LIGHT_BLOCKS = 5;   // AdvBounds
 
 // Advances the particle in slot i through steps [s0, s1) (or until its lifetime ends).
 template <int DIM, bool RK4, typename W, int FT>
@@ -847,28 +848,29 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     const int uplift_mode = LEAN ? 0 : P.uplift_mode;
     const bool compensated = LEAN ? (FT & FT_COMP) != 0 : P.compensated != 0;
     const bool topography = LEAN ? false : P.topography != 0;
-    const int border_mode = LEAN ? 0 : P.border_mode;
+    const int border_mode = LEAN && !(FT & FT_BORDER) ? 0 : P.border_mode;
     unsigned *const alive_at = LEAN ? nullptr : P.alive_at;
     const bool valid = i < n_live;
     int32_t st = valid ? P.status[i] : 1;
     bool alive = st == 0;
-    const int64_t pid = valid ? (int64_t)P.id[i] : 0;
+    const int64_t pid = valid && P.id ? (int64_t)P.id[i] : 0;   // no ids: a launch without records
 
-    V3 p{0.f, 0.f, 0.f}, q{0.f, 0.f, 0.f}, comp{0.f, 0.f, 0.f}, ld{0.f, 0.f, 0.f};
+    const V3 zero{{0.f, 0.f}, 0.f};
+    V3 p = zero, q = zero, comp = zero, ld = zero;
     float len = 0.f, tc = 0.f, cv = 0.f;
 
     const bool curv_prev = curvature_mode == 1 || curvature_mode == 3;
     float seg = 0.f;   // |p - q| (curvature's ds): carried from the step that formed it
     if (valid) {
-        p.x = P.px[i]; p.y = P.py[i];
+        p.xy = make_float2(P.px[i], P.py[i]);
         if (DIM == 3) p.z = P.pz[i];
         if (curv_prev) {
-            q.x = P.qx[i]; q.y = P.qy[i]; if (DIM == 3) q.z = P.qz[i];
-            const V3 a{p.x - q.x, p.y - q.y, p.z - q.z};
+            q.xy = make_float2(P.qx[i], P.qy[i]); if (DIM == 3) q.z = P.qz[i];
+            const V3 a{sub2(p.xy, q.xy), p.z - q.z};
             seg = sqrtf(dot3(a, a, DIM));
         }
-        if (compensated) { comp.x = P.kx[i]; comp.y = P.ky[i]; if (DIM == 3) comp.z = P.kz[i]; }
-        if (curvature_mode == 2) { ld.x = P.lx[i]; ld.y = P.ly[i]; if (DIM == 3) ld.z = P.lz[i]; }
+        if (compensated) { comp.xy = make_float2(P.kx[i], P.ky[i]); if (DIM == 3) comp.z = P.kz[i]; }
+        if (curvature_mode == 2) { ld.xy = make_float2(P.lx[i], P.ly[i]); if (DIM == 3) ld.z = P.lz[i]; }
         if (abort_mode != 0) len = P.length[i];
         if (curvature_mode != 0) tc = P.tc[i];
         if (curvature_mode == 3) cv = P.curv[i];
@@ -878,72 +880,79 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     const int32_t life = (valid && P.life) ? P.life[i] : 0x7fffffff;   // steps this particle may run
     const int32_t birth = (valid && P.birth) ? P.birth[i] : 0;          // first step it runs
     const bool extras = LEAN ? (FT & FT_EXTRAS) != 0 : ((P.volume_mode != 0 && P.nvol > 0) || P.nexpr > 0);
-    V3 vc_last{0.f, 0.f, 0.f};
+    V3 vc_last = zero;
     int last_s = P.s0;
     bool dirty = false;   // volumes / expressions not yet evaluated for the last alive step
-    const int sph = !LEAN && P.sphere && DIM == 2;
+    const int sph = (!LEAN || (FT & FT_BORDER)) && P.sphere && DIM == 2;
 
     SampleCache cc;
     cc.reset();
+    int slot = -1;   // ring layouts: back slot of the cached cell
     for (int s = P.s0; s < P.s1; ++s) {
         const StepEntry E = P.sched[s];
+        const int sb = P.wind_dynamic ? E.slot_back : 0, sf = P.wind_dynamic ? E.slot_front : 0;
+        const void *wb = IsPair<W>::value ? P.pair : reinterpret_cast<const char *>(P.wind) + (int64_t)sb * P.wind_stride;
+        const void *wf = reinterpret_cast<const char *>(P.wind) + (int64_t)sf * P.wind_stride;
+        // the cached cell belongs to the window's two snapshots
+        if (!IsPair<W>::value && sb != slot) {
+            cc.reset();
+            slot = sb;
+        }
         if (alive && s < life && s >= birth) {
             ++my_steps;
-            const int sb = P.wind_dynamic ? E.slot_back : 0, sf = P.wind_dynamic ? E.slot_front : 0;
-            const void *wb = IsPair<W>::value ? P.pair : reinterpret_cast<const char *>(P.wind) + (int64_t)sb * P.wind_stride;
-            const void *wf = reinterpret_cast<const char *>(P.wind) + (int64_t)sf * P.wind_stride;
             const float t0 = P.dyn_any ? E.t0 : 0.f;
 
             // integrator (tpp:135-231)
             V3 v, vc;
             if (RK4) {
-                // the four stages as one loop (one copy of the sampling code, which keeps the
-                // step loop within the instruction cache): stage k samples at a with its time
-                // weight, and the sum ((k1 + 2 k2) + 2 k3) + k4 is accumulated in that order
-                V3 a = p, acc{0.f, 0.f, 0.f}, accc{0.f, 0.f, 0.f};
-#pragma unroll 1
+                // stage k samples at a with its time weight, and the sum ((k1 + 2 k2) + 2 k3) + k4
+                // is accumulated in that order (wgt * k is exact, so the fused sum rounds like the
+                // separate one).  Unrolled in the lean variants, where the weights and time
+                // selects become constants: 30 launches of the 1e6-particle plain configuration
+                // take 7.63 ms against 8.08 ms as one loop of four and 7.94 ms two by two.  The
+                // generic variant's longer step stays ahead two by two (65,000 particles with
+                // every option: 1.007 ms against 1.018 ms unrolled).
+                V3 a = p, acc = zero, accc = zero;
+                constexpr int kUnroll = LEAN ? 4 : 2;
+#pragma unroll kUnroll
                 for (int stage = 0; stage < 4; ++stage) {
                     const float tw = stage == 0 ? t0 : (stage == 3 ? E.t2 : E.t1);
                     const V3 kc = wind_at<DIM, W, FT>(P, a, tw, wb, wf, cc);
-                    const V3 k = sph ? sphere_(P, a.y, kc) : kc;
+                    const V3 k = sph ? sphere_(P, a.xy.y, kc) : kc;
                     if (stage == 0) {
                         acc = k;
                         accc = kc;
                     } else {
-                        const float wgt = stage == 3 ? 1.f : 2.f;   // 1 * k is exact: the same sum
-                        acc = V3{acc.x + wgt * k.x, acc.y + wgt * k.y, acc.z + wgt * k.z};
-                        if (sph) accc = V3{accc.x + wgt * kc.x, accc.y + wgt * kc.y, 0.f};
+                        const float wgt = stage == 3 ? 1.f : 2.f;
+                        acc.xy = fma2(both(wgt), k.xy, acc.xy);
+                        if (DIM == 3) acc.z = __fmaf_rn(wgt, k.z, acc.z);
+                        if (sph) accc.xy = fma2(both(wgt), kc.xy, accc.xy);
                     }
                     const float c = stage < 2 ? P.hh : P.h;
-                    a = V3{__fmaf_rn(k.x, c, p.x), __fmaf_rn(k.y, c, p.y), DIM == 3 ? __fmaf_rn(k.z, c, p.z) : 0.f};
+                    a.xy = fma2(k.xy, both(c), p.xy);
+                    if (DIM == 3) a.z = __fmaf_rn(k.z, c, p.z);
                 }
-                v.x = acc.x * P.sixth;
-                v.y = acc.y * P.sixth;
-                v.z = DIM == 3 ? acc.z * P.sixth : 0.f;
-                if (sph) {
-                    vc.x = accc.x * P.sixth;
-                    vc.y = accc.y * P.sixth;
-                    vc.z = 0.f;
-                } else {
-                    vc = v;
-                }
+                v = V3{mul2(acc.xy, both(P.sixth)), DIM == 3 ? acc.z * P.sixth : 0.f};
+                vc = sph ? V3{mul2(accc.xy, both(P.sixth)), 0.f} : v;
             } else {
                 vc = wind_at<DIM, W, FT>(P, p, t0, wb, wf, cc);
-                v = sph ? sphere_(P, p.y, vc) : vc;
+                v = sph ? sphere_(P, p.xy.y, vc) : vc;
             }
 
-            // displacement, reverse and uplift (tpp:233-250)
-            V3 dp{v.x * P.h, v.y * P.h, DIM == 3 ? v.z * P.h : 0.f};
-            if (P.reverse) { dp.x = -dp.x; dp.y = -dp.y; dp.z = -dp.z; }
+            // displacement, reverse and uplift (tpp:233-250).  A reversed step subtracts the
+            // negated displacement: without uplift that is the forward step, bit for bit, so the
+            // lean variants leave the option out.
+            const bool reverse = !LEAN && P.reverse;
+            V3 dp{mul2(v.xy, both(P.h)), DIM == 3 ? v.z * P.h : 0.f};
+            if (reverse) { dp.xy = make_float2(-dp.xy.x, -dp.xy.y); dp.z = -dp.z; }
             if (DIM == 3 && uplift_mode != 0) {
                 const int lb = uplift_mode == 2 ? E.slot_back : 0, lf = uplift_mode == 2 ? E.slot_front : 0;
                 const float *LB = P.lift + (int64_t)lb * P.n_total * 3 + pid * 3;
                 const float *LF = P.lift + (int64_t)lf * P.n_total * 3 + pid * 3;
                 if (uplift_mode == 1) {
-                    dp.x = dp.x + LB[0]; dp.y = dp.y + LB[1]; dp.z = dp.z + LB[2];
+                    dp.xy = add2(dp.xy, make_float2(LB[0], LB[1])); dp.z = dp.z + LB[2];
                 } else {
-                    dp.x = dp.x + lerp_(LB[0], LF[0], t0);
-                    dp.y = dp.y + lerp_(LB[1], LF[1], t0);
+                    dp.xy = add2(dp.xy, lerp2_(make_float2(LB[0], LB[1]), make_float2(LF[0], LF[1]), t0));
                     dp.z = dp.z + lerp_(LB[2], LF[2], t0);
                 }
             }
@@ -956,7 +965,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                 if (abort_mode == 2) {
                     if (nl > P.max_length) {
                         const float sc = (P.max_length - len) / dpl;
-                        dp.x = sc * dp.x; dp.y = sc * dp.y; dp.z = sc * dp.z;
+                        dp.xy = mul2(both(sc), dp.xy); dp.z = sc * dp.z;
                         len = P.max_length;
                         abort = 1;
                     } else {
@@ -969,37 +978,37 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
             }
 
             // new position (tpp:282); Kahan-compensated in the precision form
-            V3 np;
+            V3 np = zero;
             if (compensated) {
-                const V3 sd{P.reverse ? -dp.x : dp.x, P.reverse ? -dp.y : dp.y, P.reverse ? -dp.z : dp.z};
-                float y = sd.x - comp.x, t = p.x + y;
-                np.x = t; comp.x = (t - p.x) - y;
-                y = sd.y - comp.y; t = p.y + y;
-                np.y = t; comp.y = (t - p.y) - y;
-                if (DIM == 3) { y = sd.z - comp.z; t = p.z + y; np.z = t; comp.z = (t - p.z) - y; }
-                else np.z = 0.f;
+                const V3 sd = reverse ? V3{{-dp.xy.x, -dp.xy.y}, -dp.z} : dp;
+                const float2 y = sub2(sd.xy, comp.xy);
+                np.xy = add2(p.xy, y);
+                comp.xy = sub2(sub2(np.xy, p.xy), y);
+                if (DIM == 3) { const float yz = sd.z - comp.z; np.z = p.z + yz; comp.z = (np.z - p.z) - yz; }
             } else {
-                np.x = P.reverse ? p.x - dp.x : p.x + dp.x;
-                np.y = P.reverse ? p.y - dp.y : p.y + dp.y;
-                np.z = DIM == 3 ? (P.reverse ? p.z - dp.z : p.z + dp.z) : 0.f;
+                np.xy = reverse ? sub2(p.xy, dp.xy) : add2(p.xy, dp.xy);
+                if (DIM == 3) np.z = reverse ? p.z - dp.z : p.z + dp.z;
             }
 
             // border and abort checks (tpp:284-323, icc:7-20, tpp:13-96)
             if (abort == 0) {
                 const float dp2 = dot3(dp, dp, DIM);
                 const int bm = DIM == 3 ? 0 : border_mode;
+                const float2 rel = add2(np.xy, make_float2(P.noff[0], P.noff[1]));   // np - off
                 if (bm == 0) {
                     bool topo = false;
                     if (DIM == 3 && topography) {
-                        const Cell2 c = make_cell2(P.nx, P.ny, P.filter_weights, np.x / P.scale[0], np.y / P.scale[1]);
+                        const Cell2 c = make_cell2(P.nx, P.ny, P.filter_weights, np.xy.x / P.scale[0], np.xy.y / P.scale[1]);
                         topo = bil1(P.topo, c) > np.z;
                     }
                     if (topo) abort = 3;
                     else if (dp2 < 1e-9f) abort = 4;
                     else {
-                        bool out = np.x - P.off[0] > P.dom[0] || np.x - P.off[0] < 0.f ||
-                                   np.y - P.off[1] > P.dom[1] || np.y - P.off[1] < 0.f;
-                        if (DIM == 3) out = out || np.z - P.off[2] > P.dom[2] || np.z - P.off[2] < 0.f;
+                        bool out = rel.x > P.dom[0] || rel.x < 0.f || rel.y > P.dom[1] || rel.y < 0.f;
+                        if (DIM == 3) {
+                            const float rz = np.z + P.noff[2];
+                            out = out || rz > P.dom[2] || rz < 0.f;
+                        }
                         if (out) abort = 2;
                     }
                 } else if (dp2 < 1e-9f) {
@@ -1007,31 +1016,31 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                 } else {
                     const float ox = P.off[0], oy = P.off[1], DX = P.dom[0], DY = P.dom[1];
                     if (bm == 1) {
-                        np.x = fmodf(np.x - ox + DX, DX) + ox;
-                        if (np.y - oy > DY || np.y - oy < 0.f) abort = 2;
+                        np.xy.x = fmodf(rel.x + DX, DX) + ox;
+                        if (rel.y > DY || rel.y < 0.f) abort = 2;
                     } else if (bm == 2) {
                         if (sph) {
-                            if (np.x - ox > DX || np.x - ox < 0.f || np.y - oy > DY || np.y - oy < 0.f) abort = 2;
+                            if (rel.x > DX || rel.x < 0.f || rel.y > DY || rel.y < 0.f) abort = 2;
                         } else {
-                            np.y = fmodf(np.y - oy + DY, DY) + oy;
-                            if (np.x - ox > DX || np.x - ox < 0.f) abort = 2;
+                            np.xy.y = fmodf(rel.y + DY, DY) + oy;
+                            if (rel.x > DX || rel.x < 0.f) abort = 2;
                         }
                     } else {
                         if (sph) {
-                            const float nx_ = np.x - ox, ny_ = np.y - oy, px_ = p.x - ox, py_ = p.y - oy;
-                            if (ny_ < 0.f) {
-                                const float tx = (-py_) / (ny_ - py_) * (nx_ - px_) + px_;
-                                np.y = -ny_ + oy;
-                                np.x = fmodf(DX + 180.0f - nx_ + 2.f * tx, DX) + ox;
-                            } else if (ny_ >= DY) {
-                                const float tx = (DY - py_) / (ny_ - py_) * (nx_ - px_) + px_;
-                                np.y = (ny_ - DY) + oy;
-                                np.x = fmodf(DX + 180.0f - nx_ + 2.f * tx, DX) + ox;
+                            const float px_ = p.xy.x - ox, py_ = p.xy.y - oy;
+                            if (rel.y < 0.f) {
+                                const float tx = (-py_) / (rel.y - py_) * (rel.x - px_) + px_;
+                                np.xy.y = -rel.y + oy;
+                                np.xy.x = fmodf(DX + 180.0f - rel.x + 2.f * tx, DX) + ox;
+                            } else if (rel.y >= DY) {
+                                const float tx = (DY - py_) / (rel.y - py_) * (rel.x - px_) + px_;
+                                np.xy.y = (rel.y - DY) + oy;
+                                np.xy.x = fmodf(DX + 180.0f - rel.x + 2.f * tx, DX) + ox;
                             }
                         } else {
-                            np.y = fmodf(np.y - oy + DY, DY) + oy;
+                            np.xy.y = fmodf(rel.y + DY, DY) + oy;
                         }
-                        np.x = fmodf(np.x - ox + DX, DX) + ox;
+                        np.xy.x = fmodf(np.xy.x - ox + DX, DX) + ox;
                     }
                 }
             }
@@ -1045,7 +1054,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                 // curvature (tpp:335-361)
                 if (curvature_mode == 2) {
                     const float inv = 1.0f / sqrtf(dot3(v, v, DIM));
-                    const V3 u{v.x * inv, v.y * inv, v.z * inv};
+                    const V3 u{mul2(v.xy, both(inv)), v.z * inv};
                     if (E.flags & SF_TIME_POS) {
                         const float k = acosf(dot3(ld, u, DIM));
                         if (!isnan(k)) tc += k;
@@ -1053,17 +1062,19 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                     ld = u;
                 } else if (curv_prev) {
                     // |np - p|: this segment's length, the next step's |p - q|
-                    const V3 b{np.x - p.x, np.y - p.y, np.z - p.z};
+                    const V3 b{sub2(np.xy, p.xy), np.z - p.z};
                     const float nseg = sqrtf(dot3(b, b, DIM));
                     if (E.flags & SF_TIME_POS) {
                         float k = 0.f;
                         if (DIM == 3) {
                             // central differences scaled by the float reciprocals of 2 h and h h
-                            // (the reference divides, icc:151-154: within one rounding of these)
-                            const V3 d1{(np.x - q.x) * P.inv_2h, (np.y - q.y) * P.inv_2h, (np.z - q.z) * P.inv_2h};
-                            const V3 d2{((q.x + np.x) - 2.f * p.x) * P.inv_hh, ((q.y + np.y) - 2.f * p.y) * P.inv_hh,
-                                        ((q.z + np.z) - 2.f * p.z) * P.inv_hh};
-                            const V3 x{d1.y * d2.z - d1.z * d2.y, d1.z * d2.x - d1.x * d2.z, d1.x * d2.y - d1.y * d2.x};
+                            // (the reference divides, icc:151-154: within one rounding of these);
+                            // the fused (q + np) - 2 p rounds like the separate one (2 p is exact)
+                            const V3 d1{mul2(sub2(np.xy, q.xy), both(P.inv_2h)), (np.z - q.z) * P.inv_2h};
+                            const V3 d2{mul2(fma2(p.xy, both(-2.f), add2(q.xy, np.xy)), both(P.inv_hh)),
+                                        __fmaf_rn(-2.f, p.z, q.z + np.z) * P.inv_hh};
+                            const V3 x{{d1.xy.y * d2.z - d1.z * d2.xy.y, d1.z * d2.xy.x - d1.xy.x * d2.z},
+                                       d1.xy.x * d2.xy.y - d1.xy.y * d2.xy.x};
                             const float l = sqrtf(dot3(d1, d1, 3));
                             k = fabsf(sqrtf(dot3(x, x, 3)) / (l * l * l));
                         }
@@ -1077,7 +1088,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                 // volumes and expressions are evaluated lazily (eval_extras), or after the launch
                 // from the stored inputs (FT_DEFER, deferred_extras_kernel)
                 if constexpr ((FT & FT_DEFER) != 0)
-                    P.vlast[i] = make_float4(vc.x, vc.y, DIM == 3 ? vc.z : 0.f, __int_as_float(s));
+                    P.vlast[i] = make_float4(vc.xy.x, vc.xy.y, DIM == 3 ? vc.z : 0.f, __int_as_float(s));
                 vc_last = vc;
                 last_s = s;
                 dirty = true;
@@ -1090,14 +1101,14 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
 
         if (valid && (E.flags & SF_SAVE)) {
             float *hp = P.hpos + ((int64_t)E.rec * P.n_total + pid) * DIM;
-            hp[0] = p.x; hp[1] = p.y;
+            hp[0] = p.xy.x; hp[1] = p.xy.y;
             if (DIM == 3) hp[2] = p.z;
             if (curvature_mode == 3 && (E.flags & SF_CURV_REC)) P.hcurv[(int64_t)E.crec * P.n_total + pid] = cv;
             if constexpr ((FT & FT_DEFER) != 0) {
                 // the record's inputs: the position and the last moved step's (if any since the
                 // last evaluation)
                 const float4 v = P.vlast[i];
-                P.vrec[2 * i] = make_float4(p.x, p.y, DIM == 3 ? p.z : 0.f, 0.f);
+                P.vrec[2 * i] = make_float4(p.xy.x, p.xy.y, DIM == 3 ? p.z : 0.f, 0.f);
                 P.vrec[2 * i + 1] = v;
                 if (__float_as_int(v.w) >= 0) reinterpret_cast<int32_t *>(P.vlast + i)[3] = -1;
             }
@@ -1107,11 +1118,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                 // refill the sample cache for the next step's first sample (at p): the cached
                 // nodes are then dead while the values above are evaluated, which frees their
                 // registers there
-                if constexpr (IsPair<W>::value && DIM == 3) {
-                    const PCell c = make_pcell(P, (p.x - P.off[0]) * P.inv_scale[0], (p.y - P.off[1]) * P.inv_scale[1],
-                                               (p.z - P.off[2]) * P.inv_scale[2], LEAN ? 0 : P.filter_weights);
-                    fill_padded<typename PairElem<W>::type>(P, P.pair, c.base, cc);
-                }
+                if constexpr (DIM == 3) fill<DIM, W>(P, wb, wf, cell_at<DIM, W, FT>(P, p), cc);
             }
         }
 
@@ -1127,11 +1134,11 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     if (valid && was_alive) {
         if (extras && dirty) record_extras<DIM>(P, i, pid, true, last_s, p, vc_last, cv, -1);
         P.status[i] = st;
-        P.px[i] = p.x; P.py[i] = p.y;
+        P.px[i] = p.xy.x; P.py[i] = p.xy.y;
         if (DIM == 3) P.pz[i] = p.z;
-        if (curv_prev) { P.qx[i] = q.x; P.qy[i] = q.y; if (DIM == 3) P.qz[i] = q.z; }
-        if (compensated) { P.kx[i] = comp.x; P.ky[i] = comp.y; if (DIM == 3) P.kz[i] = comp.z; }
-        if (curvature_mode == 2) { P.lx[i] = ld.x; P.ly[i] = ld.y; if (DIM == 3) P.lz[i] = ld.z; }
+        if (curv_prev) { P.qx[i] = q.xy.x; P.qy[i] = q.xy.y; if (DIM == 3) P.qz[i] = q.z; }
+        if (compensated) { P.kx[i] = comp.xy.x; P.ky[i] = comp.xy.y; if (DIM == 3) P.kz[i] = comp.z; }
+        if (curvature_mode == 2) { P.lx[i] = ld.xy.x; P.ly[i] = ld.xy.y; if (DIM == 3) P.lz[i] = ld.z; }
         if (abort_mode != 0) P.length[i] = len;
         if (curvature_mode != 0) P.tc[i] = tc;
         if (curvature_mode == 3) P.curv[i] = cv;
@@ -1144,33 +1151,22 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
 // One thread per particle, or (P.grid_stride) a persistent grid striding over the live
 // prefix, whose size is read on the device: the launch shape then stays fixed while the live
 // count shrinks, as a captured CUDA graph needs.
-// Launch bounds: 256 threads, 2 blocks per SM (128 registers).  The float32 3D pair kernel keeps
-// 48 cached floats in 128-thread blocks: 4 per SM (128 registers) in the generic variant and the
-// lean ones with volume / expression values or with both Kahan positions and curvature, 5 per SM
-// (96 registers, 20 warps) in the other lean ones, whose state fits there without spills; the
-// extra warps hide more of the sampling and curvature latency.  The 16-bit kernels: AdvBounds16.
-template <int DIM, typename W, int FT> struct AdvBounds { static constexpr int threads = 256, blocks = GR_ADV_MIN_BLOCKS; };
-#ifndef GR_F32_PAIR_BLOCKS
-#define GR_F32_PAIR_BLOCKS 4
-#endif
-#ifndef GR_F32_LIGHT_BLOCKS
-#define GR_F32_LIGHT_BLOCKS 5
-#endif
-// 16-bit 3D pair kernels: 128 x 5 for the lean variants with curvature or deferred values
-// (measured 5-6% faster than 256 x 2 on the 3D benchmark configuration), 256 x 2 for the rest
-// (the positions-only variant of the batching and serving forms measured 2% slower at 128 x 5).
-template <typename H, int FT> struct AdvBounds16 {
+// Launch bounds: 256 threads, 2 blocks per SM (128 registers).  The float32 3D kernels keep 48
+// cached floats in 128-thread blocks: 4 per SM (128 registers) in the generic variant and the lean
+// ones with volume / expression values or with both Kahan positions and curvature, 5 per SM (96
+// registers, 20 warps) in the other lean ones, whose state fits there without spills; the extra warps
+// hide more of the sampling and curvature latency.  16-bit 3D kernels: 128 x 5 for the lean variants
+// with curvature or deferred values (measured 5-6% faster than 256 x 2 on the 3D benchmark
+// configuration), 256 x 2 for the rest (the positions-only variant of the batching and serving forms
+// measured 2% slower at 128 x 5).
+template <int DIM, typename W, int FT> struct AdvBounds {
+    static constexpr bool f32 = std::is_same<typename Elem<W>::type, float>::value;
     static constexpr bool light = (FT & FT_LEAN) != 0 && (FT & FT_EXTRAS) == 0 &&
                                   (FT & (FT_COMP | FT_CURV)) != (FT_COMP | FT_CURV) &&
-                                  (FT & (FT_CURV | FT_DEFER)) != 0;
-    static constexpr int threads = light ? 128 : 256, blocks = light ? GR_F32_LIGHT_BLOCKS : GR_ADV_MIN_BLOCKS;
-};
-template <int FT> struct AdvBounds<3, Pair<__nv_bfloat16>, FT> : AdvBounds16<__nv_bfloat16, FT> {};
-template <int FT> struct AdvBounds<3, Pair<__half>, FT> : AdvBounds16<__half, FT> {};
-template <int FT> struct AdvBounds<3, Pair<float>, FT> {
-    static constexpr bool light = (FT & FT_LEAN) != 0 && (FT & FT_EXTRAS) == 0 &&
-                                  (FT & (FT_COMP | FT_CURV)) != (FT_COMP | FT_CURV);
-    static constexpr int threads = 128, blocks = light ? GR_F32_LIGHT_BLOCKS : GR_F32_PAIR_BLOCKS;
+                                  (f32 || (FT & (FT_CURV | FT_DEFER)) != 0);
+    static constexpr bool small = DIM == 3 && (f32 || light);   // 128-thread blocks
+    static constexpr int threads = small ? 128 : 256;
+    static constexpr int blocks = !small ? GR_ADV_MIN_BLOCKS : light ? GR_LIGHT_BLOCKS : GR_F32_BLOCKS;
 };
 
 template <int DIM, bool RK4, typename W, int FT>

@@ -16,7 +16,7 @@
 #include <string>
 
 #include "../../include/granite_b200.h"
-#include "granite_kernels.cuh"
+#include "advance.h"
 
 namespace granite_b200 {
 void set_last_error(const char *msg);   // engine.cu
@@ -69,116 +69,6 @@ __global__ void __launch_bounds__(256) noalloc_schedule_kernel(NoAllocScratch *S
         E.slot_back = 0;
         E.slot_front = 1;
         S->sched[k] = E;
-    }
-}
-
-// The plain step loop of advance_kernel (granite_kernels.cuh) with the same arithmetic:
-// no curvature, volumes, expressions, uplift, constants, topography or length abort.
-template <int DIM, bool RK4>
-__global__ void __launch_bounds__(256) advance_plain_kernel(const __grid_constant__ KParams P,
-                                                            NoAllocScratch *S) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < P.n;
-    bool alive = valid && P.status[i] == 0;
-    const bool was_alive = alive;
-    int32_t st = 0;
-    V3 p{0.f, 0.f, 0.f};
-    if (valid) {
-        p.x = P.px[i];
-        p.y = P.py[i];
-        if (DIM == 3) p.z = P.pz[i];
-    }
-    unsigned my_steps = 0;
-    const int sph = P.sphere && DIM == 2;
-    const void *wb = P.wind;
-    const void *wf = reinterpret_cast<const char *>(P.wind) + P.wind_stride;
-    for (int s = P.s0; s < P.s1 && alive; ++s) {
-        const StepEntry E = S->sched[s];
-        ++my_steps;
-        V3 v;
-        if (RK4) {
-            const V3 k1c = wind_at<DIM, float>(P, p, E.t0, wb, wf);
-            const V3 k1 = sph ? sphere_(P, p.y, k1c) : k1c;
-            V3 a{__fmaf_rn(k1.x, P.hh, p.x), __fmaf_rn(k1.y, P.hh, p.y), DIM == 3 ? __fmaf_rn(k1.z, P.hh, p.z) : 0.f};
-            const V3 k2c = wind_at<DIM, float>(P, a, E.t1, wb, wf);
-            const V3 k2 = sph ? sphere_(P, a.y, k2c) : k2c;
-            a = V3{__fmaf_rn(k2.x, P.hh, p.x), __fmaf_rn(k2.y, P.hh, p.y), DIM == 3 ? __fmaf_rn(k2.z, P.hh, p.z) : 0.f};
-            const V3 k3c = wind_at<DIM, float>(P, a, E.t1, wb, wf);
-            const V3 k3 = sph ? sphere_(P, a.y, k3c) : k3c;
-            a = V3{__fmaf_rn(k3.x, P.h, p.x), __fmaf_rn(k3.y, P.h, p.y), DIM == 3 ? __fmaf_rn(k3.z, P.h, p.z) : 0.f};
-            const V3 k4c = wind_at<DIM, float>(P, a, E.t2, wb, wf);
-            const V3 k4 = sph ? sphere_(P, a.y, k4c) : k4c;
-            v.x = (((k1.x + 2.f * k2.x) + 2.f * k3.x) + k4.x) * P.sixth;
-            v.y = (((k1.y + 2.f * k2.y) + 2.f * k3.y) + k4.y) * P.sixth;
-            v.z = DIM == 3 ? (((k1.z + 2.f * k2.z) + 2.f * k3.z) + k4.z) * P.sixth : 0.f;
-        } else {
-            const V3 vc = wind_at<DIM, float>(P, p, E.t0, wb, wf);
-            v = sph ? sphere_(P, p.y, vc) : vc;
-        }
-        V3 dp{v.x * P.h, v.y * P.h, DIM == 3 ? v.z * P.h : 0.f};
-        if (P.reverse) { dp.x = -dp.x; dp.y = -dp.y; dp.z = -dp.z; }
-        V3 np;
-        np.x = P.reverse ? p.x - dp.x : p.x + dp.x;
-        np.y = P.reverse ? p.y - dp.y : p.y + dp.y;
-        np.z = DIM == 3 ? (P.reverse ? p.z - dp.z : p.z + dp.z) : 0.f;
-        int32_t abort = 0;
-        const float dp2 = dot3(dp, dp, DIM);
-        const int bm = DIM == 3 ? 0 : P.border_mode;
-        if (bm == 0) {
-            if (dp2 < 1e-9f) abort = 4;
-            else {
-                bool out = np.x - P.off[0] > P.dom[0] || np.x - P.off[0] < 0.f ||
-                           np.y - P.off[1] > P.dom[1] || np.y - P.off[1] < 0.f;
-                if (DIM == 3) out = out || np.z - P.off[2] > P.dom[2] || np.z - P.off[2] < 0.f;
-                if (out) abort = 2;
-            }
-        } else if (dp2 < 1e-9f) {
-            abort = 4;
-        } else {
-            const float ox = P.off[0], oy = P.off[1], DX = P.dom[0], DY = P.dom[1];
-            if (bm == 1) {
-                np.x = fmodf(np.x - ox + DX, DX) + ox;
-                if (np.y - oy > DY || np.y - oy < 0.f) abort = 2;
-            } else if (bm == 2) {
-                if (sph) {
-                    if (np.x - ox > DX || np.x - ox < 0.f || np.y - oy > DY || np.y - oy < 0.f) abort = 2;
-                } else {
-                    np.y = fmodf(np.y - oy + DY, DY) + oy;
-                    if (np.x - ox > DX || np.x - ox < 0.f) abort = 2;
-                }
-            } else {
-                if (sph) {
-                    const float nx_ = np.x - ox, ny_ = np.y - oy, px_ = p.x - ox, py_ = p.y - oy;
-                    if (ny_ < 0.f) {
-                        const float tx = (-py_) / (ny_ - py_) * (nx_ - px_) + px_;
-                        np.y = -ny_ + oy;
-                        np.x = fmodf(DX + 180.0f - nx_ + 2.f * tx, DX) + ox;
-                    } else if (ny_ >= DY) {
-                        const float tx = (DY - py_) / (ny_ - py_) * (nx_ - px_) + px_;
-                        np.y = (ny_ - DY) + oy;
-                        np.x = fmodf(DX + 180.0f - nx_ + 2.f * tx, DX) + ox;
-                    }
-                } else {
-                    np.y = fmodf(np.y - oy + DY, DY) + oy;
-                }
-                np.x = fmodf(np.x - ox + DX, DX) + ox;
-            }
-        }
-        st = abort;
-        if (abort != 0) alive = false;
-        else p = np;
-    }
-    if (valid && was_alive) {
-        P.status[i] = st;
-        P.px[i] = p.x;
-        P.py[i] = p.y;
-        if (DIM == 3) P.pz[i] = p.z;
-    }
-    const unsigned warp_steps = __reduce_add_sync(0xffffffffu, my_steps);
-    const unsigned alive_mask = __ballot_sync(0xffffffffu, valid && alive);
-    if ((threadIdx.x & 31) == 0) {
-        if (warp_steps) atomicAdd(&S->counters[0], (unsigned long long)warp_steps);
-        if (alive_mask) atomicAdd(&S->counters[1], (unsigned long long)__popc(alive_mask));
     }
 }
 
@@ -242,14 +132,21 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
         P.scale[d] = scale[d];
         P.inv_scale[d] = 1.0f / scale[d];
         P.off[d] = off[d];
+        P.noff[d] = -off[d];
         P.dom[d] = g[d] * scale[d];
     }
     P.nx = (int32_t)nx; P.ny = (int32_t)ny; P.nz = (int32_t)(dim == 3 ? nz : 1); P.dim = dim;
-    P.fn[0] = (float)P.nx; P.fn[1] = (float)P.ny; P.fn[2] = (float)P.nz;
+    const int64_t padded = (nx + 3) * (ny + 3) * (dim == 3 ? nz + 3 : 1);
+    P.wide = wide_grid(nx, ny, dim == 3 ? nz : 1) || padded > 0x7fffffffLL;
+    P.pnx = (int32_t)(nx + 3);
+    P.pnxy = P.wide ? 0 : (int32_t)((nx + 3) * (ny + 3));
+    clamp_cells(P, false);
     P.wind = wind_back;
     P.wind_stride = reinterpret_cast<const char *>(wind_front) - reinterpret_cast<const char *>(wind_back);
     P.px = px; P.py = py; P.pz = pz; P.status = status;
     P.n = n;
+    P.sched = S->sched;
+    P.counters = S->counters;
     P.s0 = 0;
     P.s1 = steps;
     P.h = h;
@@ -264,16 +161,13 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
     P.border_mode = dim == 2 ? s->border_mode : 0;
     P.reverse = s->reverse ? 1 : 0;
     P.sphere = dim == 2 && s->sphere_radius > 0.f;
-    const int threads = 256;
+    // the step kernel of the engine, reading the caller's two snapshots as ring slots (one thread
+    // per particle; 32-thread blocks spread a small set over the SMs)
+    const AdvanceFn fn = advance_f32(dim, s->integrator == 1, false, kernel_features(P));
+    int threads = 128;
+    while (threads > 32 && (n + threads - 1) / threads < 2 * 148) threads /= 2;
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (n + threads - 1) / threads);
-    const bool rk4 = s->integrator == 1;
-    if (dim == 3) {
-        if (rk4) advance_plain_kernel<3, true><<<blocks, threads, 0, st>>>(P, S);
-        else advance_plain_kernel<3, false><<<blocks, threads, 0, st>>>(P, S);
-    } else {
-        if (rk4) advance_plain_kernel<2, true><<<blocks, threads, 0, st>>>(P, S);
-        else advance_plain_kernel<2, false><<<blocks, threads, 0, st>>>(P, S);
-    }
+    fn<<<blocks, threads, 0, st>>>(P);
     if (cudaGetLastError() != cudaSuccess) return err(GR_ERR_RUNTIME, "ERROR < RUNTIME | launch failed >");
     if (particle_steps) {
         unsigned long long c = 0;

@@ -61,8 +61,9 @@ __global__ void pack_wind_kernel<__half>(const float *__restrict__ u, const floa
     }
 }
 
-// The window pair interleaves the two snapshots component by component (granite_kernels.cuh,
-// Store<Pair<...>>): from ring nodes b (back) and f (front) of storage type S to one pair node.
+// The window pair holds (u, v) of the back and of the front snapshot, then the two w
+// (granite_kernels.cuh, Store<Pair<...>>): from ring nodes b (back) and f (front) of storage type S
+// to one pair node.
 // float32: ring nodes float4 {u, v, w, 0} / float2 {u, v}; 16-bit: uint2 {(u, v), (w, 0)} /
 // one word (u, v), each word two 16-bit values (low half first).
 template <typename S> struct PairNode;
@@ -73,22 +74,22 @@ template <> struct PairNode<float> {
     using Out3 = uint4;   // written as two of these: 32 bytes
     using Out2 = float4;
     static __device__ __forceinline__ void pack3(const float4 &b, const float4 &f, float4 *o) {
-        o[0] = make_float4(b.x, f.x, b.y, f.y);
+        o[0] = make_float4(b.x, b.y, f.x, f.y);
         o[1] = make_float4(b.z, f.z, 0.f, 0.f);
     }
-    static __device__ __forceinline__ float4 pack2(const float2 &b, const float2 &f) { return make_float4(b.x, f.x, b.y, f.y); }
+    static __device__ __forceinline__ float4 pack2(const float2 &b, const float2 &f) { return make_float4(b.x, b.y, f.x, f.y); }
 };
 
 template <> struct PairNode<uint16_t> {
     using Ring3 = uint2;
     using Ring2 = unsigned;
     using Out2 = uint2;
-    // __byte_perm(x, y, 0x5410): the low halves of x and y; 0x7632: their high halves
+    // __byte_perm(x, y, 0x5410): the low halves of x and y
     static __device__ __forceinline__ uint4 pack3(const uint2 &b, const uint2 &f) {
-        return make_uint4(__byte_perm(b.x, f.x, 0x5410), __byte_perm(b.x, f.x, 0x7632), __byte_perm(b.y, f.y, 0x5410), 0u);
+        return make_uint4(b.x, f.x, __byte_perm(b.y, f.y, 0x5410), 0u);
     }
     static __device__ __forceinline__ uint2 pack2(unsigned b, unsigned f) {
-        return make_uint2(__byte_perm(b, f, 0x5410), __byte_perm(b, f, 0x7632));
+        return make_uint2(b, f);
     }
 };
 

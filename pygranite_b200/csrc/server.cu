@@ -245,8 +245,8 @@ __global__ void planar_pack_kernel(const float *__restrict__ u, const float *__r
 }
 
 // Two planar slots -> the window-pair layout the step kernel reads (granite_kernels.cuh,
-// Store<Pair<...>>): per node, component by component, back then front: {u_b, u_f, v_b, v_f,
-// w_b, w_f, 0, 0} (3D) or {u_b, u_f, v_b, v_f} (2D), vector stores.  3D pairs carry the zero
+// Store<Pair<...>>): per node (u, v) of the back and of the front snapshot, then w: {u_b, v_b, u_f,
+// v_f, w_b, w_f, 0, 0} (3D) or {u_b, v_b, u_f, v_f} (2D), vector stores.  3D pairs carry the zero
 // border of pair_pack_padded_kernel (pack_kernels.cuh): every padded node (nx + 3) x (ny + 3) x
 // (nz + 3) is written, zeros outside the grid; 2D pairs replicate the edge nodes.
 template <typename T>
@@ -264,7 +264,7 @@ __global__ void planar_pair_kernel(const T *__restrict__ b, const T *__restrict_
             alignas(sizeof(V)) T hi[4] = {zero, zero, zero, zero};
             if ((unsigned)x < (unsigned)nx && (unsigned)y < (unsigned)ny && (unsigned)z < (unsigned)nz) {
                 const int64_t i = ((int64_t)z * ny + y) * nx + x;
-                lo[0] = b[i]; lo[1] = f[i]; lo[2] = b[nodes + i]; lo[3] = f[nodes + i];
+                lo[0] = b[i]; lo[1] = b[nodes + i]; lo[2] = f[i]; lo[3] = f[nodes + i];
                 hi[0] = b[2 * nodes + i]; hi[1] = f[2 * nodes + i];
             }
             V *po = reinterpret_cast<V *>(out + 8 * (int64_t)o);
@@ -279,7 +279,7 @@ __global__ void planar_pair_kernel(const T *__restrict__ b, const T *__restrict_
     for (int32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total; o += gridDim.x * blockDim.x) {
         const int32_t x = min(max(o % pnx - 1, 0), nx - 1), y = min(max(o / pnx - 1, 0), ny - 1);
         const int64_t i = (int64_t)y * nx + x;
-        alignas(sizeof(V)) T q[4] = {b[i], f[i], b[nodes + i], f[nodes + i]};
+        alignas(sizeof(V)) T q[4] = {b[i], b[nodes + i], f[i], f[nodes + i]};
         *reinterpret_cast<V *>(out + 4 * (int64_t)o) = *reinterpret_cast<const V *>(q);
     }
 }
@@ -378,10 +378,10 @@ int allocate(gr_server *S, int64_t budget) {
         P.threads = 256;
         const int st = S->s.storage;
         // positions only (no curvature, volumes, constants, uplift, length abort, compensation):
-        // the lean variant unless 2D loop borders, sphere coordinates or 1/256 filter weights are on
+        // the lean variant, with 2D loop borders, sphere coordinates and 1/256 filter weights where on
         const bool lean = !(S->dim == 2 && (S->s.border_mode != 0 || S->s.sphere_radius > 0.f)) &&
                           !S->s.filter_weights;
-        const int ft = lean ? FT_LEAN : FT_GENERIC;
+        const int ft = lean ? FT_LEAN : FT_LEAN | FT_BORDER;
         P.fn = st == GR_STORE_BF16 ? advance_bf16(S->dim, p == 1, true, ft)
              : st == GR_STORE_F16 ? advance_f16(S->dim, p == 1, true, ft) : advance_f32(S->dim, p == 1, true, ft);
         cudaFuncAttributes fa{};
@@ -409,11 +409,12 @@ KParams pool_params(gr_server *S, Pool &P) {
     for (int d = 0; d < 3; ++d) {
         K.inv_scale[d] = S->inv_scale[d];
         K.off[d] = S->off[d];
+        K.noff[d] = -S->off[d];
         K.dom[d] = S->dom[d];
         K.scale[d] = S->scale[d];
     }
     K.nx = (int32_t)S->nx; K.ny = (int32_t)S->ny; K.nz = (int32_t)S->nz; K.dim = S->dim;
-    K.fn[0] = (float)S->nx; K.fn[1] = (float)S->ny; K.fn[2] = (float)S->nz;
+    clamp_cells(K, true);
     K.wind = S->ring.p;
     K.wind_stride = S->slot_stride;
     K.pair = S->pair.p;
