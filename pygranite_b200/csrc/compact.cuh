@@ -9,18 +9,24 @@
 //
 // Kernels are static: every translation unit that includes this header owns its instances.
 //
-// One pass: bin (key + warp-aggregated histogram) -> two-level exclusive scan -> rank
-// (destination of every source slot, written as a permutation) -> gather (coalesced writes
-// of every state array) -> commit (counts).
+// One pass is three launches: bin (key + warp-aggregated histogram), scan (offsets of the bins within
+// chunks) and move (the destination of every slot by a warp-aggregated ticket, its state written
+// there; the last block commits the counts).
 #pragma once
 
+#include <cuda_runtime.h>
+
+#include <algorithm>
 #include <cstdint>
 
 #include "granite_kernels.cuh"
+#include "host_util.h"
 
 namespace granite_b200 {
 
-constexpr int SCAN_CHUNK = 1024;   // bins per block of the first scan level
+constexpr int SCAN_THREADS = 1024, SCAN_CHUNK = 4 * SCAN_THREADS;   // bins per block of the scan
+constexpr int MAX_BINS = 1 << 20;                                    // bricks of a grid
+constexpr int MAX_CHUNKS = MAX_BINS / SCAN_CHUNK + 1;
 
 struct StateView {
     float *px, *py, *pz, *qx, *qy, *qz, *kx, *ky, *kz, *lx, *ly, *lz;
@@ -33,9 +39,10 @@ struct StateView {
 struct CompactParams {
     StateView src, dst, ret;
     int32_t *key;              // bin of each active slot
-    int32_t *hist;             // nbins + 1 counters -> offsets within the chunk -> cursors
-    int32_t *chunk;            // per-chunk sums -> chunk base offsets
-    int32_t *perm;             // destination slot -> source slot
+    int32_t *hist;             // counters of nbins + 1 bins (whole chunks), zero between passes
+    int32_t *cursor;           // next free place of each bin, within its chunk
+    int32_t *chunk;            // per-chunk sums
+    int32_t *ticket;           // blocks of the move done, zero between passes
     const int32_t *bintab;     // brick linear index -> Morton rank
     int32_t *n_act;            // active count (device)
     int32_t *n_new;            // live count after the pass (device)
@@ -64,7 +71,7 @@ __device__ __forceinline__ int32_t bin_of(const CompactParams &C, int64_t i) {
     return C.bintab[((iz / C.bz) * C.nby + iy / C.by) * C.nbx + ix / C.bx];
 }
 
-// key + histogram; lanes of a warp with the same key add once (sorted input: mostly one key per warp)
+// key + histogram (zero when the pass begins); lanes of a warp with the same key add once (sorted input: mostly one key per warp)
 static __global__ void bin_kernel(const __grid_constant__ CompactParams C) {
     const int64_t n = *C.n_act;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -79,14 +86,22 @@ static __global__ void bin_kernel(const __grid_constant__ CompactParams C) {
     }
 }
 
-// level 1: exclusive scan inside chunks of SCAN_CHUNK bins; chunk totals to C.chunk
-static __global__ void __launch_bounds__(SCAN_CHUNK) scan_chunks_kernel(const __grid_constant__ CompactParams C) {
-    __shared__ int32_t warp_sum[SCAN_CHUNK / 32];
-    const int nb = C.nbins + 1;
-    const int b = blockIdx.x * SCAN_CHUNK + threadIdx.x;
-    const int32_t v = b < nb ? C.hist[b] : 0;
+// Exclusive scan of the counters inside chunks of SCAN_CHUNK bins, one block each; leaves the
+// counters zero.  The chunk totals are scanned by every block of the move for itself (at most
+// MAX_CHUNKS of them), which is shorter than a second level here.  The last bin holds the retiring
+// slots, so its counter gives the live count.
+static __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const __grid_constant__ CompactParams C) {
+    __shared__ int32_t warp_sum[SCAN_THREADS / 32];
+    const int t = blockIdx.x * SCAN_THREADS + threadIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int32_t x = v;
+    const int4 v = reinterpret_cast<const int4 *>(C.hist)[t];
+    reinterpret_cast<int4 *>(C.hist)[t] = make_int4(0, 0, 0, 0);
+    if (t == C.nbins / 4) {
+        const int q = C.nbins & 3;
+        *C.n_new = *C.n_act - (q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w);
+    }
+    const int32_t own = v.x + v.y + v.z + v.w;
+    int32_t x = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -104,55 +119,9 @@ static __global__ void __launch_bounds__(SCAN_CHUNK) scan_chunks_kernel(const __
         warp_sum[lane] = s;   // inclusive over warps
     }
     __syncthreads();
-    const int32_t incl = x + (wid > 0 ? warp_sum[wid - 1] : 0);
-    if (b < nb) C.hist[b] = incl - v;
-    if (threadIdx.x == SCAN_CHUNK - 1) C.chunk[blockIdx.x] = incl;
-}
-
-// level 2: exclusive scan of the chunk totals (one block); n_new = start of the retired bin
-static __global__ void __launch_bounds__(1024) scan_top_kernel(const __grid_constant__ CompactParams C, int nchunks) {
-    __shared__ int32_t part[1024];
-    const int per = (nchunks + 1023) / 1024;
-    const int c0 = threadIdx.x * per, c1 = min(nchunks, c0 + per);
-    int32_t s = 0;
-    for (int c = c0; c < c1; ++c) s += C.chunk[c];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const int32_t y = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += y;
-        __syncthreads();
-    }
-    int32_t run = part[threadIdx.x] - s;
-    for (int c = c0; c < c1; ++c) {
-        const int32_t t = C.chunk[c];
-        C.chunk[c] = run;
-        run += t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) *C.n_new = C.hist[C.nbins] + C.chunk[C.nbins / SCAN_CHUNK];
-}
-
-// destination of every source slot, as a permutation dest -> source
-static __global__ void rank_kernel(const __grid_constant__ CompactParams C) {
-    const int64_t n = *C.n_act;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        const bool ok = i < n;
-        const int32_t k = ok ? C.key[i] : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, k);
-        const int lane = threadIdx.x & 31;
-        const int leader = __ffs(peers) - 1;
-        int32_t first = 0;
-        if (ok && lane == leader) first = atomicAdd(C.hist + k, __popc(peers));
-        first = __shfl_sync(0xffffffffu, first, leader);
-        if (ok) {
-            const int32_t d = C.chunk[k / SCAN_CHUNK] + first + __popc(peers & ((1u << lane) - 1));
-            C.perm[d] = (int32_t)i;
-        }
-    }
+    const int32_t before = x - own + (wid > 0 ? warp_sum[wid - 1] : 0);
+    reinterpret_cast<int4 *>(C.cursor)[t] = make_int4(before, before + v.x, before + v.x + v.y, before + v.x + v.y + v.z);
+    if (threadIdx.x == SCAN_THREADS - 1) C.chunk[blockIdx.x] = before + own;
 }
 
 __device__ __forceinline__ void move_live(const CompactParams &C, int64_t i, int64_t d) {
@@ -195,19 +164,88 @@ __device__ __forceinline__ void move_retired(const CompactParams &C, int64_t i, 
     R.retire[r] = C.rec_now;
 }
 
-// coalesced writes in destination order; the scattered reads hit L2
-static __global__ void gather_kernel(const __grid_constant__ CompactParams C) {
-    const int64_t n = *C.n_act, live = *C.n_new, base = *C.n_ret;
-    for (int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; d < n; d += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = C.perm[d];
-        if (d < live) move_live(C, i, d);
-        else move_retired(C, i, base + (d - live));
+// Destination of every slot, and its state moved there; the last block commits the counts.
+static __global__ void move_kernel(const __grid_constant__ CompactParams C) {
+    __shared__ int32_t chunk_base[MAX_CHUNKS];
+    const int64_t n = *C.n_act, live = *C.n_new, retired = *C.n_ret;
+    if (threadIdx.x < 32) {
+        const int chunks = (C.nbins + SCAN_CHUNK) / SCAN_CHUNK, per = (chunks + 31) / 32;
+        const int c0 = min(threadIdx.x * per, chunks), c1 = min(c0 + per, chunks);
+        int32_t own = 0;
+        for (int c = c0; c < c1; ++c) own += C.chunk[c];
+        int32_t x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)threadIdx.x >= o) x += y;
+        }
+        x -= own;
+        for (int c = c0; c < c1; ++c) {
+            chunk_base[c] = x;
+            x += C.chunk[c];
+        }
+    }
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int64_t i = base + threadIdx.x;
+        const bool ok = i < n;
+        const int32_t k = ok ? C.key[i] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, k);
+        const int lane = threadIdx.x & 31;
+        const int leader = __ffs(peers) - 1;
+        int32_t first = 0;
+        if (ok && lane == leader) first = atomicAdd(C.cursor + k, __popc(peers));
+        first = __shfl_sync(0xffffffffu, first, leader);
+        if (ok) {
+            const int64_t d = chunk_base[k / SCAN_CHUNK] + first + __popc(peers & ((1u << lane) - 1));
+            if (d < live) move_live(C, i, d);
+            else move_retired(C, i, retired + (d - live));
+        }
+    }
+    // every block has read the counts by the time the last one is done
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (atomicAdd(C.ticket, 1) == (int32_t)gridDim.x - 1) {
+            *C.ticket = 0;
+            if (!C.ret_by_id) *C.n_ret = (int32_t)(retired + (n - live));
+            *C.n_act = (int32_t)live;
+        }
     }
 }
 
-static __global__ void commit_kernel(const __grid_constant__ CompactParams C) {
-    *C.n_ret += *C.n_act - *C.n_new;
-    *C.n_act = *C.n_new;
+// Enqueues a pass over at most `n` active slots.
+static inline void launch_compaction(const CompactParams &C, int64_t n, cudaStream_t stream) {
+    const int threads = 256;
+    // grid-stride kernels over the device count: a few resident waves cover any count
+    const int blocks = std::min(grid_for(n, threads), 148 * 16);
+    bin_kernel<<<blocks, threads, 0, stream>>>(C);
+    scan_kernel<<<(C.nbins + SCAN_CHUNK) / SCAN_CHUNK, SCAN_THREADS, 0, stream>>>(C);
+    move_kernel<<<blocks, threads, 0, stream>>>(C);
 }
+constexpr int COMPACTION_LAUNCHES = 3;
+
+// Scratch of the passes: zeroed when it is allocated, left zero by every pass.
+struct CompactScratch {
+    DevBuf<int32_t> hist, cursor, chunk, ticket;
+    cudaError_t alloc(int nbins) {
+        if (ticket.p) return cudaSuccess;
+        const size_t chunks = ((size_t)nbins + SCAN_CHUNK) / SCAN_CHUNK, nb = chunks * SCAN_CHUNK;
+        cudaError_t e = hist.alloc(nb);
+        if (e == cudaSuccess) e = cursor.alloc(nb);
+        if (e == cudaSuccess) e = chunk.alloc(chunks);
+        if (e == cudaSuccess) e = cudaMemset(hist.p, 0, nb * sizeof(int32_t));
+        if (e == cudaSuccess) e = ticket.alloc(1);
+        if (e == cudaSuccess) e = cudaMemset(ticket.p, 0, sizeof(int32_t));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // the runs' streams do not wait for it
+        return e;
+    }
+    void set(CompactParams &C) const {
+        C.hist = hist.p;
+        C.cursor = cursor.p;
+        C.chunk = chunk.p;
+        C.ticket = ticket.p;
+    }
+};
 
 }  // namespace granite_b200

@@ -255,7 +255,8 @@ struct gr_engine {
     DevBuf<int32_t> d_counts;          // [0] live, [1] live after a pass, [2] retired
     int32_t *h_live = nullptr;         // pinned copy of the live count
     cudaEvent_t live_ready = nullptr;
-    DevBuf<int32_t> c_key, c_hist, c_bintab, c_chunk, c_perm;
+    DevBuf<int32_t> c_key, c_bintab;
+    CompactScratch c_scratch;
     int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
 
     DevBuf<float> hpos, hcurv, hvol, hcmp;   // record-major (KParams)
@@ -512,12 +513,18 @@ int ensure_particles(gr_engine *e) {
 
 extern "C" {
 
-// Automatic compaction (sort_interval < 0): a Morton re-sort every 8 launches measured best on
-// the 3D benchmark configuration (1e6 particles: 2.05e10 against 1.99e10 every 4 and 2.03e10
-// every 12); below 65,536 particles the passes cost more than the sorted warps save (the 2D
-// double gyre, 10,000 particles: 1.74e10 with them, 1.95e10 without).
-constexpr int kAutoSortInterval = 8;
-constexpr int64_t kAutoSortMin = 65536;
+// Automatic compaction (sort_interval < 0), from 65,536 particles: every 8 launches from 400,000
+// particles or with lifetimes (particles retire all the time), every 16 below, where a pass costs
+// more launches' worth of what it saves (1e6 x 300 steps: 8.38 ms every 8, 8.59 every 4, 8.76 sorted
+// once; 300,000 x 200 steps: 2.84, 2.91, 2.82; a batch of uneven lifetimes: 3.45, 3.53, 4.25 ms).
+// Below 65,536 particles one wave of warps holds the whole set and a launch's time is that of
+// its slowest warp: passes cost more than they save (70,000 x 200 steps: 1.02 ms without, 1.20 with).
+constexpr int kAutoSortInterval = 8, kAutoSortSmall = 16;
+constexpr int64_t kAutoSortMin = 65536, kAutoSortLarge = 400000;
+
+int auto_sort_interval(const gr_engine *e) {
+    return e->n >= kAutoSortLarge || e->has_life ? kAutoSortInterval : kAutoSortSmall;
+}
 
 void gr_settings_default(gr_settings *s) {
     std::memset(s, 0, sizeof *s);
@@ -531,7 +538,7 @@ void gr_settings_default(gr_settings *s) {
     s->offset_len = 3;
     s->save_interval = 1;
     s->maximum_simulation_time = 100.f;
-    s->sort_interval = -1;  // automatic: kAutoSortInterval launches from kAutoSortMin particles, else off
+    s->sort_interval = -1;  // automatic (auto_sort_interval) from kAutoSortMin particles, else off
 }
 
 const char *gr_last_error(void) { return g_last_error.c_str(); }
@@ -897,7 +904,7 @@ int alloc_state(gr_engine *e) {
             e->nbx = (int)((e->nx + e->bx - 1) / e->bx);
             e->nby = (int)((e->ny + e->by - 1) / e->by);
             e->nbz = (int)((e->nz + e->bz - 1) / e->bz);
-            if ((int64_t)e->nbx * e->nby * e->nbz <= (1 << 20) && e->nbx <= 1024 && e->nby <= 1024 && e->nbz <= 1024) break;
+            if ((int64_t)e->nbx * e->nby * e->nbz <= MAX_BINS && e->nbx <= 1024 && e->nby <= 1024 && e->nbz <= 1024) break;
             e->bx *= 2; e->by *= 2; if (e->dim == 3) e->bz *= 2;
         }
         e->nbins = e->nbx * e->nby * e->nbz;
@@ -922,9 +929,7 @@ int alloc_state(gr_engine *e) {
         CK(e->c_bintab.alloc(tab.size()));
         CK(cudaMemcpy(e->c_bintab.p, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
-    CK(e->c_hist.alloc((size_t)e->nbins + 1));
-    CK(e->c_chunk.alloc((size_t)(e->nbins + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK));
-    CK(e->c_perm.alloc(N));
+    CK(e->c_scratch.alloc(e->nbins));
     return GR_OK;
 }
 
@@ -1273,9 +1278,7 @@ int compact_pass(gr_engine *e, int32_t rec_now, int32_t k_end, bool graph) {
     if (!e->has_life) C.src.life = C.dst.life = nullptr;
     C.ret.life = nullptr;
     C.key = e->c_key.p;
-    C.hist = e->c_hist.p;
-    C.chunk = e->c_chunk.p;
-    C.perm = e->c_perm.p;
+    e->c_scratch.set(C);
     C.bintab = e->c_bintab.p;
     C.n_act = e->d_counts.p;
     C.n_new = e->d_counts.p + 1;
@@ -1297,24 +1300,14 @@ int compact_pass(gr_engine *e, int32_t rec_now, int32_t k_end, bool graph) {
     C.curv_ind = cm == 3;
     C.rec_now = rec_now;
     C.k_end = k_end;
-    const int threads = 256;
-    // grid-stride kernels over the device live count: a few resident waves cover any count
-    const int blocks = std::min(grid_for(N, threads), 148 * 16);
-    const int nchunks = (e->nbins + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    CK(cudaMemsetAsync(e->c_hist.p, 0, ((size_t)e->nbins + 1) * sizeof(int32_t), e->cs));
-    bin_kernel<<<blocks, threads, 0, e->cs>>>(C);
-    scan_chunks_kernel<<<nchunks, SCAN_CHUNK, 0, e->cs>>>(C);
-    scan_top_kernel<<<1, 1024, 0, e->cs>>>(C, nchunks);
-    rank_kernel<<<blocks, threads, 0, e->cs>>>(C);
-    gather_kernel<<<blocks, threads, 0, e->cs>>>(C);
-    commit_kernel<<<1, 1, 0, e->cs>>>(C);
+    launch_compaction(C, N, e->cs);
     CK(cudaGetLastError());
     if (!graph) {
         CK(cudaMemcpyAsync(e->h_live, e->d_counts.p, sizeof(int32_t), cudaMemcpyDeviceToHost, e->cs));
         CK(cudaEventRecord(e->live_ready, e->cs));
     }
     e->cur = 1 - e->cur;
-    e->stats.aux_launches += 6;
+    e->stats.aux_launches += COMPACTION_LAUNCHES;
     return GR_OK;
 }
 
@@ -1558,25 +1551,44 @@ int launch_deferred_extras(RunCtx &r, int64_t save_step, int64_t k_end, bool all
     return GR_OK;
 }
 
-// After a launch that ended before step k_end: maybe retire / re-sort (compact.cuh).
-int after_launch(RunCtx &r, int64_t k_end) {
+// A compaction after step k_end; the launches that follow read the new live prefix.
+int sort_now(RunCtx &r, int64_t k_end) {
     gr_engine *e = r.e;
-    const RunPlan &R = *r.R;
-    if (!e->compacting || k_end >= R.nsteps) return 0;
-    if (++r.since_sort < (e->s.sort_interval > 0 ? e->s.sort_interval : kAutoSortInterval)) return 0;
     r.since_sort = 0;
-    if (r.defer) {   // retiring particles take their final values along
-        const int q = launch_deferred_extras(r, -1, k_end, false);
-        if (q) return q;
-    }
-    int q = compact_pass(e, R.rec_before[k_end], (int32_t)k_end, R.graph);
+    const int q = compact_pass(e, r.R->rec_before[k_end], (int32_t)k_end, r.R->graph);
     if (q) return q;
     const int32_t gs = r.P.grid_stride;
     r.P = make_params(e);
     r.P.grid_stride = gs;
     // live count of the last completed pass: an upper bound of the current one
-    if (!R.graph) r.P.n = std::max<int64_t>(1, *(volatile int32_t *)e->h_live);
+    if (!r.R->graph) r.P.n = std::max<int64_t>(1, *(volatile int32_t *)e->h_live);
     return 0;
+}
+
+// Seeds come in any order: before the first step they are sorted like the live set is later, so
+// the first launches gather as the others do (unsorted, the first eight launches of the
+// 1e6-particle plain configuration took 340 us each against 225 us).  What a pass saves grows with
+// the samples that follow and is four times as much in 3D; it breaks even at about 40 RK4 steps of
+// 100,000 particles in 3D, 100 in 2D, against the line's 50 and 200.
+constexpr int64_t kSortWork = 20000000;
+int sort_seeds(RunCtx &r) {
+    const gr_engine *e = r.e;
+    const int64_t weight = (e->dim == 3 ? 4 : 1) * (e->s.integrator == 1 ? 4 : 1);
+    if (!e->compacting || e->n * r.R->nsteps < 4 * kSortWork / weight) return 0;
+    return sort_now(r, 0);
+}
+
+// After a launch that ended before step k_end: maybe retire / re-sort (compact.cuh).
+int after_launch(RunCtx &r, int64_t k_end) {
+    gr_engine *e = r.e;
+    const RunPlan &R = *r.R;
+    if (!e->compacting || k_end >= R.nsteps) return 0;
+    if (++r.since_sort < (e->s.sort_interval > 0 ? e->s.sort_interval : auto_sort_interval(e))) return 0;
+    if (r.defer) {   // retiring particles take their final values along
+        const int q = launch_deferred_extras(r, -1, k_end, false);
+        if (q) return q;
+    }
+    return sort_now(r, k_end);
 }
 
 // Steps [b, t): returns 1 when MinimumAliveParticles stopped the run.
@@ -1972,6 +1984,8 @@ extern "C" int gr_run(gr_engine *e, gr_loader_fn loader, void *user) {
     for (int k = 0; k < e->K; ++k)
         if (e->wind_holds[k] >= 0 || e->vol_holds[k] >= 0 || e->cons_holds[k] >= 0 || e->lift_holds[k] >= 0)
             CK(cudaStreamWaitEvent(e->cs, e->slot_ready[k], 0));
+    rc = sort_seeds(r);
+    if (rc) return rc;
 
     const int64_t nwin = R.nwin;
     const int64_t gmax = std::max(1, e->K - 1);
@@ -2063,6 +2077,8 @@ int graph_enqueue(gr_engine *e) {
     if (rc) return rc;
     RunCtx r;
     rc = make_ctx(e, R, r);
+    if (rc) return rc;
+    rc = sort_seeds(r);
     if (rc) return rc;
     rc = launch_range(r, 0, R.nsteps);
     if (rc < 0) return rc;

@@ -101,7 +101,7 @@ struct Pool {
     int64_t cap = 0;                   // particle slots
     int64_t in_flight = 0;             // particles of active requests (upper bound of the live count)
     DevBuf<int32_t> counts;            // [0] live, [1] live after a pass, [2] retired
-    DevBuf<int32_t> key, perm;
+    DevBuf<int32_t> key;
     AdvanceFn fn = nullptr;
     int threads = 256;
     int64_t grid = 1;
@@ -162,7 +162,8 @@ struct gr_server {
     };
     Stage stage[2];
     int stage_next = 0;
-    DevBuf<int32_t> bintab, hist, chunk;
+    DevBuf<int32_t> bintab;
+    CompactScratch scratch;
     int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
     DevBuf<unsigned long long> counters;   // [0] particle-steps
     cudaStream_t cs = nullptr, xs = nullptr;
@@ -326,7 +327,7 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx) {
         S->nbx = (int)((S->nx + S->bx - 1) / S->bx);
         S->nby = (int)((S->ny + S->by - 1) / S->by);
         S->nbz = (int)((S->nz + S->bz - 1) / S->bz);
-        if ((int64_t)S->nbx * S->nby * S->nbz <= (1 << 20) && S->nbx <= 1024 && S->nby <= 1024 && S->nbz <= 1024) break;
+        if ((int64_t)S->nbx * S->nby * S->nbz <= MAX_BINS && S->nbx <= 1024 && S->nby <= 1024 && S->nbz <= 1024) break;
         S->bx *= 2; S->by *= 2; if (S->dim == 3) S->bz *= 2;
     }
     S->nbins = S->nbx * S->nby * S->nbz;
@@ -350,14 +351,13 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx) {
     for (int32_t r = 0; r < S->nbins; ++r) tab[codes[r].second] = r;
     SK(S->bintab.alloc(tab.size()));
     SK(cudaMemcpy(S->bintab.p, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    SK(S->hist.alloc((size_t)S->nbins + 1));
-    SK(S->chunk.alloc((size_t)(S->nbins + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK));
+    SK(S->scratch.alloc(S->nbins));
     return GR_OK;
 }
 
 // Pools, result arena and staging sized from the HBM budget.
 int allocate(gr_server *S, int64_t budget) {
-    // per pool slot: 7 arrays x 2 buffers + key + perm = 64 bytes; per arena slot 16 bytes
+    // per pool slot: 7 arrays x 2 buffers + key and a reserve = 64 bytes; per arena slot 16 bytes
     const int64_t per = 2 * 64 + 2 * 16;
     int64_t cap = budget / per;
     cap = std::min<int64_t>(cap, (int64_t(1) << 31) / 2 - 1);
@@ -371,7 +371,6 @@ int allocate(gr_server *S, int64_t budget) {
             SK(a.status.alloc(cap)); SK(a.id.alloc(cap)); SK(a.life.alloc(cap)); SK(a.birth.alloc(cap));
         }
         SK(P.key.alloc(cap));
-        SK(P.perm.alloc(cap));
         SK(P.counts.alloc(4));
         init_pool_kernel<<<1, 1, 0, S->cs>>>(P.counts.p);
         SK(cudaGetLastError());
@@ -462,9 +461,7 @@ int compact_pool(gr_server *S, Pool &P, int32_t k_end) {
     C.ret = R;
     C.ret_by_id = 1;
     C.key = P.key.p;
-    C.hist = S->hist.p;
-    C.chunk = S->chunk.p;
-    C.perm = P.perm.p;
+    S->scratch.set(C);
     C.bintab = S->bintab.p;
     C.n_act = P.counts.p;
     C.n_new = P.counts.p + 1;
@@ -476,18 +473,7 @@ int compact_pool(gr_server *S, Pool &P, int32_t k_end) {
     C.nx = (int32_t)S->nx; C.ny = (int32_t)S->ny; C.nz = (int32_t)S->nz; C.dim = S->dim;
     C.bx = S->bx; C.by = S->by; C.bz = S->bz; C.nbx = S->nbx; C.nby = S->nby; C.nbz = S->nbz; C.nbins = S->nbins;
     C.k_end = k_end;
-    const int threads = 256;
-    const int blocks = std::min(grid_for(std::max<int64_t>(1, P.in_flight), threads), 148 * 16);
-    // retired particles go to their result slots: the retired count is not needed
-    SK(cudaMemsetAsync(P.counts.p + 2, 0, sizeof(int32_t), S->cs));
-    const int nchunks = (S->nbins + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    SK(cudaMemsetAsync(S->hist.p, 0, ((size_t)S->nbins + 1) * sizeof(int32_t), S->cs));
-    bin_kernel<<<blocks, threads, 0, S->cs>>>(C);
-    scan_chunks_kernel<<<nchunks, SCAN_CHUNK, 0, S->cs>>>(C);
-    scan_top_kernel<<<1, 1024, 0, S->cs>>>(C, nchunks);
-    rank_kernel<<<blocks, threads, 0, S->cs>>>(C);
-    gather_kernel<<<blocks, threads, 0, S->cs>>>(C);
-    commit_kernel<<<1, 1, 0, S->cs>>>(C);
+    launch_compaction(C, std::max<int64_t>(1, P.in_flight), S->cs);   // retired particles go to their result slots
     SK(cudaGetLastError());
     P.cur = 1 - P.cur;
     return GR_OK;
