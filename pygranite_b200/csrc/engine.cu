@@ -2009,6 +2009,12 @@ extern "C" int gr_run(gr_engine *e, gr_loader_fn loader, void *user) {
         const int q = launch_range(r, R.sched.window_begin[w], R.sched.window_begin[g_end]);
         if (q < 0) return q;
         windows_run = g_end;
+        // pending values read these windows' snapshots: a particle that stops at the next window's
+        // first step keeps the values of this one's last
+        if (r.defer && (s.volume_mode == 2 || s.constants_mode == 2)) {
+            rc = launch_deferred_extras(r, -1, R.sched.window_begin[g_end], true);
+            if (rc) return rc;
+        }
         // slots read by this group become free once it has run
         for (int64_t k = w; k <= g_end && k - w < e->K; ++k) {
             CK(cudaEventRecord(e->slot_free[k % e->K], e->cs));
