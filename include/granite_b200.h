@@ -76,9 +76,10 @@ typedef struct gr_settings {
                                       kernel's launch bound (128 for the float32 3D window-pair
                                       kernel, 256 for the others) */
     int32_t device;                /* CUDA device ordinal */
-    int32_t layout;                /* wind layout read by the step kernel: 0 = window pairs when the
-                                      windfield is dynamic (one load returns the back and the front
-                                      snapshot), 1 = the ring slots directly */
+    int32_t layout;                /* wind layout read by the step kernel: 0 = automatic: window pairs
+                                      when the windfield is dynamic (one load returns the back and
+                                      the front snapshot), the ring slots where few particles share a
+                                      large grid; 1 = the ring slots directly */
     int32_t grid_waves;            /* graph runs: resident waves of step-kernel blocks in the
                                       persistent grid (each thread walks live particles with a
                                       grid stride); 0 = 1 */

@@ -522,6 +522,9 @@ extern "C" {
 constexpr int kAutoSortInterval = 8, kAutoSortSmall = 16;
 constexpr int64_t kAutoSortMin = 65536, kAutoSortLarge = 400000;
 
+// Launches and passes placed by the engine (no setting says where).
+bool auto_launches(const gr_engine *e) { return e->s.sort_interval < 0 && e->s.steps_per_launch <= 0; }
+
 int auto_sort_interval(const gr_engine *e) {
     return e->n >= kAutoSortLarge || e->has_life ? kAutoSortInterval : kAutoSortSmall;
 }
@@ -585,9 +588,9 @@ int gr_create(const gr_settings *settings, gr_engine **out) {
     e->vol_holds.assign(e->K, -1);
     e->cons_holds.assign(e->K, -1);
     e->lift_holds.assign(e->K, -1);
-    CK(e->counters.alloc(4));
+    CK(e->counters.alloc(1));
     // small page-locked words from the host cache: no page-locking per engine
-    if (gr_host_alloc(4 * sizeof(unsigned long long), reinterpret_cast<void **>(&e->h_counters)) != GR_OK)
+    if (gr_host_alloc(sizeof(unsigned long long), reinterpret_cast<void **>(&e->h_counters)) != GR_OK)
         return GR_ERR_RUNTIME;
     *out = e.release();
     return GR_OK;
@@ -856,6 +859,7 @@ struct RunPlan {
     std::vector<int64_t> save_next;    // first save step >= k (nsteps if none)
     int64_t spl = 0;                   // steps per launch
     bool graph = false;                // fixed launch shapes and no host reads (graph capture)
+    bool small_set = false;            // few particles for the grid (small_set)
 };
 
 namespace {
@@ -970,7 +974,7 @@ int reset_state(gr_engine *e) {
     seed_record_kernel<<<grid_for(n * e->dim, threads), threads, 0, e->cs>>>(e->seeds.p, n, e->dim, e->hpos.p);
     CK(cudaGetLastError());
     if (e->ret_rec.p) CK(cudaMemsetAsync(e->ret_rec.p, 0x7f, (size_t)n * sizeof(int32_t), e->cs));   // never retired
-    CK(cudaMemsetAsync(e->counters.p, 0, 4 * sizeof(unsigned long long), e->cs));
+    CK(cudaMemsetAsync(e->counters.p, 0, sizeof(unsigned long long), e->cs));
     if (e->compacting) *e->h_live = (int32_t)n;
     e->stats.aux_launches += 3;
     return GR_OK;
@@ -1052,6 +1056,31 @@ int pair_elem(const gr_engine *e) {
 // pair_pack_edge2_kernel).
 size_t pair_bytes(const gr_engine *e) {
     return (size_t)padded_pair_nodes(e->dim, e->nx, e->ny, e->nz) * 2 * pair_elem(e);
+}
+
+// Few particles for the grid: they read the ring slots directly (fill_ring: 16 loads a cell instead of
+// 8) instead of having every window's pair packed first, and one launch runs until the next pass
+// or the end of the resident windows, with the values of volumes and expressions evaluated in it.
+// A window costs a launch (about 10 us of launch, first gathers and tail; 18 us with the deferred
+// kernel) and half of its pack's time that does not hide behind the launch before; the direct reads
+// cost a longer chain per step, 0.5 us in 3D and 0.18 us in 2D, and 8.6 / 3 us per million
+// particles and step (25 us with volumes or expressions, whose evaluation costs the deferred kernel
+// its lower register count).  Measured, ring against pair, ms of device time a run:
+// 192 x 192 x 64 nodes, 200 steps, 10 a window: positions of 70,000 particles 0.87 / 1.10, 150,000
+// 1.44 / 1.46, 300,000 2.18 / 2.01, with a volume, an expression and records 10,000 0.91 / 1.37, 70,000
+// 1.30 / 1.59, 150,000 2.29 / 2.03; 512 x 512 x 96 bf16, 777,777 x 100 steps 2.84 / 3.73; 24 x 24 x 16,
+// 100 steps, 50,000 0.26 / 0.28, 150,000 0.61 / 0.52; 2D 1024 x 512 nodes, 200 steps, 150,000 0.58 /
+// 0.63, 400,000 1.16 / 1.08; 256 x 128, 10,000 x 1024 Euler steps, 128 a window, 0.58 / 0.42.  Where the
+// settings place the launches, only the pack is saved.
+bool small_set(const gr_engine *e, const RunPlan &R) {
+    if (R.nsteps == 0 || !e->wind_dynamic) return false;
+    const gr_settings &s = e->s;
+    const bool extras = (s.volume_mode != 0 && e->nvol > 0) || e->nexpr > 0;
+    const double launch = s.sort_interval > 0 || s.steps_per_launch > 0 ? 0.0 : extras ? 18.0 : 10.0;
+    const double pack = (double)e->nodes * 4 * pair_elem(e) / 5e6;   // us at 5 TB/s
+    const double steps = (double)R.nsteps / (double)R.nwin;          // a window
+    const double chain = e->dim == 3 ? 0.5 : 0.18, gathers = extras ? 25.0 : e->dim == 3 ? 8.6 : 3.0;
+    return steps * (chain + gathers * 1e-6 * (double)e->n) < launch + 0.5 * pack;
 }
 
 // Validation, schedule, device schedule and programs, state and history buffers.
@@ -1171,13 +1200,16 @@ int run_prepare(gr_engine *e, RunPlan &R, bool graph) {
     for (int64_t k = 0; k < R.nsteps; ++k) R.rec_before[k + 1] = R.rec_before[k] + (R.sched.steps[k].save ? 1 : 0);
     R.save_next.assign((size_t)R.nsteps + 1, R.nsteps);
     for (int64_t k = R.nsteps - 1; k >= 0; --k) R.save_next[k] = R.sched.steps[k].save ? k : R.save_next[k + 1];
-    R.spl = s.steps_per_launch > 0 ? s.steps_per_launch : (int64_t)1 << 40;
-    if (e->compacting && s.steps_per_launch <= 0 && R.nwin > 0)
-        R.spl = std::max<int64_t>(1, R.sched.window_begin[1] - R.sched.window_begin[0]);   // one window per launch
-
     // window-pair layout: one load per corner returns both snapshots; launches never cross a
     // window boundary then
-    e->use_pair = e->wind_dynamic && s.layout == 0 && !wide_grid(e->nx, e->ny, e->nz);
+    R.small_set = small_set(e, R);
+    e->use_pair = e->wind_dynamic && s.layout == 0 && !wide_grid(e->nx, e->ny, e->nz) && !R.small_set;
+    R.spl = s.steps_per_launch > 0 ? s.steps_per_launch : (int64_t)1 << 40;
+    if (e->compacting && s.steps_per_launch <= 0 && R.nwin > 0) {
+        // compacting runs launch window by window, or from pass to pass
+        const int64_t windows = auto_launches(e) ? std::min<int64_t>(R.nwin, auto_sort_interval(e)) : 1;
+        R.spl = std::max<int64_t>(1, R.sched.window_begin[windows]);
+    }
     {
         const int rc = settle_pairs(e);
         if (rc) return rc;
@@ -1219,7 +1251,8 @@ KParams make_params(gr_engine *e) {
     }
     P.nx = (int32_t)e->nx; P.ny = (int32_t)e->ny; P.nz = (int32_t)e->nz; P.dim = e->dim;
     P.wide = wide_grid(e->nx, e->ny, e->nz);
-    clamp_cells(P, e->use_pair);
+    // the ring slots in place of a pair keep the pair's clamp
+    clamp_cells(P, e->wind_dynamic && e->s.layout == 0 && !P.wide);
     P.pnx = (int32_t)(e->nx + 3); P.pnxy = (int32_t)((e->nx + 3) * (e->ny + 3));
     P.wind = e->wind.p; P.wind_stride = e->wind_stride;
     P.vol = e->vol.p; P.vol_plane = e->nodes;
@@ -1446,9 +1479,9 @@ int make_ctx(gr_engine *e, RunPlan &R, RunCtx &r) {
     r.e = e;
     r.R = &R;
     r.P = make_params(e);
-    // deferred volume / expression values: not in graph runs (fixed launch shapes) and only
-    // where a lean variant applies
-    r.defer = !R.graph && r.P.vlast != nullptr && (kernel_features(r.P, true) & FT_DEFER) != 0;
+    // deferred volume / expression values: not in graph runs (fixed launch shapes), not in small
+    // sets (small_set) and only where a lean variant applies
+    r.defer = !R.graph && !R.small_set && r.P.vlast != nullptr && (kernel_features(r.P, true) & FT_DEFER) != 0;
     // resolved per run (a cache lookup after the first compile): expressions and settings may
     // change between runs
     e->jit_extras = nullptr;
@@ -1496,7 +1529,6 @@ int launch_steps(RunCtx &r, int64_t s0, int64_t s1, int64_t window) {
         e->stats.launches++;
         return GR_OK;
     }
-    CK(cudaMemsetAsync(e->counters.p + 1, 0, sizeof(unsigned long long), e->cs));
     cudaEvent_t a = pool_event(e, r.ev_used++), b = pool_event(e, r.ev_used++);
     CK(cudaEventRecord(a, e->cs));
     // one thread per particle: the step kernel is not grid-strided
@@ -1578,12 +1610,14 @@ int sort_seeds(RunCtx &r) {
     return sort_now(r, 0);
 }
 
-// After a launch that ended before step k_end: maybe retire / re-sort (compact.cuh).
-int after_launch(RunCtx &r, int64_t k_end) {
+// After a launch of steps [k, k_end): maybe retire / re-sort (compact.cuh).
+int after_launch(RunCtx &r, int64_t k, int64_t k_end) {
     gr_engine *e = r.e;
     const RunPlan &R = *r.R;
     if (!e->compacting || k_end >= R.nsteps) return 0;
-    if (++r.since_sort < (e->s.sort_interval > 0 ? e->s.sort_interval : auto_sort_interval(e))) return 0;
+    // automatic passes count windows (a launch may span several), the settings' interval launches
+    r.since_sort += auto_launches(e) ? R.sched.steps[k_end - 1].window - R.sched.steps[k].window + 1 : 1;
+    if (r.since_sort < (e->s.sort_interval > 0 ? e->s.sort_interval : auto_sort_interval(e))) return 0;
     if (r.defer) {   // retiring particles take their final values along
         const int q = launch_deferred_extras(r, -1, k_end, false);
         if (q) return q;
@@ -1646,7 +1680,7 @@ int launch_range(RunCtx &r, int64_t b, int64_t t) {
             r.alive_known = alive_after(L - 1);
             r.ps_known = e->h_counters[0];
             r.executed += L;
-            q = after_launch(r, k1);
+            q = after_launch(r, k, k1);
             if (q) return q;
             k = k1;
         }
@@ -1664,7 +1698,7 @@ int launch_range(RunCtx &r, int64_t b, int64_t t) {
             q = launch_deferred_extras(r, R.save_next[k], k1, false);
             if (q) return q;
         }
-        q = after_launch(r, k1);
+        q = after_launch(r, k, k1);
         if (q) return q;
         k = k1;
     }
@@ -1912,7 +1946,7 @@ int run_tail(RunCtx &r, RecordCounts &c) {
 int run_collect(gr_engine *e, const RunPlan &R, int64_t executed, int64_t windows_run, const RecordCounts &c,
                 size_t ev_used) {
     const gr_settings &s = e->s;
-    CK(cudaMemcpyAsync(e->h_counters, e->counters.p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->cs));
+    CK(cudaMemcpyAsync(e->h_counters, e->counters.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->cs));
     CK(cudaStreamSynchronize(e->cs));
     if (ev_used >= 2) {
         float ms = 0.f;

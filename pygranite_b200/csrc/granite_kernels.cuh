@@ -129,7 +129,7 @@ struct KParams {
     int32_t nvol, ncon, nexpr;
     int32_t filter_weights;       // 1: interpolation fractions rounded to the nearest 1/256
     const Program *prog;          // [4]
-    unsigned long long *counters; // [0] particle-steps, [1] alive at the end of the launch
+    unsigned long long *counters; // [0] particle-steps
     unsigned *alive_at;           // if set: [step - s0][32 shards] particles alive after each step
 };
 
@@ -839,7 +839,7 @@ constexpr int GR_ADV_MIN_BLOCKS = 2, GR_F32_BLOCKS = 4, GR_LIGHT_BLOCKS = 5;   /
 // Advances the particle in slot i through steps [s0, s1) (or until its lifetime ends).
 template <int DIM, bool RK4, typename W, int FT>
 __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t i, const int64_t n_live,
-                                                 unsigned long long &steps_acc, unsigned &alive_acc) {
+                                                 unsigned long long &steps_acc) {
     // options: runtime values in the generic variant; in a lean variant (FT_LEAN) the ones the
     // host checked are off, and curvature / extras are the variant's compile-time choice
     constexpr bool LEAN = (FT & FT_LEAN) != 0;
@@ -1145,7 +1145,6 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     }
 
     steps_acc += my_steps;
-    alive_acc += (valid && alive) ? 1u : 0u;
 }
 
 // One thread per particle, or (P.grid_stride) a persistent grid striding over the live
@@ -1174,21 +1173,16 @@ __global__ void __launch_bounds__(AdvBounds<DIM, W, FT>::threads, AdvBounds<DIM,
     advance_kernel(const __grid_constant__ KParams P) {
     const int64_t n_live = P.n_dev ? (int64_t)*P.n_dev : P.n;
     unsigned long long steps = 0;
-    unsigned alive = 0;
     if (P.grid_stride) {
         const int64_t stride = (int64_t)gridDim.x * blockDim.x;
         for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_live; base += stride)
-            advance_particle<DIM, RK4, W, FT>(P, base + threadIdx.x, n_live, steps, alive);
+            advance_particle<DIM, RK4, W, FT>(P, base + threadIdx.x, n_live, steps);
     } else {
-        advance_particle<DIM, RK4, W, FT>(P, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_live, steps, alive);
+        advance_particle<DIM, RK4, W, FT>(P, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_live, steps);
     }
-    // counters: particle-steps and the alive count after the launch (warp-aggregated)
+    // particle-steps, warp-aggregated
     const unsigned long long warp_steps = __reduce_add_sync(0xffffffffu, (unsigned)steps);
-    const unsigned warp_alive = __reduce_add_sync(0xffffffffu, alive);
-    if ((threadIdx.x & 31) == 0) {
-        if (warp_steps) atomicAdd(P.counters, warp_steps);
-        if (warp_alive) atomicAdd(P.counters + 1, (unsigned long long)warp_alive);
-    }
+    if ((threadIdx.x & 31) == 0 && warp_steps) atomicAdd(P.counters, warp_steps);
 }
 
 }  // namespace granite_b200

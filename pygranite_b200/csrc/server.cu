@@ -396,8 +396,8 @@ int allocate(gr_server *S, int64_t budget) {
     if (S->dim == 3) SK(S->res_pz.alloc(S->arena_cap));
     SK(S->res_status.alloc(S->arena_cap));
     S->arena.reset(S->arena_cap);
-    SK(S->counters.alloc(4));
-    SK(cudaMemsetAsync(S->counters.p, 0, 4 * sizeof(unsigned long long), S->cs));
+    SK(S->counters.alloc(1));
+    SK(cudaMemsetAsync(S->counters.p, 0, sizeof(unsigned long long), S->cs));
     S->st.capacity_particles = cap;
     return GR_OK;
 }
