@@ -107,20 +107,23 @@ struct RowFill {
 // Record-major history rows -> particle-major rows: records [r0, r1) of particles [p0, p1), D
 // floats each, from src[(r * n + p) * D + d] to dst[((p - p0) * nr + r - r0) * D + d], rows of nr
 // records (the layout of TrajectorySet's accessors, TrajectorySet.cpp:110-160), with the frozen
-// values of retired particles substituted (RowFill).  A 32-record x 32-particle tile through
-// shared memory: reads run along a record row, writes along a particle's records, both coalesced.
-template <int D>
+// values of retired particles substituted (RowFill).  A tile of TR records x 1024 / TR particles
+// through shared memory: reads run along a record row, writes along a particle's records, both
+// coalesced.  TR follows the records asked for: one row of 777,777 particles (the final positions)
+// took 103 us in tiles of 32 records, 31 of them empty, and takes 9 us now.
+template <int D, int TR>
 __global__ void __launch_bounds__(256) records_to_rows_kernel(const float *__restrict__ src, int64_t n, int32_t r0,
                                                               int32_t r1, int64_t p0, int64_t p1,
                                                               float *__restrict__ dst, int32_t nr, RowFill fill) {
-    __shared__ float tile[32][32 * D + 1];
-    __shared__ int32_t ret[32];
-    const int32_t rt = r0 + (int32_t)blockIdx.y * 32;
-    const int64_t pt = p0 + (int64_t)blockIdx.x * 32;
-    if (threadIdx.x < 32) ret[threadIdx.x] = (fill.ret && pt + threadIdx.x < p1) ? fill.ret[pt + threadIdx.x] : 0x7fffffff;
+    constexpr int TP = 1024 / TR;
+    __shared__ float tile[TR][TP * D + 1];
+    __shared__ int32_t ret[TP];
+    const int32_t rt = r0 + (int32_t)blockIdx.y * TR;
+    const int64_t pt = p0 + (int64_t)blockIdx.x * TP;
+    for (int q = threadIdx.x; q < TP; q += blockDim.x) ret[q] = (fill.ret && pt + q < p1) ? fill.ret[pt + q] : 0x7fffffff;
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * 32 * D; idx += blockDim.x) {
-        const int rr = idx / (32 * D), f = idx - rr * (32 * D);
+    for (int idx = threadIdx.x; idx < TR * TP * D; idx += blockDim.x) {
+        const int rr = idx / (TP * D), f = idx - rr * (TP * D);
         const int q = f / D;
         if (rt + rr < r1 && pt + q < p1) {
             const int32_t r = rt + rr;
@@ -129,8 +132,8 @@ __global__ void __launch_bounds__(256) records_to_rows_kernel(const float *__res
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * 32 * D; idx += blockDim.x) {
-        const int q = idx / (32 * D), g = idx - q * (32 * D);
+    for (int idx = threadIdx.x; idx < TR * TP * D; idx += blockDim.x) {
+        const int q = idx / (TR * D), g = idx - q * (TR * D);
         const int rr = g / D, d = g - rr * D;
         if (rt + rr < r1 && pt + q < p1)
             dst[((pt + q - p0) * nr + (rt + rr - r0)) * D + d] = tile[rr][q * D + d];
@@ -227,7 +230,6 @@ struct gr_engine {
     PinnedBuf pin[2];
     int pin_next = 0;
     cudaEvent_t upload_done = nullptr; // end of a DMA straight from a caller's page-locked buffer
-    PinnedBuf bounce[2];               // pinned staging of result copies
 
     // expressions
     Program progs[GR_MAX_EXPR]{};
@@ -260,7 +262,10 @@ struct gr_engine {
     int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
 
     DevBuf<float> hpos, hcurv, hvol, hcmp;   // record-major (KParams)
-    DevBuf<float> stage, sstage;             // particle-major chunks for the fetch / the streaming
+    DevBuf<float> stage[2], sstage;          // particle-major chunks for the fetch / the streaming
+    struct OutChunk {
+        cudaEvent_t ready = nullptr, done = nullptr;   // of the fetch's chunks (copy_out)
+    } out_chunk[2];
     DevBuf<int32_t> ret_rec;                 // retirement record per particle (RowFill)
     DevBuf<float> frz_pos, frz_vol, frz_cmp, frz_curv;   // frozen values of retired particles
     DevBuf<int32_t> rec_of_crec;             // position record of each curvature record
@@ -316,6 +321,10 @@ struct gr_engine {
         if (h_live) gr_host_free(h_live);
         if (live_ready) cudaEventDestroy(live_ready);
         if (upload_done) cudaEventDestroy(upload_done);
+        for (auto &c : out_chunk) {
+            if (c.ready) cudaEventDestroy(c.ready);
+            if (c.done) cudaEventDestroy(c.done);
+        }
         if (ds) cudaStreamSynchronize(ds);
         if (ds_ev) cudaEventDestroy(ds_ev);
         if (ds) cudaStreamDestroy(ds);
@@ -1777,25 +1786,38 @@ RowFill row_fill(const gr_engine *e, const float *frz, int32_t rec_offset, const
 
 // Record-major history -> particle-major rows on the device: records [r0, r1) of particles
 // [p0, p1) of a quantity with D floats per particle (records_to_rows_kernel), on `st`.
-int launch_records_to_rows(gr_engine *e, cudaStream_t st, const float *src, int64_t n, int D, int32_t r0,
-                           int32_t r1, int64_t p0, int64_t p1, float *dst, const RowFill &fill) {
-    constexpr int32_t kRowsPerLaunch = 32 * 65535;   // the grid's y extent
+template <int D, int TR>
+int rows_launch(gr_engine *e, cudaStream_t st, const float *src, int64_t n, int32_t r0, int32_t r1, int64_t p0,
+                int64_t p1, float *dst, const RowFill &fill) {
+    constexpr int32_t kRowsPerLaunch = TR * 65535;   // the grid's y extent
     for (int32_t a = r0; a < r1; a += kRowsPerLaunch) {
         const int32_t b = std::min(r1, a + kRowsPerLaunch);
         // each launch covers records [a, b) of the destination rows sized for [r0, r1)
-        const dim3 grid((unsigned)((p1 - p0 + 31) / 32), (unsigned)((b - a + 31) / 32));
-        float *d = dst + (int64_t)(a - r0) * D;
-        const int32_t nr = r1 - r0;
-        if (D == 1) records_to_rows_kernel<1><<<grid, 256, 0, st>>>(src, n, a, b, p0, p1, d, nr, fill);
-        else if (D == 2) records_to_rows_kernel<2><<<grid, 256, 0, st>>>(src, n, a, b, p0, p1, d, nr, fill);
-        else records_to_rows_kernel<3><<<grid, 256, 0, st>>>(src, n, a, b, p0, p1, d, nr, fill);
+        const dim3 grid((unsigned)((p1 - p0 + 1024 / TR - 1) / (1024 / TR)), (unsigned)((b - a + TR - 1) / TR));
+        records_to_rows_kernel<D, TR><<<grid, 256, 0, st>>>(src, n, a, b, p0, p1, dst + (int64_t)(a - r0) * D, r1 - r0,
+                                                            fill);
         CK(cudaGetLastError());
         e->stats.aux_launches++;
     }
     return GR_OK;
 }
 
-// Particles per staging chunk for particle-major rows of `row_floats` floats.
+template <int D>
+int rows_pick(gr_engine *e, cudaStream_t st, const float *src, int64_t n, int32_t r0, int32_t r1, int64_t p0,
+              int64_t p1, float *dst, const RowFill &fill) {
+    if (r1 - r0 == 1) return rows_launch<D, 1>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+    if (r1 - r0 <= 8) return rows_launch<D, 8>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+    return rows_launch<D, 32>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+}
+
+int launch_records_to_rows(gr_engine *e, cudaStream_t st, const float *src, int64_t n, int D, int32_t r0,
+                           int32_t r1, int64_t p0, int64_t p1, float *dst, const RowFill &fill) {
+    if (D == 1) return rows_pick<1>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+    if (D == 2) return rows_pick<2>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+    return rows_pick<3>(e, st, src, n, r0, r1, p0, p1, dst, fill);
+}
+
+// Particles per staging chunk of the streaming for particle-major rows of `row_floats` floats.
 int64_t stage_particles(int64_t n, int64_t row_floats) {
     constexpr int64_t kStageBytes = int64_t(256) << 20;
     return std::max<int64_t>(1, std::min<int64_t>(n, kStageBytes / std::max<int64_t>(1, row_floats * 4)));
@@ -2171,69 +2193,105 @@ int gr_stats_get(gr_engine *e, gr_stats *out) {
     return GR_OK;
 }
 
-static int fetch_rows(gr_engine *e, void *out, int64_t capacity, const void *src, int64_t rows, int64_t row_used,
-                      int64_t row_stride, size_t elem) {
-    if (!e || !out) return USER_ERR("null argument >");
-    if (!e->have_result) return USER_ERR("No result: run() has not completed. >");
-    if (capacity < rows * row_used) return USER_ERR("Output buffer too small. >");
-    if (rows == 0 || row_used == 0) return GR_OK;
-    int rc = set_device(e);
-    if (rc) return rc;
-    const size_t row_bytes = (size_t)row_used * elem, total = row_bytes * (size_t)rows;
+}  // extern "C"
+
+namespace {
+
+// `items` items of `item_bytes` bytes each to host memory, in chunks: produce(k0, k1, j) enqueues
+// items [k0, k1) on the step stream and returns where they lie (a staging buffer of its own per j, or
+// the data itself).  Chunks take turns in two buffers, so a chunk is produced while the one before
+// is on the link.  Every copy is contiguous: a 2D copy of the same bytes ran at 35 GB/s in rows of
+// 372 bytes and at 0.4 GB/s from rows of 80 bytes into pageable memory, against 55 GB/s.  Page-locked
+// destinations take one DMA a chunk; others go through two page-locked bounce buffers, emptied by the
+// copy threads (which also take the first-touch page faults of a fresh array) while the other fills.
+// 32 MB chunks keep every copy thread busy (80 MB of records in pageable memory: 9.9 ms a run, 13.4 ms
+// in chunks of 8 MB, 10.3 ms in chunks of 64).
+constexpr size_t kOutChunk = size_t(32) << 20, kDirect = size_t(64) << 10;
+
+int64_t chunk_items(int64_t items, size_t item_bytes) {
+    return std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)(kOutChunk / item_bytes)));
+}
+
+template <typename Produce>
+int copy_out(gr_engine *e, void *out, int64_t items, size_t item_bytes, Produce produce) {
+    const size_t total = (size_t)items * item_bytes;
     e->stats.d2h_bytes += (int64_t)total;
-    if (pinned_range(out, total)) {
-        // page-locked destination: one DMA, no staging
-        CK(cudaMemcpy2DAsync(out, row_bytes, src, row_stride * elem, row_bytes, rows, cudaMemcpyDeviceToHost, e->cs));
-        CK(cudaStreamSynchronize(e->cs));
-        return GR_OK;
+    const bool pinned = pinned_range(out, total);
+    const int64_t step = chunk_items(items, item_bytes);
+    char *const dst = static_cast<char *>(out);
+    for (auto &c : e->out_chunk) {
+        if (!c.ready) CK(cudaEventCreateWithFlags(&c.ready, cudaEventDisableTiming));
+        if (!c.done) CK(cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming));
     }
-    // up to 64 MB per bounce buffer; results from 8 MB on go through them, so the host copies
-    // (and the first-touch page faults of a fresh destination) run on the copy threads
-    constexpr size_t kBounce = size_t(64) << 20, kBounceFrom = size_t(8) << 20;
-    if (total < kBounceFrom || row_bytes > kBounce) {
-        CK(cudaMemcpy2D(out, row_bytes, src, row_stride * elem, row_bytes, rows, cudaMemcpyDeviceToHost));
-        return GR_OK;
-    }
-    // large results: DMA into two pinned bounce buffers, each emptied by a parallel host copy
-    // while the other fills
-    const size_t chunk = std::min(kBounce, total);
-    for (auto &b : e->bounce) {
-        if (b.bytes < chunk) {
-            if (b.p) gr_host_free(b.p);
-            b.p = nullptr;
-            b.bytes = 0;
-            if (gr_host_alloc((int64_t)chunk, &b.p) != GR_OK) return GR_ERR_RUNTIME;
-            b.bytes = chunk;
+    // bounce buffers from the host cache for the time of the copy, in few sizes, so that every
+    // engine finds them there (page-locking a fresh block takes a millisecond per 2 MB)
+    struct Bounce {
+        void *p = nullptr;
+        cudaStream_t st;
+        ~Bounce() {
+            if (!p) return;
+            cudaStreamSynchronize(st);   // after an error a copy may still be on its way
+            gr_host_free(p);
         }
-        if (!b.done) CK(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming));
+    } bounce[2];
+    for (auto &b : bounce) b.st = e->us;
+    if (!pinned && total > kDirect) {
+        size_t bytes = size_t(2) << 20;
+        while (bytes < (size_t)step * item_bytes) bytes *= 4;
+        for (int k = 0; k < (step < items ? 2 : 1); ++k)
+            if (gr_host_alloc((int64_t)bytes, &bounce[k].p) != GR_OK) return GR_ERR_RUNTIME;
     }
-    const int64_t rows_per = (int64_t)(std::min(e->bounce[0].bytes, e->bounce[1].bytes) / row_bytes);
-    const char *s8 = static_cast<const char *>(src);
-    char *d8 = static_cast<char *>(out);
-    int64_t prev_rows = 0, prev_row0 = 0;
+    int64_t before = 0, held = 0;   // the chunk that waits in the other bounce buffer
     int j = 0;
-    for (int64_t r0 = 0; r0 < rows; r0 += rows_per, j ^= 1) {
-        const int64_t nr = std::min(rows_per, rows - r0);
-        CK(cudaMemcpy2DAsync(e->bounce[j].p, row_bytes, s8 + (size_t)r0 * row_stride * elem, row_stride * elem,
-                             row_bytes, nr, cudaMemcpyDeviceToHost, e->cs));
-        CK(cudaEventRecord(e->bounce[j].done, e->cs));
-        if (prev_rows) {
-            CK(cudaEventSynchronize(e->bounce[j ^ 1].done));
-            parallel_memcpy(d8 + (size_t)prev_row0 * row_bytes, e->bounce[j ^ 1].p, (size_t)prev_rows * row_bytes);
+    for (int64_t k = 0; k < items; k += step, j ^= 1) {
+        const int64_t m = std::min(step, items - k);
+        const size_t bytes = (size_t)m * item_bytes;
+        gr_engine::OutChunk &c = e->out_chunk[j];
+        if (k >= 2 * step) CK(cudaStreamWaitEvent(e->cs, c.done, 0));   // its buffer has been read
+        const void *src = nullptr;
+        const int rc = produce(k, k + m, j, src);
+        if (rc) return rc;
+        if (!pinned && total <= kDirect) {   // a few pages: not worth the hand-over
+            CK(cudaMemcpyAsync(dst + (size_t)k * item_bytes, src, bytes, cudaMemcpyDeviceToHost, e->cs));
+            CK(cudaStreamSynchronize(e->cs));
+            continue;
         }
-        prev_rows = nr;
-        prev_row0 = r0;
+        CK(cudaEventRecord(c.ready, e->cs));
+        CK(cudaStreamWaitEvent(e->us, c.ready, 0));
+        CK(cudaMemcpyAsync(pinned ? dst + (size_t)k * item_bytes : static_cast<char *>(bounce[j].p), src, bytes,
+                           cudaMemcpyDeviceToHost, e->us));
+        CK(cudaEventRecord(c.done, e->us));
+        if (pinned) continue;
+        if (held) {
+            CK(cudaEventSynchronize(e->out_chunk[j ^ 1].done));
+            parallel_memcpy(dst + (size_t)before * item_bytes, bounce[j ^ 1].p, (size_t)held * item_bytes);
+        }
+        before = k;
+        held = m;
     }
-    CK(cudaEventSynchronize(e->bounce[j ^ 1].done));
-    parallel_memcpy(d8 + (size_t)prev_row0 * row_bytes, e->bounce[j ^ 1].p, (size_t)prev_rows * row_bytes);
+    CK(cudaStreamSynchronize(e->us));
+    if (held) parallel_memcpy(dst + (size_t)before * item_bytes, bounce[j ^ 1].p, (size_t)held * item_bytes);
     return GR_OK;
 }
 
+// One value per particle.
+int fetch_values(gr_engine *e, void *out, int64_t capacity, const void *src, int64_t n) {
+    if (!e || !out) return USER_ERR("null argument >");
+    if (!e->have_result) return USER_ERR("No result: run() has not completed. >");
+    if (capacity < n) return USER_ERR("Output buffer too small. >");
+    if (n == 0) return GR_OK;
+    const int rc = set_device(e);
+    if (rc) return rc;
+    return copy_out(e, out, n, 4, [&](int64_t k0, int64_t, int, const void *&at) {
+        at = static_cast<const char *>(src) + k0 * 4;
+        return GR_OK;
+    });
+}
+
 // Records [r0, r1) of a record-major quantity (D floats per particle) into particle-major host
-// rows of (r1 - r0) * D floats: chunks of particles transposed on the device into the staging
-// buffer (retired particles' frozen values substituted, RowFill), each fetched like any device
-// rows.
-static int fetch_records(gr_engine *e, float *out, int64_t cap, const float *src, int D, int64_t r0, int64_t r1,
+// rows of (r1 - r0) * D floats: chunks of particles transposed on the device into a staging
+// buffer (retired particles' frozen values substituted, RowFill).
+int fetch_records(gr_engine *e, float *out, int64_t cap, const float *src, int D, int64_t r0, int64_t r1,
                          const RowFill &fill) {
     if (!e || !out) return USER_ERR("null argument >");
     if (!e->have_result) return USER_ERR("No result: run() has not completed. >");
@@ -2242,18 +2300,18 @@ static int fetch_records(gr_engine *e, float *out, int64_t cap, const float *src
     if (n == 0 || w == 0) return GR_OK;
     int rc = set_device(e);
     if (rc) return rc;
-    const int64_t cp = stage_particles(n, w);
-    CK(e->stage.alloc((size_t)(cp * w)));
-    for (int64_t p0 = 0; p0 < n; p0 += cp) {
-        const int64_t p1 = std::min(n, p0 + cp);
-        rc = launch_records_to_rows(e, e->cs, src, n, D, (int32_t)r0, (int32_t)r1, p0, p1, e->stage.p, fill);
-        if (rc) return rc;
-        CK(cudaStreamSynchronize(e->cs));
-        rc = fetch_rows(e, out + p0 * w, (p1 - p0) * w, e->stage.p, p1 - p0, w, w, sizeof(float));
-        if (rc) return rc;
-    }
-    return GR_OK;
+    const size_t row = (size_t)w * sizeof(float);
+    const int64_t step = chunk_items(n, row);
+    for (int j = 0; j < (step < n ? 2 : 1); ++j) CK(e->stage[j].alloc((size_t)(step * w)));
+    return copy_out(e, out, n, row, [&](int64_t p0, int64_t p1, int j, const void *&at) {
+        at = e->stage[j].p;
+        return launch_records_to_rows(e, e->cs, src, n, D, (int32_t)r0, (int32_t)r1, p0, p1, e->stage[j].p, fill);
+    });
 }
+
+}  // namespace
+
+extern "C" {
 
 int gr_fetch_positions(gr_engine *e, float *out, int64_t cap) {
     if (!e) return USER_ERR("null engine >");
@@ -2270,19 +2328,19 @@ int gr_fetch_final_positions(gr_engine *e, float *out, int64_t cap) {
 
 int gr_fetch_status(gr_engine *e, int32_t *out, int64_t cap) {
     if (!e) return USER_ERR("null engine >");
-    return fetch_rows(e, out, cap, e->out_status.p, 1, e->n, e->n, sizeof(int32_t));
+    return fetch_values(e, out, cap, e->out_status.p, e->n);
 }
 
 int gr_fetch_lengths(gr_engine *e, float *out, int64_t cap) {
     if (!e) return USER_ERR("null engine >");
     if (e->s.abort_mode == 0) return GR_OK;
-    return fetch_rows(e, out, cap, e->out_length.p, 1, e->n, e->n, sizeof(float));
+    return fetch_values(e, out, cap, e->out_length.p, e->n);
 }
 
 int gr_fetch_total_curvature(gr_engine *e, float *out, int64_t cap) {
     if (!e) return USER_ERR("null engine >");
     if (e->s.curvature_mode == 0) return GR_OK;
-    return fetch_rows(e, out, cap, e->out_tc.p, 1, e->n, e->n, sizeof(float));
+    return fetch_values(e, out, cap, e->out_tc.p, e->n);
 }
 
 int gr_fetch_curvatures(gr_engine *e, float *out, int64_t cap) {
