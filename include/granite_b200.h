@@ -333,8 +333,9 @@ int gr_tune(gr_engine *engine, int32_t trial_steps, gr_tune_result *out);
  * in the reference, which integrates one seed set per TrajectoryIntegrator.
  *
  * The field (n_snapshots snapshots of nz x ny x nx nodes, DataTimeDistance apart, stored as
- * settings->storage) is packed once into pinned host memory by gr_server_set_snapshot.  A
- * worker thread sweeps it window by window through a 4-slot device ring refilled from there.
+ * settings->storage) is packed once by gr_server_set_snapshot: into device memory where the
+ * whole field fits a quarter of what is free at creation, else into pinned host memory.  A
+ * worker thread sweeps it window by window, the field in host memory through a 4-slot device ring.
  * A request is a seed set, a start time (seconds on the field's clock, rounded down to the
  * step grid DeltaT), a step count and an integrator (0 Euler, 1 RK4); it runs from its start step
  * until the step count, an abort, or the end of the field, whichever comes first.  Requests

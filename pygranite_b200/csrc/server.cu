@@ -2,24 +2,25 @@
 //
 // No counterpart in the reference, which integrates one seed set per TrajectoryIntegrator.
 // Requests (a seed set, a start time, a step count, Euler or RK4) arrive at any time from
-// any thread.  One worker thread sweeps the field window by window: a 4-slot device ring
-// holds the snapshots of the current window and the next ones, refilled from pinned host
-// memory on a copy stream while the current window integrates.  All requests share the
-// field's global step clock (start times are rounded down to the step grid), so the particles of
-// every request active in a window advance in the same launch (continuous batching):
+// any thread.  One worker thread sweeps the field window by window.  A field that fits a quarter of
+// the free device memory stays there, packed, and so does every window's pair once it has been built;
+// a larger one is kept in pinned host memory and a 4-slot device ring holds the snapshots of the
+// current window and the next ones, refilled on a copy stream while the current window integrates.
+// All requests share the field's global step clock (start times are rounded down to the step grid), so
+// the particles of every request active in a window advance in the same launch (continuous batching):
 //
 //   per window, on the compute stream:
 //     admit   requests whose start step falls in the window, while their state fits the
 //             HBM budget: seeds -> the tail of the integrator's particle pool;
-//     pack    the window-pair buffer from the two ring slots (planar, unpadded on the host
-//             and in the ring: 25% less upload than padded 3D nodes);
+//     pack    the window-pair buffer from the two slots (planar, unpadded: 25% less upload
+//             than padded 3D nodes), unless it is there already;
 //     advance one persistent grid-stride launch per pool over the window's steps (a
 //             particle runs steps [start, end) of the clock);
 //     retire  compaction + Morton re-sort of each pool; particles that aborted or reached
 //             their end step leave the pool, their final state written to their request's
 //             slots of the result arena;
-//     return  requests whose end step is in the window are complete: their result slices
-//             go to pinned host memory, and the worker hands them out when the copy is done.
+//     return  requests whose end step is in the window are complete: a kernel writes their
+//             result slices to pinned host memory, and the worker hands them out when it is done.
 //
 // With no particle in flight the sweep jumps to the earliest start window waiting.  A
 // request whose start window the sweep has passed waits for the next sweep.  Per-particle
@@ -31,6 +32,7 @@
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
+#include <cstdlib>
 #include <deque>
 #include <map>
 #include <memory>
@@ -51,7 +53,7 @@ using namespace granite_b200;
 
 namespace {
 
-constexpr int kRing = 4;         // ring slots
+constexpr int kRing = 4;         // ring slots of a field that is not resident
 constexpr int kLag = 2;          // windows the host may enqueue ahead of the device
 
 // First-fit allocator of index ranges (result arena, pinned staging).
@@ -135,11 +137,16 @@ struct gr_server {
     Schedule sched;
     DevBuf<StepEntry> d_sched;
     int64_t elem = 4;                  // bytes per stored value
-    std::vector<void *> host_snap;     // pinned packed snapshots
+    bool resident = false;             // every snapshot has a slot of its own
+    int64_t K = kRing;                 // slots
+    std::vector<char> have;            // snapshots set
+    std::vector<void *> host_snap;     // pinned packed snapshots (not resident)
     int64_t snap_bytes = 0, slot_stride = 0;
     DevBuf<char> ring, pair;
+    int64_t pair_stride = 0;           // > 0: window w's pair stays at w * pair_stride
+    std::vector<char> pair_built;
     DevBuf<float> raw;
-    int64_t ring_holds[kRing];
+    int64_t ring_holds[kRing];         // not resident: snapshots in the slots, and their events
     bool slot_used[kRing]{};
     cudaEvent_t slot_ready[kRing]{}, slot_free[kRing]{};
     std::vector<cudaEvent_t> win_done;   // kLag + 1 events: windows in flight
@@ -226,6 +233,19 @@ __global__ void append_kernel(const float *__restrict__ seeds, const int32_t *__
 
 __global__ void grow_kernel(int32_t *counts, int32_t m) { counts[0] += m; }
 
+// The results of one request, from its slots of the arena: positions (n, dim), then abort codes, in
+// pinned host memory.  One launch instead of four copies of a few kilobytes, and the rows need no
+// transposing on the host.
+__global__ void return_kernel(const float *__restrict__ px, const float *__restrict__ py, const float *__restrict__ pz,
+                              const int32_t *__restrict__ status, int64_t n, int dim, float *__restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * dim; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t q = i / dim;
+        const int d = (int)(i - q * dim);
+        out[i] = d == 0 ? px[q] : d == 1 ? py[q] : pz[q];
+        if (i < n) reinterpret_cast<int32_t *>(out)[n * dim + i] = status[i];
+    }
+}
+
 // Host snapshots and ring slots are planar, unpadded (u, v[, w] planes of the storage type,
 // round to nearest even): 25% fewer bytes per 3D upload than padded nodes.
 template <typename T>
@@ -292,7 +312,7 @@ __global__ void init_pool_kernel(int32_t *counts) {
     counts[3] = 0;
 }
 
-int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx) {
+int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx, int64_t field_budget) {
     S->nx = nx; S->ny = ny; S->nz = S->dim == 3 ? nz : 1;
     S->nodes = S->nx * S->ny * S->nz;
     const gr_settings &s = S->s;
@@ -313,11 +333,29 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx) {
     S->elem = s.storage == GR_STORE_F32 ? 4 : 2;
     S->snap_bytes = S->nodes * S->dim * S->elem;                  // planar, unpadded
     S->slot_stride = ((S->snap_bytes + 255) / 256) * 256;
-    SK(S->ring.alloc((size_t)S->slot_stride * kRing));
     // window pairs carry a border (padded_pair_nodes); the kernel indexes them with int32
     if (padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) > (int64_t(1) << 31) - 1)
         return SUSER("Invalid dataset was provided. Grid too large.");
-    SK(S->pair.alloc((size_t)padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) * (S->dim == 3 ? 8 : 4) * S->elem));
+    const int64_t pair_bytes = ((padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) * (S->dim == 3 ? 8 : 4) * S->elem + 255) / 256) * 256;
+    // the whole field on the device where it fits the budget, with all its pairs if they fit too
+    const int64_t field = S->slot_stride * S->n_snap;
+    const char *env = std::getenv("GR_SERVE_RESIDENT");   // 0: host memory whatever fits
+    S->resident = !(env && env[0] == '0') && field + pair_bytes <= field_budget;
+    if (S->resident && field + pair_bytes * (S->n_snap - 1) <= field_budget) S->pair_stride = pair_bytes;
+    if (S->resident && (S->ring.alloc((size_t)field) != cudaSuccess ||
+                        S->pair.alloc((size_t)(S->pair_stride > 0 ? S->pair_stride * (S->n_snap - 1) : pair_bytes)) !=
+                            cudaSuccess)) {
+        cudaGetLastError();   // not in one piece after all
+        S->resident = false;
+        S->pair_stride = 0;
+        S->ring.reset();
+        S->pair.reset();
+    }
+    S->K = S->resident ? S->n_snap : kRing;
+    SK(S->ring.alloc((size_t)(S->slot_stride * S->K)));
+    SK(S->pair.alloc((size_t)pair_bytes));
+    S->pair_built.assign((size_t)S->n_snap, 0);
+    S->have.assign((size_t)S->n_snap, 0);
     SK(S->raw.alloc((size_t)S->nodes * S->dim));
     S->host_snap.assign((size_t)S->n_snap, nullptr);
     for (int k = 0; k < kRing; ++k) S->ring_holds[k] = -1;
@@ -402,6 +440,9 @@ int allocate(gr_server *S, int64_t budget) {
     return GR_OK;
 }
 
+// Window w's pair.
+char *pair_at(gr_server *S, int64_t w) { return S->pair.p + w * S->pair_stride; }
+
 KParams pool_params(gr_server *S, Pool &P) {
     KParams K;
     std::memset(&K, 0, sizeof K);
@@ -416,7 +457,7 @@ KParams pool_params(gr_server *S, Pool &P) {
     clamp_cells(K, true);
     K.wind = S->ring.p;
     K.wind_stride = S->slot_stride;
-    K.pair = S->pair.p;
+    K.pair = pair_at(S, S->w);
     K.pnx = (int32_t)(S->nx + 3); K.pnxy = (int32_t)((S->nx + 3) * (S->ny + 3));
     Pool::Arrays &A = P.st[P.cur];
     K.px = A.px.p; K.py = A.py.p; K.pz = A.pz.p;
@@ -495,23 +536,26 @@ int ensure_snapshot(gr_server *S, int64_t v) {
 }
 
 int pack_pair(gr_server *S, int64_t v) {
-    const char *back = S->ring.p + (v % kRing) * S->slot_stride;
-    const char *front = S->ring.p + ((v + 1) % kRing) * S->slot_stride;
+    if (S->pair_stride > 0 && S->pair_built[S->w]) return GR_OK;
+    S->pair_built[S->w] = 1;
+    char *const out = pair_at(S, S->w);
+    const char *back = S->ring.p + (v % S->K) * S->slot_stride;
+    const char *front = S->ring.p + ((v + 1) % S->K) * S->slot_stride;
     const int threads = 256, blocks = grid_for(S->nodes, threads);
     switch (S->s.storage) {
         case GR_STORE_BF16:
             planar_pair_kernel<__nv_bfloat16><<<blocks, threads, 0, S->cs>>>(
-                (const __nv_bfloat16 *)back, (const __nv_bfloat16 *)front, (__nv_bfloat16 *)S->pair.p, S->nodes, S->dim,
+                (const __nv_bfloat16 *)back, (const __nv_bfloat16 *)front, (__nv_bfloat16 *)out, S->nodes, S->dim,
                 (int32_t)S->nx, (int32_t)S->ny, (int32_t)S->nz);
             break;
         case GR_STORE_F16:
             planar_pair_kernel<__half><<<blocks, threads, 0, S->cs>>>((const __half *)back, (const __half *)front,
-                                                                     (__half *)S->pair.p, S->nodes, S->dim,
+                                                                     (__half *)out, S->nodes, S->dim,
                                                                      (int32_t)S->nx, (int32_t)S->ny, (int32_t)S->nz);
             break;
         default:
             planar_pair_kernel<float><<<blocks, threads, 0, S->cs>>>((const float *)back, (const float *)front,
-                                                                    (float *)S->pair.p, S->nodes, S->dim,
+                                                                    (float *)out, S->nodes, S->dim,
                                                                     (int32_t)S->nx, (int32_t)S->ny, (int32_t)S->nz);
             break;
     }
@@ -573,7 +617,7 @@ int run_window(gr_server *S, const std::vector<Req *> &adm, const std::vector<Re
     // keep at most kLag windows in flight
     cudaEvent_t lag = S->win_done[S->win_count % S->win_done.size()];
     if (S->win_count >= (int64_t)S->win_done.size()) SK(cudaEventSynchronize(lag));
-    for (int64_t k = v; k < v + kRing && k < (S->sweep + 1) * S->n_snap; ++k) {
+    for (int64_t k = v; !S->resident && k < v + kRing && k < (S->sweep + 1) * S->n_snap; ++k) {
         const int slot = (int)(k % kRing);
         if (k >= v + 2 && S->slot_used[slot] && S->ring_holds[slot] != k) {
             // prefetch only into slots whose previous use has finished
@@ -582,8 +626,10 @@ int run_window(gr_server *S, const std::vector<Req *> &adm, const std::vector<Re
         const int rc = ensure_snapshot(S, k);
         if (rc) return rc;
     }
-    SK(cudaStreamWaitEvent(S->cs, S->slot_ready[v % kRing], 0));
-    SK(cudaStreamWaitEvent(S->cs, S->slot_ready[(v + 1) % kRing], 0));
+    if (!S->resident) {
+        SK(cudaStreamWaitEvent(S->cs, S->slot_ready[v % kRing], 0));
+        SK(cudaStreamWaitEvent(S->cs, S->slot_ready[(v + 1) % kRing], 0));
+    }
     int rc = admit(S, adm);
     if (rc) return rc;
     const int64_t k0 = S->sched.window_begin[S->w], k1 = S->sched.window_begin[S->w + 1];
@@ -603,7 +649,7 @@ int run_window(gr_server *S, const std::vector<Req *> &adm, const std::vector<Re
         rc = compact_pool(S, P, (int32_t)k1);
         if (rc) return rc;
     }
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 2 && !S->resident; ++k) {
         const int slot = (int)((v + k) % kRing);
         SK(cudaEventRecord(S->slot_free[slot], S->cs));
         S->slot_used[slot] = true;
@@ -612,10 +658,10 @@ int run_window(gr_server *S, const std::vector<Req *> &adm, const std::vector<Re
     for (Req *r : finishing) {
         const int64_t n = r->n, D = S->dim;
         float *dst = S->pin_res + r->stage;
-        SK(cudaMemcpyAsync(dst, S->res_px.p + r->slot, n * 4, cudaMemcpyDeviceToHost, S->cs));
-        SK(cudaMemcpyAsync(dst + n, S->res_py.p + r->slot, n * 4, cudaMemcpyDeviceToHost, S->cs));
-        if (D == 3) SK(cudaMemcpyAsync(dst + 2 * n, S->res_pz.p + r->slot, n * 4, cudaMemcpyDeviceToHost, S->cs));
-        SK(cudaMemcpyAsync(dst + D * n, S->res_status.p + r->slot, n * 4, cudaMemcpyDeviceToHost, S->cs));
+        return_kernel<<<grid_for(n * D, 256), 256, 0, S->cs>>>(S->res_px.p + r->slot, S->res_py.p + r->slot,
+                                                               D == 3 ? S->res_pz.p + r->slot : nullptr,
+                                                               S->res_status.p + r->slot, n, (int)D, dst);
+        SK(cudaGetLastError());
         if (!r->done_ev) SK(cudaEventCreateWithFlags(&r->done_ev, cudaEventDisableTiming));
         SK(cudaEventRecord(r->done_ev, S->cs));
         S->pools[r->integrator].in_flight -= n;
@@ -639,11 +685,9 @@ void collect(gr_server *S, bool block) {
         if (q != cudaSuccess && S->failure.empty()) S->failure = cudaGetErrorString(q);
         const int64_t n = r->n, D = S->dim;
         const float *src = S->pin_res + r->stage;
-        r->pos.resize((size_t)n * D);
-        r->status.resize((size_t)n);
-        for (int64_t i = 0; i < n; ++i)
-            for (int64_t d = 0; d < D; ++d) r->pos[i * D + d] = src[d * n + i];
-        std::memcpy(r->status.data(), src + D * n, (size_t)n * 4);
+        const int32_t *st = reinterpret_cast<const int32_t *>(src + D * n);
+        r->pos.assign(src, src + n * D);
+        r->status.assign(st, st + n);
         S->pin_alloc.give(r->stage, n * (D + 1));
         S->arena.give(r->slot, n);
         r->state = r->cancelled ? GR_REQ_CANCELLED : GR_REQ_DONE;
@@ -847,7 +891,10 @@ int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t n
     }
     S->win_done.assign(kLag + 1, nullptr);
     for (auto &e : S->win_done) SK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    int rc = setup(S.get(), S->dim == 3 ? nz : 1, ny, nx);
+    size_t fr = 0, tot = 0;
+    SK(cudaMemGetInfo(&fr, &tot));
+    const int64_t quarter = (int64_t)((fr + dev_pool_idle_bytes()) / 4);   // the pool's idle memory is ours to use
+    int rc = setup(S.get(), S->dim == 3 ? nz : 1, ny, nx, quarter);
     if (rc) return rc;
     // the field's global step clock: the reference's float32 schedule over all windows
     ScheduleInput si;
@@ -875,13 +922,7 @@ int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t n
     }
     SK(S->d_sched.alloc(hs.size()));
     SK(cudaMemcpy(S->d_sched.p, hs.data(), hs.size() * sizeof(StepEntry), cudaMemcpyHostToDevice));
-    int64_t budget = hbm_budget_bytes;
-    if (budget <= 0) {
-        size_t fr = 0, tot = 0;
-        SK(cudaMemGetInfo(&fr, &tot));
-        budget = (int64_t)((fr + dev_pool_idle_bytes()) / 4);   // the pool's idle memory is ours to use
-    }
-    rc = allocate(S.get(), budget);
+    rc = allocate(S.get(), hbm_budget_bytes > 0 ? hbm_budget_bytes : quarter);
     if (rc) return rc;
     // pinned result staging: a quarter of the arena (at most 256 MB), never less than one full
     // pool, so any admissible request fits; completions beyond it wait a window
@@ -914,7 +955,8 @@ int gr_server_set_snapshot(gr_server *S, int64_t snapshot, const float *const *c
         }
     }
     if (ncomp == 2) src[2] = src[1];
-    char *scratch = S->ring.p;   // slot 0 as packing scratch before the server starts
+    // a resident snapshot is packed where it stays; else slot 0 is packing scratch until the start
+    char *scratch = S->ring.p + (S->resident ? snapshot * S->slot_stride : 0);
     const int threads = 256, blocks = grid_for(S->nodes, threads);
     switch (S->s.storage) {
         case GR_STORE_BF16:
@@ -929,18 +971,21 @@ int gr_server_set_snapshot(gr_server *S, int64_t snapshot, const float *const *c
             break;
     }
     SK(cudaGetLastError());
-    void *&h = S->host_snap[(size_t)snapshot];
-    if (!h) SK(cudaMallocHost(&h, (size_t)S->snap_bytes));
-    SK(cudaMemcpyAsync(h, scratch, (size_t)S->snap_bytes, cudaMemcpyDeviceToHost, S->cs));
+    if (!S->resident) {
+        void *&h = S->host_snap[(size_t)snapshot];
+        if (!h) SK(cudaMallocHost(&h, (size_t)S->snap_bytes));
+        SK(cudaMemcpyAsync(h, scratch, (size_t)S->snap_bytes, cudaMemcpyDeviceToHost, S->cs));
+    }
     SK(cudaStreamSynchronize(S->cs));
+    S->have[(size_t)snapshot] = 1;
     return GR_OK;
 }
 
 int gr_server_start(gr_server *S) {
     if (!S) return SUSER("null server");
     if (S->started) return GR_OK;
-    for (void *p : S->host_snap)
-        if (!p) return SUSER("Every snapshot must be set before the server starts.");
+    for (char h : S->have)
+        if (!h) return SUSER("Every snapshot must be set before the server starts.");
     for (int k = 0; k < kRing; ++k) S->ring_holds[k] = -1;
     S->started = true;
     S->t0 = std::chrono::steady_clock::now();
