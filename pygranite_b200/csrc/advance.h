@@ -30,13 +30,47 @@ inline int kernel_features(const KParams &P, bool defer = false) {
 inline void clamp_cells(KParams &P, bool as_pair) {
     const bool one = as_pair || P.dim == 2;
     P.flo = one ? -1.f : -2.f;
+    P.below = one ? 1 : 2;
     const int32_t n[3] = {P.nx, P.ny, P.nz};
     for (int d = 0; d < 3; ++d) P.fn[d] = one ? (float)n[d] : (float)(n[d] + 1);
+}
+
+// The step constants of a time step h and the operand pairs of the paired instructions, from off and
+// inv_scale.
+inline void derive_params(KParams &P, float h) {
+    auto both = [](float a) { return make_float2(a, a); };
+    P.h = h;
+    P.hh = 0.5f * h;
+    P.sixth = 1.0f / 6;
+    P.inv_2h = 1.0f / (2.0f * h);
+    P.inv_hh = 1.0f / (h * h);
+    P.h2 = both(P.h);
+    P.hh2 = both(P.hh);
+    P.sixth2 = both(P.sixth);
+    P.i2h2 = both(P.inv_2h);
+    P.ihh2 = both(P.inv_hh);
+    P.noff2 = make_float2(-P.off[0], -P.off[1]);
+    P.noffz = -P.off[2];
+    P.inv2 = make_float2(P.inv_scale[0], P.inv_scale[1]);
 }
 
 // Grids that the fast cell arithmetic does not cover (pcell1 needs coordinates below 2^22).
 inline bool wide_grid(int64_t nx, int64_t ny, int64_t nz) {
     return nx >= (1 << 22) - 2 || ny >= (1 << 22) - 2 || nz >= (1 << 22) - 2;
+}
+
+// Threads per block of a launch over few particles: blocks of 4, 8 or 16 threads, each a warp of its
+// own, or 0 for whole warps.  A warp waits for a cell whenever one of its lanes changes cells, at 32
+// lanes nearly every sample, so with schedulers idle fewer lanes a warp are faster: 100 RK4 steps of 1,000
+// particles 0.21 -> 0.15 ms at 4 lanes, 4,097 0.26 -> 0.20 at 8 (0.20 at 4, but 1.01 against 0.85 with
+// volumes and expressions over 240 steps), 10,000 0.34 -> 0.28 at 8, 20,000 0.32 -> 0.31 at 16.  The line
+// lies where the warps would come in a second wave (16 an SM; 20,000 at 8 lanes: 0.48 ms) with some room.
+inline int block_of_few(int64_t n) {
+    constexpr int64_t sms = 148;
+    if (n <= 4 * 4 * sms) return 4;
+    if (n <= 8 * 9 * sms) return 8;
+    if (n <= 16 * 9 * sms) return 16;
+    return 0;
 }
 
 // Step kernel for a dimension, integrator, wind layout (pair = window-pair buffer) and feature

@@ -1080,12 +1080,13 @@ size_t pair_bytes(const gr_engine *e) {
 // 1.30 / 1.59, 150,000 2.29 / 2.03; 512 x 512 x 96 bf16, 777,777 x 100 steps 2.84 / 3.73; 24 x 24 x 16,
 // 100 steps, 50,000 0.26 / 0.28, 150,000 0.61 / 0.52; 2D 1024 x 512 nodes, 200 steps, 150,000 0.58 /
 // 0.63, 400,000 1.16 / 1.08; 256 x 128, 10,000 x 1024 Euler steps, 128 a window, 0.58 / 0.42.  Where the
-// settings place the launches, only the pack is saved.
+// settings place the launches, only the pack is saved; in a graph a launch costs little, all the less
+// beside another engine's (the batch of 48 sets: 3.40 ms a replay with pairs, 3.63 without).
 bool small_set(const gr_engine *e, const RunPlan &R) {
     if (R.nsteps == 0 || !e->wind_dynamic) return false;
     const gr_settings &s = e->s;
     const bool extras = (s.volume_mode != 0 && e->nvol > 0) || e->nexpr > 0;
-    const double launch = s.sort_interval > 0 || s.steps_per_launch > 0 ? 0.0 : extras ? 18.0 : 10.0;
+    const double launch = s.sort_interval > 0 || s.steps_per_launch > 0 ? 0.0 : R.graph ? 3.0 : extras ? 18.0 : 10.0;
     const double pack = (double)e->nodes * 4 * pair_elem(e) / 5e6;   // us at 5 TB/s
     const double steps = (double)R.nsteps / (double)R.nwin;          // a window
     const double chain = e->dim == 3 ? 0.5 : 0.18, gathers = extras ? 25.0 : e->dim == 3 ? 8.6 : 3.0;
@@ -1254,7 +1255,6 @@ KParams make_params(gr_engine *e) {
     for (int d = 0; d < 3; ++d) {
         P.inv_scale[d] = e->inv_scale[d];
         P.off[d] = e->off[d];
-        P.noff[d] = -e->off[d];
         P.dom[d] = e->dom[d];
         P.scale[d] = e->scale[d];
     }
@@ -1279,11 +1279,7 @@ KParams make_params(gr_engine *e) {
     P.L = e->L; P.Lc = e->Lc; P.Li = e->Li;
     P.sched = e->d_sched.p;
     const gr_settings &s = e->s;
-    P.h = s.delta_t;
-    P.hh = 0.5f * s.delta_t;
-    P.sixth = 1.0f / 6;
-    P.inv_2h = 1.0f / (2.0f * s.delta_t);
-    P.inv_hh = 1.0f / (s.delta_t * s.delta_t);
+    derive_params(P, s.delta_t);
     P.max_length = s.maximum_length;
     P.sphere_radius = s.sphere_radius;
     P.wind_dynamic = e->wind_dynamic;
@@ -1377,6 +1373,8 @@ KernelFn pick_kernel(const gr_engine *e, const KParams &P, bool defer) {
 
 int block_size_for(const gr_engine *e) {
     if (e->s.block_size > 0) return e->s.block_size;
+    // (the alive counts per step are whole warps' ballots)
+    if (const int few = e->s.minimum_alive > 0 ? 0 : block_of_few(e->n)) return few;
     // keep at least ~2 blocks per SM on small particle counts
     int bs = 256;
     while (bs > 32 && (e->n + bs - 1) / bs < 2 * 148) bs /= 2;

@@ -64,8 +64,8 @@ constexpr int SF_CURV_REC = 4;   // curvature record after this step (Individual
 struct StepEntry {
     float t0, t1, t2;      // time weights of the RK4 stages (t1 also for k3)
     int32_t flags;
-    int32_t rec, crec, irec;
     int32_t slot_back, slot_front;   // ring slots of the window's snapshots
+    int32_t rec, crec, irec;
     int32_t pad[3];
 };
 
@@ -74,8 +74,12 @@ struct KParams {
     float inv_scale[3], off[3], dom[3], scale[3];
     int32_t nx, ny, nz, dim;
     float fn[3], flo;             // clamp of a sample's grid coordinates: [flo, fn] (clamp_cells)
+    int32_t below;                // cells -below .. n + below - 1 are read as they are
     int32_t wide;                 // 1: a grid too large for pcell1 or the cell index (ring layouts only)
-    float noff[3];                // -off: world position -> grid is (p + noff) * inv_scale
+    // operand pairs of the paired instructions and -off: world position -> grid is
+    // (p + noff) * inv_scale
+    float2 noff2, inv2, h2, hh2, sixth2, i2h2, ihh2;
+    float noffz;
     // ring buffers: slot s of quantity q starts at base + s * stride
     const void *wind;
     int64_t wind_stride;          // bytes per slot
@@ -260,18 +264,24 @@ __device__ __forceinline__ Cell3 make_cell3(const KParams &P, float ax, float ay
 
 // Nodes of the last cell a particle sampled.  Consecutive samples of one particle (its RK4 stages,
 // its next step) mostly fall in the same cell, whose nodes then need no new gathers; the values and
-// the arithmetic are the same either way.  The cell is identified by its first corner's index in a
-// padded grid (`base`, the node index of the pair buffer); 3D keeps 24 float
+// the arithmetic are the same either way.  The cell is identified by its
+// node index or by its negated first corner (wind_at); 3D keeps 24 float
 // pairs (48 registers; 16-bit nodes converted when loaded; AdvBounds gives the launch shape), 2D 8
 // pairs (16 registers).
 // Corner k + 1 of each x pair (k even) is kept as its difference from corner k, formed once when
 // the cell is loaded: the x lerps of every later sample are then one paired FMA each, with the
 // difference lerp2_ would form (same instruction, same rounding).
 struct SampleCache {
-    int32_t base;
+    int32_t base;      // 3D pairs: padded node index of the first corner
+    float2 nxy;        // else: minus the first corner; NaN: no cell, or one not to be kept
+    float nz;
     float2 c2d[2][4];  // 2D: (u, v) of the back and of the front snapshot at corners 0, 2; differences 1 - 0, 3 - 2
     float2 c2[3][8];   // 3D: (u, v) back, (u, v) front, (w_b, w_f) at even corners, differences at odd ones
-    __device__ __forceinline__ void reset() { base = (int32_t)0x80000000; }   // no cell's index
+    __device__ __forceinline__ void reset() {
+        base = (int32_t)0x80000000;   // no cell's index
+        nz = __int_as_float(0x7fffffff);
+        nxy = both(nz);
+    }
 };
 
 // 2D window pair with replicated edges: padded node (x, y), x in [-1, nx + 1] and y in
@@ -282,7 +292,7 @@ struct SampleCache {
 //
 // 3D window pair with a zero border (one node below, two above the grid on every axis): the
 // coordinate is clamped to [-1, n], so every corner of the footprint is a node of the padded
-// buffer and needs no validity test, and the footprint's first corner alone identifies the cell.
+// buffer and needs no validity test.
 // Same values as make_cell3 + border addressing: inside [-1, n] the cell and fraction are
 // identical; outside it every corner the original reads is outside the grid (0), and here the
 // fraction is 0 with the weighted-away corner finite, so the interpolation is +0 either way.
@@ -294,71 +304,43 @@ inline int64_t padded_pair_nodes(int dim, int64_t nx, int64_t ny, int64_t nz) {
 }
 #endif
 
+// Cell of a coordinate without the conversion unit.  For |a| < 2^22, a + 1.5 * 2^23 rounded toward
+// -infinity lies in [2^23, 2^24), where the floats are the integers, so it is floor(a) + 1.5 * 2^23
+// exactly, its bit pattern is PCELL_BITS + floor(a), and 1.5 * 2^23 minus it is -floor(a).  The sum is
+// monotonic, so no coordinate outside that range (nor NaN) has the pattern of a cell in it.
+constexpr uint32_t PCELL_BITS = 0x4B400000u;   // bit pattern of 1.5 * 2^23
+constexpr float PCELL_MAGIC = 12582912.0f;     // 1.5 * 2^23
 struct PCell {
-    int32_t base;            // padded node index of corner (ix, iy, iz)
     uint32_t bx, by, bz;     // PCELL_BITS + cell
-    float fx, fy, fz;
+    float2 nxy;              // minus the cell
+    float nz;
 };
 
-// Cell of a coordinate without the conversion unit.  a is clamped to [lo, n] (n < 2^22, lo >= -2); a + 1.5 * 2^23 rounded toward -infinity lies in [2^23, 2^24), where the floats
-// are the integers, so it is floor(a) + 1.5 * 2^23 exactly and its bit pattern is
-// PCELL_BITS + floor(a).  The fraction a + (1.5 * 2^23 - t) equals a - floorf(a) bit for bit,
-// the sign of a zero fraction included (an exact integer is subtracted either way).
-constexpr uint32_t PCELL_BITS = 0x4B400000u;   // bit pattern of 1.5 * 2^23
-__device__ __forceinline__ float frac256(float f) { return floorf(f * 256.0f + 0.5f) * (1.0f / 256.0f); }
-
-__device__ __forceinline__ uint32_t pcell1(float a, float lo, float n, int fw, float &f) {
-    a = fminf(fmaxf(a, lo), n);
-    const float t = __fadd_rd(a, 12582912.0f);
-    f = a + (12582912.0f - t);
-    if (fw) f = frac256(f);
-    return __float_as_uint(t);   // PCELL_BITS + floor(a)
+template <int DIM>
+__device__ __forceinline__ PCell make_pcell(float2 axy, float az) {
+    PCell c;
+    const float2 t = __fadd2_rd(axy, both(PCELL_MAGIC));
+    c.bx = __float_as_uint(t.x);
+    c.by = __float_as_uint(t.y);
+    c.nxy = sub2(both(PCELL_MAGIC), t);
+    c.bz = 0;
+    c.nz = 0.f;
+    if (DIM == 3) {
+        const float tz = __fadd_rd(az, PCELL_MAGIC);
+        c.bz = __float_as_uint(tz);
+        c.nz = PCELL_MAGIC - tz;
+    }
+    return c;
 }
 
-// pcell1 of x and y at once (one paired operation for each of its additions).
-__device__ __forceinline__ void pcell2(float2 a, float lo, float nx, float ny, int fw, uint32_t &bx, uint32_t &by, float2 &f) {
-    a.x = fminf(fmaxf(a.x, lo), nx);
-    a.y = fminf(fmaxf(a.y, lo), ny);
-    const float2 t = __fadd2_rd(a, both(12582912.0f));
-    f = add2(a, sub2(both(12582912.0f), t));
-    if (fw) f = make_float2(frac256(f.x), frac256(f.y));
-    bx = __float_as_uint(t.x);
-    by = __float_as_uint(t.y);
-}
-
-// The same by the conversion unit, for grids of 2^22 nodes and more along an axis.
-__device__ __forceinline__ uint32_t pcell1_wide(float a, float lo, float n, int fw, float &f) {
-    a = fminf(fmaxf(a, lo), n);
+// The same by the conversion unit, for grids of 2^22 nodes and more along an axis (a clamped).
+__device__ __forceinline__ uint32_t pcell1_wide(float a, float &neg) {
     const float fl = floorf(a);
-    f = a - fl;
-    if (fw) f = frac256(f);
+    neg = -fl;
     return PCELL_BITS + (uint32_t)(int)fl;
 }
 
-// Cell of a sample at grid coordinates (axy, az).  fw: the launch's filter_weights (0 where the
-// variant has it off at compile time).  The index (iz + 1) pnxy + (iy + 1) pnx + (ix + 1) is formed
-// from the bit patterns of pcell1 in wrapping 32-bit arithmetic, with the patterns' offset removed
-// by one loop-invariant term.
-template <int DIM>
-__device__ __forceinline__ PCell make_pcell(const KParams &P, float2 axy, float az, int fw, float lo, int wide) {
-    PCell c;
-    float2 f;
-    c.bz = 0;
-    c.fz = 0.f;
-    if (wide) {
-        c.bx = pcell1_wide(axy.x, lo, P.fn[0], fw, f.x);
-        c.by = pcell1_wide(axy.y, lo, P.fn[1], fw, f.y);
-        if (DIM == 3) c.bz = pcell1_wide(az, lo, P.fn[2], fw, c.fz);
-    } else {
-        pcell2(axy, lo, P.fn[0], P.fn[1], fw, c.bx, c.by, f);
-        if (DIM == 3) c.bz = pcell1(az, lo, P.fn[2], fw, c.fz);
-    }
-    c.fx = f.x;
-    c.fy = f.y;
-    const uint32_t sy = (uint32_t)P.pnx, sz = DIM == 3 ? (uint32_t)P.pnxy : 0u;
-    c.base = (int32_t)(c.bz * sz + c.by * sy + c.bx - (PCELL_BITS - 1u) * (sz + sy + 1u));
-    return c;
-}
+__device__ __forceinline__ float frac256(float f) { return floorf(f * 256.0f + 0.5f) * (1.0f / 256.0f); }
 
 // lerp_ on a pair with one weight: each half equals lerp_ on that half bit for bit.
 __device__ __forceinline__ float2 lerp2_(float2 a, float2 b, float t) { return fma2(both(t), sub2(b, a), a); }
@@ -370,6 +352,14 @@ __device__ __forceinline__ float2 tri8p(const float2 (&c)[8], float fx, float fy
     const float2 a00 = fma2(tx, c[1], c[0]), a10 = fma2(tx, c[3], c[2]);
     const float2 a01 = fma2(tx, c[5], c[4]), a11 = fma2(tx, c[7], c[6]);
     return lerp2_(lerp2_(a00, a10, fy), lerp2_(a01, a11, fy), fz);
+}
+
+// Index of a cell's first corner in the padded pair: (iz + 1) pnxy + (iy + 1) pnx + (ix + 1) in wrapping
+// 32-bit arithmetic, with the patterns' offset removed by one loop-invariant term.
+template <int DIM>
+__device__ __forceinline__ int32_t padded_index(const KParams &P, const PCell &c) {
+    const uint32_t sy = (uint32_t)P.pnx, sz = DIM == 3 ? (uint32_t)P.pnxy : 0u;
+    return (int32_t)(c.bz * sz + c.by * sy + c.bx - (PCELL_BITS - 1u) * (sz + sy + 1u));
 }
 
 // Loads the 8 padded corners of the cell at `base` into the sample cache as 24 float pairs
@@ -391,7 +381,6 @@ __device__ __forceinline__ void fill_padded(const KParams &P, const void *pairs,
             cc.c2[q][k + 1] = sub2(b[q], a[q]);
         }
     }
-    cc.base = base;
 }
 
 // The four corners of a 2D cell from the window pair.
@@ -405,7 +394,6 @@ __device__ __forceinline__ void fill_edge2(const KParams &P, const void *pairs, 
         cc.c2d[0][k] = (k & 1) ? sub2(c[0], cc.c2d[0][k - 1]) : c[0];
         cc.c2d[1][k] = (k & 1) ? sub2(c[1], cc.c2d[1][k - 1]) : c[1];
     }
-    cc.base = base;
 }
 
 // The corners of a cell straight from two ring slots (unpadded grids, both snapshots): corner
@@ -462,7 +450,6 @@ __device__ __forceinline__ void fill_ring(const KParams &P, const void *wb, cons
 #pragma unroll
             for (int q = 0; q < 3; ++q) cc.c2[q][k + 1] = sub2(cc.c2[q][k + 1], cc.c2[q][k]);
     }
-    cc.base = c.base;
 }
 
 template <typename W> struct Elem { using type = W; };
@@ -474,8 +461,8 @@ template <int DIM, typename W>
 __device__ __forceinline__ void fill(const KParams &P, const void *wb, const void *wf, const PCell &c, SampleCache &cc) {
     using H = typename Elem<W>::type;
     if constexpr (!IsPair<W>::value) fill_ring<DIM, H>(P, wb, wf, c, cc);
-    else if constexpr (DIM == 3) fill_padded<H>(P, wb, c.base, cc);
-    else fill_edge2<H>(P, wb, c.base, cc);
+    else if constexpr (DIM == 3) fill_padded<H>(P, wb, padded_index<3>(P, c), cc);
+    else fill_edge2<H>(P, wb, padded_index<2>(P, c), cc);
 }
 
 // Horizontal components as a pair.
@@ -531,40 +518,99 @@ __device__ __forceinline__ float dot3(const V3 &a, const V3 &b, int dim) {
 }
 
 // World position -> grid coordinates.
-__device__ __forceinline__ float2 grid_xy(const KParams &P, float2 p) {
-    return mul2(add2(p, make_float2(P.noff[0], P.noff[1])), make_float2(P.inv_scale[0], P.inv_scale[1]));
-}
-__device__ __forceinline__ float grid_z(const KParams &P, float z) { return (z + P.noff[2]) * P.inv_scale[2]; }
+__device__ __forceinline__ float2 grid_xy(const KParams &P, float2 p) { return mul2(add2(p, P.noff2), P.inv2); }
+__device__ __forceinline__ float grid_z(const KParams &P, float z) { return (z + P.noffz) * P.inv_scale[2]; }
 
-// Cell of a sample at world position p.
-template <int DIM, typename W, int FT>
-__device__ __forceinline__ PCell cell_at(const KParams &P, const V3 &p) {
-    constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
-    const int fw = options ? P.filter_weights : 0;
-    const float lo = IsPair<W>::value || DIM == 2 ? -1.0f : P.flo;
-    const int wide = options && !IsPair<W>::value ? P.wide : 0;
-    return make_pcell<DIM>(P, grid_xy(P, p.xy), DIM == 3 ? grid_z(P, p.z) : 0.f, fw, lo, wide);
+// Loads the cell of a sample at grid coordinates (axy, az) outside the cached one; f, fz: its
+// fractions.  A coordinate outside the grid's range is clamped here, and the cell is not kept: a
+// neighbouring sample's fraction in it would be another one.
+template <int DIM, typename W>
+__device__ __forceinline__ void load_cell(const KParams &P, float2 axy, float az, bool wide, const void *wb,
+                                          const void *wf, float2 &f, float &fz, SampleCache &cc) {
+    PCell c = make_pcell<DIM>(axy, az);
+    const uint32_t first = PCELL_BITS - (uint32_t)P.below, more = 2u * (uint32_t)P.below;   // n + more cells
+    bool keep = true;
+    if (wide || c.bx - first >= (uint32_t)P.nx + more || c.by - first >= (uint32_t)P.ny + more ||
+        (DIM == 3 && c.bz - first >= (uint32_t)P.nz + more)) {
+        const float2 a = axy;
+        const float b = az;
+        axy.x = fminf(fmaxf(axy.x, P.flo), P.fn[0]);
+        axy.y = fminf(fmaxf(axy.y, P.flo), P.fn[1]);
+        if (DIM == 3) az = fminf(fmaxf(az, P.flo), P.fn[2]);
+        if (wide) {
+            c.bx = pcell1_wide(axy.x, c.nxy.x);
+            c.by = pcell1_wide(axy.y, c.nxy.y);
+            if (DIM == 3) c.bz = pcell1_wide(az, c.nz);
+        } else {
+            c = make_pcell<DIM>(axy, az);
+        }
+        keep = a.x == axy.x && a.y == axy.y && (DIM == 2 || b == az);
+    }
+    f = add2(axy, c.nxy);
+    if (DIM == 3) fz = az + c.nz;
+    if (!keep) cc.reset();
+    else cc.nxy = c.nxy, cc.nz = c.nz;
+    fill<DIM, W>(P, wb, wf, c, cc);
+}
+
+// The cell and fractions of every sample, clamped, and its padded node index for a key.
+__device__ __forceinline__ PCell clamped_cell(const KParams &P, float2 axy, float az, float2 &f, float &fz) {
+    axy.x = fminf(fmaxf(axy.x, -1.0f), P.fn[0]);
+    axy.y = fminf(fmaxf(axy.y, -1.0f), P.fn[1]);
+    az = fminf(fmaxf(az, -1.0f), P.fn[2]);
+    const PCell c = make_pcell<3>(axy, az);
+    f = add2(axy, c.nxy);
+    fz = az + c.nz;
+    return c;
 }
 
 // Wind at world position p, time weight t: interpolate() of TrajectoryIntegrator.icc:42-110.  The
 // cell's corners come from the sample cache, reloaded when the cell changes (wb: the window pair; or
 // wb, wf: the ring slots), interpolated in space, then in time.
+// 2D and ring slots: a sample lies in the cached cell when its coordinates minus the cell's first
+// corner are in [0, 1), one unsigned comparison of the bits each; those differences are then its
+// fractions (a - floor(a) bit for bit: the same subtraction), and nothing of the cell's search is
+// left on the way of such a sample.  (A fraction that rounds to 1 loads the same cell again.)
+// 3D pairs: some lane of nearly every warp loads a cell at nearly every sample, so the search is on
+// the warp's way in any case and goes before the test, where it costs no latency.  Measured, search
+// first against differences first: 1e6 particles x 300 steps 7.03 / 7.16 ms of step launches, 300,000 x 200
+// 2.30 / 2.33, 2D sphere 150,000 x 200 0.75 / 0.72, bf16 ring slots 777,777 x 100 2.66 / 2.61 ms.
 // FT: the step kernel's feature set; lean variants run with filter_weights off (kernel_features).
 template <int DIM, typename W, int FT>
 __device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf,
                                       SampleCache &cc) {
-    const PCell c = cell_at<DIM, W, FT>(P, p);
-    if (!IsPair<W>::value && (!(FT & FT_LEAN) || (FT & FT_BORDER)) && P.wide) cc.reset();
-    if (c.base != cc.base) fill<DIM, W>(P, wb, wf, c, cc);
+    constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
+    const float2 axy = grid_xy(P, p.xy);
+    const float az = DIM == 3 ? grid_z(P, p.z) : 0.f;
+    float2 fr;
+    float fz = 0.f;
+    if constexpr (IsPair<W>::value && DIM == 3) {
+        const PCell c = clamped_cell(P, axy, az, fr, fz);
+        const int32_t base = padded_index<3>(P, c);
+        if (base != cc.base) {
+            cc.base = base;
+            fill<DIM, W>(P, wb, wf, c, cc);
+        }
+    } else {
+        fr = add2(axy, cc.nxy);
+        if (DIM == 3) fz = az + cc.nz;
+        constexpr uint32_t one = 0x3f800000u;
+        if (__float_as_uint(fr.x) >= one || __float_as_uint(fr.y) >= one || (DIM == 3 && __float_as_uint(fz) >= one))
+            load_cell<DIM, W>(P, axy, az, options && !IsPair<W>::value && P.wide, wb, wf, fr, fz, cc);
+    }
+    if (options && P.filter_weights) {
+        fr = make_float2(frac256(fr.x), frac256(fr.y));
+        fz = frac256(fz);
+    }
     const bool dynamic = IsPair<W>::value || (FT & FT_LEAN) || P.wind_dynamic;
     if constexpr (DIM == 3) {
-        const float2 b = tri8p(cc.c2[0], c.fx, c.fy, c.fz), f = tri8p(cc.c2[1], c.fx, c.fy, c.fz);
-        const float2 w = tri8p(cc.c2[2], c.fx, c.fy, c.fz);
+        const float2 b = tri8p(cc.c2[0], fr.x, fr.y, fz), f = tri8p(cc.c2[1], fr.x, fr.y, fz);
+        const float2 w = tri8p(cc.c2[2], fr.x, fr.y, fz);
         return dynamic ? V3{lerp2_(b, f, t), lerp_(w.x, w.y, t)} : V3{b, w.x};
     } else {
-        const float2 tx = both(c.fx);
-        const float2 b = lerp2_(fma2(tx, cc.c2d[0][1], cc.c2d[0][0]), fma2(tx, cc.c2d[0][3], cc.c2d[0][2]), c.fy);
-        const float2 f = lerp2_(fma2(tx, cc.c2d[1][1], cc.c2d[1][0]), fma2(tx, cc.c2d[1][3], cc.c2d[1][2]), c.fy);
+        const float2 tx = both(fr.x);
+        const float2 b = lerp2_(fma2(tx, cc.c2d[0][1], cc.c2d[0][0]), fma2(tx, cc.c2d[0][3], cc.c2d[0][2]), fr.y);
+        const float2 f = lerp2_(fma2(tx, cc.c2d[1][1], cc.c2d[1][0]), fma2(tx, cc.c2d[1][3], cc.c2d[1][2]), fr.y);
         return V3{dynamic ? lerp2_(b, f, t) : b, 0.f};
     }
 }
@@ -838,8 +884,9 @@ constexpr int GR_ADV_MIN_BLOCKS = 2, GR_F32_BLOCKS = 4, GR_LIGHT_BLOCKS = 5;   /
 
 // Advances the particle in slot i through steps [s0, s1) (or until its lifetime ends).
 template <int DIM, bool RK4, typename W, int FT>
-__device__ __forceinline__ void advance_particle(const KParams &P, const int64_t i, const int64_t n_live,
-                                                 unsigned long long &steps_acc) {
+// Slots and particle ids are below 2^31 (checked where seeds are set).
+__device__ __forceinline__ void advance_particle(const KParams &P, const int32_t i, const int32_t n_live,
+                                                 unsigned &steps_acc) {
     // options: runtime values in the generic variant; in a lean variant (FT_LEAN) the ones the
     // host checked are off, and curvature / extras are the variant's compile-time choice
     constexpr bool LEAN = (FT & FT_LEAN) != 0;
@@ -853,7 +900,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     const bool valid = i < n_live;
     int32_t st = valid ? P.status[i] : 1;
     bool alive = st == 0;
-    const int64_t pid = valid && P.id ? (int64_t)P.id[i] : 0;   // no ids: a launch without records
+    const int32_t pid = valid && P.id ? P.id[i] : 0;   // no ids: a launch without records
 
     const V3 zero{{0.f, 0.f}, 0.f};
     V3 p = zero, q = zero, comp = zero, ld = zero;
@@ -876,9 +923,11 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
         if (curvature_mode == 3) cv = P.curv[i];
     }
     const bool was_alive = alive;
-    unsigned long long my_steps = 0;
+    unsigned my_steps = 0;
     const int32_t life = (valid && P.life) ? P.life[i] : 0x7fffffff;   // steps this particle may run
-    const int32_t birth = (valid && P.birth) ? P.birth[i] : 0;          // first step it runs
+    // first step it runs: the request server's, which takes positions only
+    constexpr bool births = (FT & (FT_CURV | FT_EXTRAS | FT_COMP | FT_DEFER)) == 0;
+    const int32_t birth = births && valid && P.birth ? P.birth[i] : 0;
     const bool extras = LEAN ? (FT & FT_EXTRAS) != 0 : ((P.volume_mode != 0 && P.nvol > 0) || P.nexpr > 0);
     V3 vc_last = zero;
     int last_s = P.s0;
@@ -889,8 +938,17 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
     cc.reset();
     int slot = -1;   // ring layouts: back slot of the cached cell
     for (int s = P.s0; s < P.s1; ++s) {
-        const StepEntry E = P.sched[s];
-        const int sb = P.wind_dynamic ? E.slot_back : 0, sf = P.wind_dynamic ? E.slot_front : 0;
+        // the step's time weights and flags; the rest of its entry where it is used, so that no register
+        // holds it over the step
+        const StepEntry *const entry = P.sched + s;
+        const int4 head = __ldg(reinterpret_cast<const int4 *>(entry));
+        struct {
+            float t0, t1, t2;
+            int flags;
+        } const E{__int_as_float(head.x), __int_as_float(head.y), __int_as_float(head.z), head.w};
+        int2 slots = make_int2(0, 0);
+        if (!IsPair<W>::value && P.wind_dynamic) slots = __ldg(reinterpret_cast<const int2 *>(&entry->slot_back));
+        const int sb = slots.x, sf = slots.y;
         const void *wb = IsPair<W>::value ? P.pair : reinterpret_cast<const char *>(P.wind) + (int64_t)sb * P.wind_stride;
         const void *wf = reinterpret_cast<const char *>(P.wind) + (int64_t)sf * P.wind_stride;
         // the cached cell belongs to the window's two snapshots
@@ -898,7 +956,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
             cc.reset();
             slot = sb;
         }
-        if (alive && s < life && s >= birth) {
+        if (alive && s < life && (!births || s >= birth)) {
             ++my_steps;
             const float t0 = P.dyn_any ? E.t0 : 0.f;
 
@@ -928,12 +986,11 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                         if (DIM == 3) acc.z = __fmaf_rn(wgt, k.z, acc.z);
                         if (sph) accc.xy = fma2(both(wgt), kc.xy, accc.xy);
                     }
-                    const float c = stage < 2 ? P.hh : P.h;
-                    a.xy = fma2(k.xy, both(c), p.xy);
-                    if (DIM == 3) a.z = __fmaf_rn(k.z, c, p.z);
+                    a.xy = fma2(k.xy, stage < 2 ? P.hh2 : P.h2, p.xy);
+                    if (DIM == 3) a.z = __fmaf_rn(k.z, stage < 2 ? P.hh : P.h, p.z);
                 }
-                v = V3{mul2(acc.xy, both(P.sixth)), DIM == 3 ? acc.z * P.sixth : 0.f};
-                vc = sph ? V3{mul2(accc.xy, both(P.sixth)), 0.f} : v;
+                v = V3{mul2(acc.xy, P.sixth2), DIM == 3 ? acc.z * P.sixth : 0.f};
+                vc = sph ? V3{mul2(accc.xy, P.sixth2), 0.f} : v;
             } else {
                 vc = wind_at<DIM, W, FT>(P, p, t0, wb, wf, cc);
                 v = sph ? sphere_(P, p.xy.y, vc) : vc;
@@ -943,12 +1000,12 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
             // negated displacement: without uplift that is the forward step, bit for bit, so the
             // lean variants leave the option out.
             const bool reverse = !LEAN && P.reverse;
-            V3 dp{mul2(v.xy, both(P.h)), DIM == 3 ? v.z * P.h : 0.f};
+            V3 dp{mul2(v.xy, P.h2), DIM == 3 ? v.z * P.h : 0.f};
             if (reverse) { dp.xy = make_float2(-dp.xy.x, -dp.xy.y); dp.z = -dp.z; }
             if (DIM == 3 && uplift_mode != 0) {
-                const int lb = uplift_mode == 2 ? E.slot_back : 0, lf = uplift_mode == 2 ? E.slot_front : 0;
-                const float *LB = P.lift + (int64_t)lb * P.n_total * 3 + pid * 3;
-                const float *LF = P.lift + (int64_t)lf * P.n_total * 3 + pid * 3;
+                const int lb = uplift_mode == 2 ? __ldg(&entry->slot_back) : 0, lf = uplift_mode == 2 ? __ldg(&entry->slot_front) : 0;
+                const float *LB = P.lift + ((int64_t)lb * P.n_total + pid) * 3;
+                const float *LF = P.lift + ((int64_t)lf * P.n_total + pid) * 3;
                 if (uplift_mode == 1) {
                     dp.xy = add2(dp.xy, make_float2(LB[0], LB[1])); dp.z = dp.z + LB[2];
                 } else {
@@ -994,7 +1051,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
             if (abort == 0) {
                 const float dp2 = dot3(dp, dp, DIM);
                 const int bm = DIM == 3 ? 0 : border_mode;
-                const float2 rel = add2(np.xy, make_float2(P.noff[0], P.noff[1]));   // np - off
+                const float2 rel = add2(np.xy, P.noff2);   // np - off
                 if (bm == 0) {
                     bool topo = false;
                     if (DIM == 3 && topography) {
@@ -1006,7 +1063,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                     else {
                         bool out = rel.x > P.dom[0] || rel.x < 0.f || rel.y > P.dom[1] || rel.y < 0.f;
                         if (DIM == 3) {
-                            const float rz = np.z + P.noff[2];
+                            const float rz = np.z + P.noffz;
                             out = out || rz > P.dom[2] || rz < 0.f;
                         }
                         if (out) abort = 2;
@@ -1070,8 +1127,8 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
                             // central differences scaled by the float reciprocals of 2 h and h h
                             // (the reference divides, icc:151-154: within one rounding of these);
                             // the fused (q + np) - 2 p rounds like the separate one (2 p is exact)
-                            const V3 d1{mul2(sub2(np.xy, q.xy), both(P.inv_2h)), (np.z - q.z) * P.inv_2h};
-                            const V3 d2{mul2(fma2(p.xy, both(-2.f), add2(q.xy, np.xy)), both(P.inv_hh)),
+                            const V3 d1{mul2(sub2(np.xy, q.xy), P.i2h2), (np.z - q.z) * P.inv_2h};
+                            const V3 d2{mul2(fma2(p.xy, both(-2.f), add2(q.xy, np.xy)), P.ihh2),
                                         __fmaf_rn(-2.f, p.z, q.z + np.z) * P.inv_hh};
                             const V3 x{{d1.xy.y * d2.z - d1.z * d2.xy.y, d1.z * d2.xy.x - d1.xy.x * d2.z},
                                        d1.xy.x * d2.xy.y - d1.xy.y * d2.xy.x};
@@ -1100,25 +1157,38 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
         }
 
         if (valid && (E.flags & SF_SAVE)) {
-            float *hp = P.hpos + ((int64_t)E.rec * P.n_total + pid) * DIM;
+            float *hp = P.hpos + ((int64_t)__ldg(&entry->rec) * P.n_total + pid) * DIM;
             hp[0] = p.xy.x; hp[1] = p.xy.y;
             if (DIM == 3) hp[2] = p.z;
-            if (curvature_mode == 3 && (E.flags & SF_CURV_REC)) P.hcurv[(int64_t)E.crec * P.n_total + pid] = cv;
+            if (curvature_mode == 3 && (E.flags & SF_CURV_REC)) P.hcurv[(int64_t)__ldg(&entry->crec) * P.n_total + pid] = cv;
             if constexpr ((FT & FT_DEFER) != 0) {
                 // the record's inputs: the position and the last moved step's (if any since the
                 // last evaluation)
                 const float4 v = P.vlast[i];
-                P.vrec[2 * i] = make_float4(p.xy.x, p.xy.y, DIM == 3 ? p.z : 0.f, 0.f);
-                P.vrec[2 * i + 1] = v;
+                P.vrec[2 * (int64_t)i] = make_float4(p.xy.x, p.xy.y, DIM == 3 ? p.z : 0.f, 0.f);
+                P.vrec[2 * (int64_t)i + 1] = v;
                 if (__float_as_int(v.w) >= 0) reinterpret_cast<int32_t *>(P.vlast + i)[3] = -1;
             }
             if (extras) {
-                record_extras<DIM>(P, i, pid, dirty, last_s, p, vc_last, cv, E.irec);
+                record_extras<DIM>(P, i, pid, dirty, last_s, p, vc_last, cv, __ldg(&entry->irec));
                 dirty = false;
                 // refill the sample cache for the next step's first sample (at p): the cached
                 // nodes are then dead while the values above are evaluated, which frees their
                 // registers there
-                if constexpr (DIM == 3) fill<DIM, W>(P, wb, wf, cell_at<DIM, W, FT>(P, p), cc);
+                if constexpr (DIM == 3) {
+                    float2 f;
+                    float fz;
+                    const float2 axy = grid_xy(P, p.xy);
+                    const float az = grid_z(P, p.z);
+                    if constexpr (IsPair<W>::value) {
+                        const PCell c = clamped_cell(P, axy, az, f, fz);
+                        cc.base = padded_index<3>(P, c);
+                        fill<3, W>(P, wb, wf, c, cc);
+                    } else {
+                        constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
+                        load_cell<3, W>(P, axy, az, options && P.wide, wb, wf, f, fz, cc);
+                    }
+                }
             }
         }
 
@@ -1153,8 +1223,10 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int64_t
 // Launch bounds: 256 threads, 2 blocks per SM (128 registers).  The float32 3D kernels keep 48
 // cached floats in 128-thread blocks: 4 per SM (128 registers) in the generic variant and the lean
 // ones with volume / expression values or with both Kahan positions and curvature, 5 per SM (96
-// registers, 20 warps) in the other lean ones, whose state fits there without spills; the extra warps
-// hide more of the sampling and curvature latency.  16-bit 3D kernels: 128 x 5 for the lean variants
+// registers, 20 warps) in the other lean ones on window pairs, whose state fits there without spills;
+// the extra warps hide more of the sampling and curvature latency.  Ring slots stay at 4 blocks: with 16
+// loads in flight 96 registers spill in the step loop (gr_advance_noalloc, 500,001 particles x 20
+// steps, 0.49 ms against 0.44).  16-bit 3D kernels: 128 x 5 for the lean variants
 // with curvature or deferred values (measured 5-6% faster than 256 x 2 on the 3D benchmark
 // configuration), 256 x 2 for the rest (the positions-only variant of the batching and serving forms
 // measured 2% slower at 128 x 5).
@@ -1165,24 +1237,25 @@ template <int DIM, typename W, int FT> struct AdvBounds {
                                   (f32 || (FT & (FT_CURV | FT_DEFER)) != 0);
     static constexpr bool small = DIM == 3 && (f32 || light);   // 128-thread blocks
     static constexpr int threads = small ? 128 : 256;
-    static constexpr int blocks = !small ? GR_ADV_MIN_BLOCKS : light ? GR_LIGHT_BLOCKS : GR_F32_BLOCKS;
+    static constexpr int blocks = !small ? GR_ADV_MIN_BLOCKS : light && IsPair<W>::value ? GR_LIGHT_BLOCKS : GR_F32_BLOCKS;
 };
 
 template <int DIM, bool RK4, typename W, int FT>
 __global__ void __launch_bounds__(AdvBounds<DIM, W, FT>::threads, AdvBounds<DIM, W, FT>::blocks)
     advance_kernel(const __grid_constant__ KParams P) {
-    const int64_t n_live = P.n_dev ? (int64_t)*P.n_dev : P.n;
-    unsigned long long steps = 0;
+    const int32_t n_live = P.n_dev ? *P.n_dev : (int32_t)P.n;
+    unsigned steps = 0;   // of this thread
     if (P.grid_stride) {
         const int64_t stride = (int64_t)gridDim.x * blockDim.x;
         for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_live; base += stride)
-            advance_particle<DIM, RK4, W, FT>(P, base + threadIdx.x, n_live, steps);
+            advance_particle<DIM, RK4, W, FT>(P, (int32_t)(base + threadIdx.x), n_live, steps);
     } else {
-        advance_particle<DIM, RK4, W, FT>(P, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_live, steps);
+        advance_particle<DIM, RK4, W, FT>(P, (int32_t)(blockIdx.x * blockDim.x + threadIdx.x), n_live, steps);
     }
-    // particle-steps, warp-aggregated
-    const unsigned long long warp_steps = __reduce_add_sync(0xffffffffu, (unsigned)steps);
-    if ((threadIdx.x & 31) == 0 && warp_steps) atomicAdd(P.counters, warp_steps);
+    // particle-steps, warp-aggregated (a block may be less than a warp)
+    const unsigned lanes = __activemask();
+    const unsigned warp_steps = __reduce_add_sync(lanes, steps);
+    if ((int)(threadIdx.x & 31) == __ffs(lanes) - 1 && warp_steps) atomicAdd(P.counters, (unsigned long long)warp_steps);
 }
 
 }  // namespace granite_b200

@@ -132,7 +132,6 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
         P.scale[d] = scale[d];
         P.inv_scale[d] = 1.0f / scale[d];
         P.off[d] = off[d];
-        P.noff[d] = -off[d];
         P.dom[d] = g[d] * scale[d];
     }
     P.nx = (int32_t)nx; P.ny = (int32_t)ny; P.nz = (int32_t)(dim == 3 ? nz : 1); P.dim = dim;
@@ -149,11 +148,7 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
     P.counters = S->counters;
     P.s0 = 0;
     P.s1 = steps;
-    P.h = h;
-    P.hh = 0.5f * h;
-    P.sixth = 1.0f / 6;
-    P.inv_2h = 1.0f / (2.0f * h);
-    P.inv_hh = 1.0f / (h * h);
+    derive_params(P, h);
     P.sphere_radius = s->sphere_radius;
     P.filter_weights = s->filter_weights ? 1 : 0;
     P.wind_dynamic = 1;
@@ -161,11 +156,12 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
     P.border_mode = dim == 2 ? s->border_mode : 0;
     P.reverse = s->reverse ? 1 : 0;
     P.sphere = dim == 2 && s->sphere_radius > 0.f;
-    // the step kernel of the engine, reading the caller's two snapshots as ring slots (one thread
-    // per particle; 32-thread blocks spread a small set over the SMs)
+    // the step kernel of the engine, reading the caller's two snapshots as ring slots, one thread per
+    // particle
     const AdvanceFn fn = advance_f32(dim, s->integrator == 1, false, kernel_features(P));
-    int threads = 128;
-    while (threads > 32 && (n + threads - 1) / threads < 2 * 148) threads /= 2;
+    int threads = block_of_few(n);
+    if (threads == 0)
+        for (threads = 128; threads > 32 && (n + threads - 1) / threads < 2 * 148;) threads /= 2;
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (n + threads - 1) / threads);
     fn<<<blocks, threads, 0, st>>>(P);
     if (cudaGetLastError() != cudaSuccess) return err(GR_ERR_RUNTIME, "ERROR < RUNTIME | launch failed >");

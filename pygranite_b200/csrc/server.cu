@@ -449,7 +449,6 @@ KParams pool_params(gr_server *S, Pool &P) {
     for (int d = 0; d < 3; ++d) {
         K.inv_scale[d] = S->inv_scale[d];
         K.off[d] = S->off[d];
-        K.noff[d] = -S->off[d];
         K.dom[d] = S->dom[d];
         K.scale[d] = S->scale[d];
     }
@@ -467,11 +466,7 @@ KParams pool_params(gr_server *S, Pool &P) {
     K.grid_stride = 1;
     K.sched = S->d_sched.p;
     const gr_settings &s = S->s;
-    K.h = s.delta_t;
-    K.hh = 0.5f * s.delta_t;
-    K.sixth = 1.0f / 6;
-    K.inv_2h = 1.0f / (2.0f * s.delta_t);
-    K.inv_hh = 1.0f / (s.delta_t * s.delta_t);
+    derive_params(K, s.delta_t);
     K.sphere_radius = s.sphere_radius;
     K.wind_dynamic = 1;
     K.dyn_any = 1;
