@@ -71,25 +71,41 @@ namespace {
 
 // ------------------------------------------------------------------ aux kernels
 
-// Seeds (AoS, n x dim) -> state SoA; zeroes the per-particle accumulators.
-__global__ void seed_kernel(const float *__restrict__ seeds, int64_t n, int dim, float *px, float *py,
-                            float *pz, int32_t *status, int32_t *id, const int32_t *__restrict__ life_src,
-                            int32_t *life) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        px[i] = seeds[i * dim];
-        py[i] = seeds[i * dim + 1];
-        if (dim == 3) pz[i] = seeds[i * dim + 2];
-        status[i] = 0;
-        id[i] = (int32_t)i;
-        if (life_src) life[i] = life_src[i];
-    }
-}
+// Start of a run: seeds (AoS, n x dim) -> state SoA and record 0 of the history, the first row of the
+// record-major history (TrajectoryIntegrator.cpp:424-442); zeroed accumulators, counters and counts.
+// One launch instead of three kernels and eight memsets.
+struct StartParams {
+    const float *seeds;
+    int64_t n;
+    int32_t dim, nzero;
+    float *px, *py, *pz, *hpos;
+    int32_t *status, *id, *life, *retired;
+    const int32_t *life_src;
+    float4 *vlast;
+    float *zero[24];       // nzero arrays of n values
+    int32_t *counts;       // live, live after the last pass, retired
+    unsigned long long *counters;
+};
 
-// Record 0 of the history = the seeds (TrajectoryIntegrator.cpp:424-442): the first row of the
-// record-major history.
-__global__ void seed_record_kernel(const float *__restrict__ seeds, int64_t n, int dim, float *hpos) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * dim; i += (int64_t)gridDim.x * blockDim.x)
-        hpos[i] = seeds[i];
+__global__ void start_kernel(const __grid_constant__ StartParams S) {
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    if (first == 0) {
+        S.counts[0] = S.counts[1] = (int32_t)S.n;
+        S.counts[2] = S.counts[3] = 0;
+        S.counters[0] = 0ull;
+    }
+    for (int64_t i = first; i < S.n; i += stride) {
+        S.px[i] = S.seeds[i * S.dim];
+        S.py[i] = S.seeds[i * S.dim + 1];
+        if (S.dim == 3) S.pz[i] = S.seeds[i * S.dim + 2];
+        S.status[i] = 0;
+        S.id[i] = (int32_t)i;
+        if (S.life_src) S.life[i] = S.life_src[i];
+        if (S.retired) S.retired[i] = 0x7f7f7f7f;   // never
+        if (S.vlast) S.vlast[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));   // no step to evaluate
+        for (int k = 0; k < S.nzero; ++k) S.zero[k][i] = 0.f;
+    }
+    for (int64_t i = first; i < S.n * S.dim; i += stride) S.hpos[i] = S.seeds[i];
 }
 
 // Records of particles that left the live set (retired at compaction) are not written after
@@ -946,13 +962,6 @@ int alloc_state(gr_engine *e) {
     return GR_OK;
 }
 
-__global__ void init_counts_kernel(int32_t *counts, int32_t n) {
-    counts[0] = n;   // live
-    counts[1] = n;   // live after the last pass
-    counts[2] = 0;   // retired
-    counts[3] = 0;
-}
-
 // Device start of a run on the compute stream: zeroed accumulators and counters, live and
 // retired counts, seeds -> state, record 0.  Capturable.
 int reset_state(gr_engine *e) {
@@ -960,32 +969,30 @@ int reset_state(gr_engine *e) {
     const size_t N = (size_t)n;
     e->cur = 0;
     gr_engine::State &S = e->st[0];
-    if (e->s.compensated) {
-        CK(cudaMemsetAsync(S.kx.p, 0, N * 4, e->cs)); CK(cudaMemsetAsync(S.ky.p, 0, N * 4, e->cs));
-        CK(cudaMemsetAsync(S.kz.p, 0, N * 4, e->cs));
-    }
-    if (e->s.curvature_mode == 2) {
-        CK(cudaMemsetAsync(S.lx.p, 0, N * 4, e->cs)); CK(cudaMemsetAsync(S.ly.p, 0, N * 4, e->cs));
-        CK(cudaMemsetAsync(S.lz.p, 0, N * 4, e->cs));
-    }
-    CK(cudaMemsetAsync(S.length.p, 0, N * 4, e->cs));
-    CK(cudaMemsetAsync(S.tc.p, 0, N * 4, e->cs));
-    CK(cudaMemsetAsync(S.curv.p, 0, N * 4, e->cs));
-    const int nv = std::max(1, e->nvol), ne = std::max(1, e->nexpr);
-    CK(cudaMemsetAsync(S.volc.p, 0, N * nv * 4, e->cs));
-    CK(cudaMemsetAsync(S.cmpc.p, 0, N * ne * 4, e->cs));
-    if (S.vlast.p) CK(cudaMemsetAsync(S.vlast.p, 0xff, N * sizeof(float4), e->cs));   // step index -1
-    init_counts_kernel<<<1, 1, 0, e->cs>>>(e->d_counts.p, (int32_t)n);
-    const int threads = 256;
-    seed_kernel<<<grid_for(n, threads), threads, 0, e->cs>>>(e->seeds.p, n, e->dim, S.px.p, S.py.p, S.pz.p,
-                                                             S.status.p, S.id.p,
-                                                             e->has_life ? e->life_src.p : nullptr, S.life.p);
-    seed_record_kernel<<<grid_for(n * e->dim, threads), threads, 0, e->cs>>>(e->seeds.p, n, e->dim, e->hpos.p);
+    StartParams T{};
+    T.seeds = e->seeds.p;
+    T.n = n;
+    T.dim = e->dim;
+    T.px = S.px.p; T.py = S.py.p; T.pz = S.pz.p;
+    T.hpos = e->hpos.p;
+    T.status = S.status.p; T.id = S.id.p; T.life = S.life.p;
+    T.life_src = e->has_life ? e->life_src.p : nullptr;
+    T.retired = e->ret_rec.p;
+    T.vlast = S.vlast.p;
+    T.counts = e->d_counts.p;
+    T.counters = e->counters.p;
+    auto zero = [&](float *a) { T.zero[T.nzero++] = a; };   // at most 6 + 3 + 8 + 4
+    if (e->s.compensated)
+        for (float *a : {S.kx.p, S.ky.p, S.kz.p}) zero(a);
+    if (e->s.curvature_mode == 2)
+        for (float *a : {S.lx.p, S.ly.p, S.lz.p}) zero(a);
+    for (float *a : {S.length.p, S.tc.p, S.curv.p}) zero(a);
+    for (int k = 0; k < std::max(1, e->nvol); ++k) zero(S.volc.p + (size_t)k * N);
+    for (int k = 0; k < std::max(1, e->nexpr); ++k) zero(S.cmpc.p + (size_t)k * N);
+    start_kernel<<<grid_for(n, 256), 256, 0, e->cs>>>(T);
     CK(cudaGetLastError());
-    if (e->ret_rec.p) CK(cudaMemsetAsync(e->ret_rec.p, 0x7f, (size_t)n * sizeof(int32_t), e->cs));   // never retired
-    CK(cudaMemsetAsync(e->counters.p, 0, sizeof(unsigned long long), e->cs));
     if (e->compacting) *e->h_live = (int32_t)n;
-    e->stats.aux_launches += 3;
+    e->stats.aux_launches++;
     return GR_OK;
 }
 
@@ -2144,13 +2151,14 @@ int graph_enqueue(gr_engine *e) {
     if (rc) return rc;
     rc = sort_seeds(r);
     if (rc) return rc;
-    rc = launch_range(r, 0, R.nsteps);
-    if (rc < 0) return rc;
     RecordCounts c;
-    rc = run_tail(r, c);
-    if (rc) return rc;
-    rc = settle_pairs(e);   // a capture ends with every branch joined
-    if (rc) return rc;
+    rc = launch_range(r, 0, R.nsteps);
+    if (rc >= 0) rc = run_tail(r, c);
+    if (rc == GR_OK) rc = settle_pairs(e);   // a capture ends with every branch joined
+    if (rc) {
+        e->pair_pending[0] = e->pair_pending[1] = false;   // their events belong to the failed capture
+        return rc;
+    }
     e->graph_executed = r.executed;
     e->graph_records = c.rec;
     return GR_OK;
