@@ -225,6 +225,56 @@ static inline void launch_compaction(const CompactParams &C, int64_t n, cudaStre
 }
 constexpr int COMPACTION_LAUNCHES = 3;
 
+// Morton ranks of a box of nbx x nby x nbz bricks (each below 1024): a brick's rank is the number of
+// bricks with smaller codes, summed level by level over the octants before its own, each clipped to
+// the box.  (Sorting the codes of 73,728 bricks on the host took 3 ms of every engine's first run.)
+static __global__ void morton_rank_kernel(int32_t *rank, int32_t nbx, int32_t nby, int32_t nbz) {
+    const int32_t lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= nbx * nby * nbz) return;
+    const int32_t x = lin % nbx, y = lin / nbx % nby, z = lin / nbx / nby;
+    int32_t below = 0, cx = 0, cy = 0, cz = 0;   // (cx, cy, cz): corner of the octant descended into
+    for (int b = 9; b >= 0; --b) {
+        const int32_t size = 1 << b;
+        const int own = (x >> b & 1) | (y >> b & 1) << 1 | (z >> b & 1) << 2;
+        for (int o = 0; o < own; ++o) {
+            const int32_t ox = cx + (o & 1) * size, oy = cy + (o >> 1 & 1) * size, oz = cz + (o >> 2) * size;
+            below += max(min(size, nbx - ox), 0) * max(min(size, nby - oy), 0) * max(min(size, nbz - oz), 0);
+        }
+        cx += (x >> b & 1) * size;
+        cy += (y >> b & 1) * size;
+        cz += (z >> b & 1) * size;
+    }
+    rank[lin] = below;
+}
+
+// The bricks of a grid that compaction sorts by: 4 x 4 x 2 nodes (4 x 4 in 2D), larger where there
+// would be more than MAX_BINS of them, and their Morton ranks.
+struct Bricks {
+    int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
+    DevBuf<int32_t> rank;
+    cudaError_t build(int dim, int64_t nx, int64_t ny, int64_t nz, cudaStream_t stream) {
+        bx = 4; by = 4; bz = dim == 3 ? 2 : 1;
+        for (;;) {
+            nbx = (int)((nx + bx - 1) / bx);
+            nby = (int)((ny + by - 1) / by);
+            nbz = (int)((nz + bz - 1) / bz);
+            if ((int64_t)nbx * nby * nbz <= MAX_BINS && nbx <= 1024 && nby <= 1024 && nbz <= 1024) break;
+            bx *= 2; by *= 2; if (dim == 3) bz *= 2;
+        }
+        nbins = nbx * nby * nbz;
+        const cudaError_t e = rank.alloc((size_t)nbins);
+        if (e != cudaSuccess) return e;
+        morton_rank_kernel<<<(nbins + 255) / 256, 256, 0, stream>>>(rank.p, nbx, nby, nbz);
+        return cudaGetLastError();
+    }
+    void set(CompactParams &C) const {
+        C.bx = bx; C.by = by; C.bz = bz;
+        C.nbx = nbx; C.nby = nby; C.nbz = nbz;
+        C.nbins = nbins;
+        C.bintab = rank.p;
+    }
+};
+
 // Scratch of the passes: zeroed when it is allocated, left zero by every pass.
 struct CompactScratch {
     DevBuf<int32_t> hist, cursor, chunk, ticket;

@@ -273,9 +273,9 @@ struct gr_engine {
     DevBuf<int32_t> d_counts;          // [0] live, [1] live after a pass, [2] retired
     int32_t *h_live = nullptr;         // pinned copy of the live count
     cudaEvent_t live_ready = nullptr;
-    DevBuf<int32_t> c_key, c_bintab;
+    DevBuf<int32_t> c_key;
+    Bricks bricks;
     CompactScratch c_scratch;
-    int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
 
     DevBuf<float> hpos, hcurv, hvol, hcmp;   // record-major (KParams)
     DevBuf<float> stage[2], sstage;          // particle-major chunks for the fetch / the streaming
@@ -343,11 +343,7 @@ struct gr_engine {
         }
         if (ds) cudaStreamSynchronize(ds);
         if (ds_ev) cudaEventDestroy(ds_ev);
-        if (ds) cudaStreamDestroy(ds);
-        if (cs) cudaStreamDestroy(cs);
-        if (xs) cudaStreamDestroy(xs);
-        if (us) cudaStreamDestroy(us);
-        if (ps) cudaStreamDestroy(ps);
+        for (cudaStream_t st : {ds, cs, xs, us, ps}) stream_give(st, s.device);
     }
 };
 
@@ -594,8 +590,7 @@ int gr_create(const gr_settings *settings, gr_engine **out) {
     e->K = s.ring_slots >= 3 ? s.ring_slots : 3;
     if (e->K > 100000) return USER_ERR("ring_slots too large >");
     CK(cudaSetDevice(s.device));
-    CK(cudaStreamCreateWithFlags(&e->cs, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&e->xs, cudaStreamNonBlocking));
+    for (cudaStream_t *st : {&e->cs, &e->xs, &e->us, &e->ps}) CK(stream_take(st));
     e->slot_free.resize(e->K);
     e->slot_ready.resize(e->K);
     e->slot_used.assign(e->K, false);
@@ -604,8 +599,6 @@ int gr_create(const gr_settings *settings, gr_engine **out) {
         CK(cudaEventCreateWithFlags(&e->slot_ready[k], cudaEventDisableTiming));
     }
     CK(cudaEventCreateWithFlags(&e->upload_done, cudaEventDisableTiming));
-    CK(cudaStreamCreateWithFlags(&e->us, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&e->ps, cudaStreamNonBlocking));
     for (auto &ev : e->pair_ready) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&e->pair_go, cudaEventDisableTiming));
     for (auto &ev : e->raw_free) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -908,7 +901,7 @@ int alloc_set(gr_engine *e, gr_engine::State &S, bool retired) {
     return GR_OK;
 }
 
-// Device buffers and host tables of a run; enqueues no device work.
+// Device buffers and tables of a run.
 int alloc_state(gr_engine *e) {
     const size_t N = (size_t)e->n;
     int rc = alloc_set(e, e->st[0], false);
@@ -926,39 +919,8 @@ int alloc_state(gr_engine *e) {
     if (!e->h_live && gr_host_alloc(sizeof(int32_t), reinterpret_cast<void **>(&e->h_live)) != GR_OK)
         return GR_ERR_RUNTIME;
     if (!e->live_ready) CK(cudaEventCreateWithFlags(&e->live_ready, cudaEventDisableTiming));
-    if (e->nbins == 0) {
-        // Morton-ranked brick table (bricks of bx x by x bz nodes)
-        e->bx = 4; e->by = 4; e->bz = e->dim == 3 ? 2 : 1;
-        for (;;) {
-            e->nbx = (int)((e->nx + e->bx - 1) / e->bx);
-            e->nby = (int)((e->ny + e->by - 1) / e->by);
-            e->nbz = (int)((e->nz + e->bz - 1) / e->bz);
-            if ((int64_t)e->nbx * e->nby * e->nbz <= MAX_BINS && e->nbx <= 1024 && e->nby <= 1024 && e->nbz <= 1024) break;
-            e->bx *= 2; e->by *= 2; if (e->dim == 3) e->bz *= 2;
-        }
-        e->nbins = e->nbx * e->nby * e->nbz;
-        auto spread = [](uint32_t v) {
-            uint64_t x = v & 0x3ff;
-            x = (x | (x << 16)) & 0x030000FF;
-            x = (x | (x << 8)) & 0x0300F00F;
-            x = (x | (x << 4)) & 0x030C30C3;
-            x = (x | (x << 2)) & 0x09249249;
-            return x;
-        };
-        std::vector<std::pair<uint64_t, int32_t>> codes((size_t)e->nbins);
-        for (int z = 0; z < e->nbz; ++z)
-            for (int y = 0; y < e->nby; ++y)
-                for (int x = 0; x < e->nbx; ++x) {
-                    const int32_t lin = (z * e->nby + y) * e->nbx + x;
-                    codes[lin] = {spread(x) | (spread(y) << 1) | (spread(z) << 2), lin};
-                }
-        std::sort(codes.begin(), codes.end());
-        std::vector<int32_t> tab((size_t)e->nbins);
-        for (int32_t r = 0; r < e->nbins; ++r) tab[codes[r].second] = r;
-        CK(e->c_bintab.alloc(tab.size()));
-        CK(cudaMemcpy(e->c_bintab.p, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    }
-    CK(e->c_scratch.alloc(e->nbins));
+    if (e->bricks.nbins == 0) CK(e->bricks.build(e->dim, e->nx, e->ny, e->nz, e->cs));
+    CK(e->c_scratch.alloc(e->bricks.nbins));
     return GR_OK;
 }
 
@@ -1324,7 +1286,6 @@ int compact_pass(gr_engine *e, int32_t rec_now, int32_t k_end, bool graph) {
     C.ret.life = nullptr;
     C.key = e->c_key.p;
     e->c_scratch.set(C);
-    C.bintab = e->c_bintab.p;
     C.n_act = e->d_counts.p;
     C.n_new = e->d_counts.p + 1;
     C.n_ret = e->d_counts.p + 2;
@@ -1333,7 +1294,7 @@ int compact_pass(gr_engine *e, int32_t rec_now, int32_t k_end, bool graph) {
         C.inv_scale[d] = e->inv_scale[d];
     }
     C.nx = (int32_t)e->nx; C.ny = (int32_t)e->ny; C.nz = (int32_t)e->nz; C.dim = e->dim;
-    C.bx = e->bx; C.by = e->by; C.bz = e->bz; C.nbx = e->nbx; C.nby = e->nby; C.nbz = e->nbz; C.nbins = e->nbins;
+    e->bricks.set(C);
     const int cm = e->s.curvature_mode;
     C.nvol = (e->nvol > 0 && e->s.volume_mode != 0) ? e->nvol : 0;
     C.nexpr = e->nexpr;
@@ -1761,7 +1722,7 @@ int stream_begin(gr_engine *e, const RunPlan &R) {
         const int rc = check_info(d.compute_info[k]);
         if (rc) return rc;
     }
-    if (!e->ds) CK(cudaStreamCreateWithFlags(&e->ds, cudaStreamNonBlocking));
+    if (!e->ds) CK(stream_take(&e->ds));
     if (!e->ds_ev) CK(cudaEventCreateWithFlags(&e->ds_ev, cudaEventDisableTiming));
     e->dest_run = true;
     e->dest_during = e->s.minimum_alive == 0;

@@ -24,6 +24,9 @@ namespace granite_b200 {
 cudaError_t dev_alloc(void **p, size_t bytes);
 void dev_free(void *p);
 size_t dev_pool_idle_bytes();
+// Idle streams kept for reuse (memory.cu).
+cudaError_t stream_take(cudaStream_t *out);
+void stream_give(cudaStream_t st, int dev);
 
 inline int grid_for(int64_t n, int threads) {
     int64_t b = (n + threads - 1) / threads;

@@ -117,6 +117,52 @@ void dev_free(void *p) {
     if (a.device != cur) cudaSetDevice(cur);
 }
 
+// Streams of engines: creating and destroying four takes a millisecond, as long as a small run, so
+// idle ones are kept for the next engine of their device, up to kStreamsKept each.
+namespace {
+constexpr size_t kStreamsKept = 16;
+struct StreamPool {
+    std::mutex mu;
+    std::vector<cudaStream_t> idle[kMaxDevices];
+};
+// Never destroyed: an engine may be released after static destruction.
+StreamPool &streams() {
+    static StreamPool *p = new StreamPool;
+    return *p;
+}
+}  // namespace
+
+// A non-blocking stream of the current device.
+cudaError_t stream_take(cudaStream_t *out) {
+    int dev = 0;
+    const cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev >= 0 && dev < kMaxDevices) {
+        StreamPool &p = streams();
+        std::lock_guard<std::mutex> g(p.mu);
+        if (!p.idle[dev].empty()) {
+            *out = p.idle[dev].back();
+            p.idle[dev].pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+}
+
+// Gives a stream of device `dev` back once its work is done; one in error is destroyed.
+void stream_give(cudaStream_t st, int dev) {
+    if (!st) return;
+    if (cudaStreamSynchronize(st) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        StreamPool &p = streams();
+        std::lock_guard<std::mutex> g(p.mu);
+        if (p.idle[dev].size() < kStreamsKept) {
+            p.idle[dev].push_back(st);
+            return;
+        }
+    }
+    cudaStreamDestroy(st);
+}
+
 // Bytes the current device's pool holds mapped but unused (free to the library, not counted
 // as free by cudaMemGetInfo).
 size_t dev_pool_idle_bytes() {

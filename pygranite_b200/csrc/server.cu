@@ -169,9 +169,8 @@ struct gr_server {
     };
     Stage stage[2];
     int stage_next = 0;
-    DevBuf<int32_t> bintab;
+    Bricks bricks;
     CompactScratch scratch;
-    int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
     DevBuf<unsigned long long> counters;   // [0] particle-steps
     cudaStream_t cs = nullptr, xs = nullptr;
 
@@ -359,37 +358,8 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx, int64_t field_budget
     SK(S->raw.alloc((size_t)S->nodes * S->dim));
     S->host_snap.assign((size_t)S->n_snap, nullptr);
     for (int k = 0; k < kRing; ++k) S->ring_holds[k] = -1;
-    // Morton-ranked bricks for the pools' spatial sort (as in the engine)
-    S->bx = 4; S->by = 4; S->bz = S->dim == 3 ? 2 : 1;
-    for (;;) {
-        S->nbx = (int)((S->nx + S->bx - 1) / S->bx);
-        S->nby = (int)((S->ny + S->by - 1) / S->by);
-        S->nbz = (int)((S->nz + S->bz - 1) / S->bz);
-        if ((int64_t)S->nbx * S->nby * S->nbz <= MAX_BINS && S->nbx <= 1024 && S->nby <= 1024 && S->nbz <= 1024) break;
-        S->bx *= 2; S->by *= 2; if (S->dim == 3) S->bz *= 2;
-    }
-    S->nbins = S->nbx * S->nby * S->nbz;
-    auto spread = [](uint32_t v) {
-        uint64_t x = v & 0x3ff;
-        x = (x | (x << 16)) & 0x030000FF;
-        x = (x | (x << 8)) & 0x0300F00F;
-        x = (x | (x << 4)) & 0x030C30C3;
-        x = (x | (x << 2)) & 0x09249249;
-        return x;
-    };
-    std::vector<std::pair<uint64_t, int32_t>> codes((size_t)S->nbins);
-    for (int z = 0; z < S->nbz; ++z)
-        for (int y = 0; y < S->nby; ++y)
-            for (int x = 0; x < S->nbx; ++x) {
-                const int32_t lin = (z * S->nby + y) * S->nbx + x;
-                codes[lin] = {spread(x) | (spread(y) << 1) | (spread(z) << 2), lin};
-            }
-    std::sort(codes.begin(), codes.end());
-    std::vector<int32_t> tab((size_t)S->nbins);
-    for (int32_t r = 0; r < S->nbins; ++r) tab[codes[r].second] = r;
-    SK(S->bintab.alloc(tab.size()));
-    SK(cudaMemcpy(S->bintab.p, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    SK(S->scratch.alloc(S->nbins));
+    SK(S->bricks.build(S->dim, S->nx, S->ny, S->nz, S->cs));
+    SK(S->scratch.alloc(S->bricks.nbins));
     return GR_OK;
 }
 
@@ -498,7 +468,6 @@ int compact_pool(gr_server *S, Pool &P, int32_t k_end) {
     C.ret_by_id = 1;
     C.key = P.key.p;
     S->scratch.set(C);
-    C.bintab = S->bintab.p;
     C.n_act = P.counts.p;
     C.n_new = P.counts.p + 1;
     C.n_ret = P.counts.p + 2;
@@ -507,7 +476,7 @@ int compact_pool(gr_server *S, Pool &P, int32_t k_end) {
         C.inv_scale[d] = S->inv_scale[d];
     }
     C.nx = (int32_t)S->nx; C.ny = (int32_t)S->ny; C.nz = (int32_t)S->nz; C.dim = S->dim;
-    C.bx = S->bx; C.by = S->by; C.bz = S->bz; C.nbx = S->nbx; C.nby = S->nby; C.nbz = S->nbz; C.nbins = S->nbins;
+    S->bricks.set(C);
     C.k_end = k_end;
     launch_compaction(C, std::max<int64_t>(1, P.in_flight), S->cs);   // retired particles go to their result slots
     SK(cudaGetLastError());
