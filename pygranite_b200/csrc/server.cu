@@ -16,7 +16,8 @@
 //             than padded 3D nodes), unless it is there already;
 //     advance one persistent grid-stride launch per pool over the window's steps (a
 //             particle runs steps [start, end) of the clock);
-//     retire  compaction + Morton re-sort of each pool; particles that aborted or reached
+//     retire  compaction + Morton re-sort of each pool, where requests entered or end and every
+//             few windows; particles that aborted or reached
 //             their end step leave the pool, their final state written to their request's
 //             slots of the result arena;
 //     return  requests whose end step is in the window are complete: a kernel writes their
@@ -55,6 +56,7 @@ namespace {
 
 constexpr int kRing = 4;         // ring slots of a field that is not resident
 constexpr int kLag = 2;          // windows the host may enqueue ahead of the device
+constexpr int kPassWindows = 4;  // windows from one compaction to the next at most
 
 // First-fit allocator of index ranges (result arena, pinned staging).
 class RangeAlloc {
@@ -102,6 +104,7 @@ struct Pool {
     int cur = 0;
     int64_t cap = 0;                   // particle slots
     int64_t in_flight = 0;             // particles of active requests (upper bound of the live count)
+    int since = 0;                     // windows since the last compaction
     DevBuf<int32_t> counts;            // [0] live, [1] live after a pass, [2] retired
     DevBuf<int32_t> key;
     AdvanceFn fn = nullptr;
@@ -382,7 +385,7 @@ int allocate(gr_server *S, int64_t budget) {
         SK(P.counts.alloc(4));
         init_pool_kernel<<<1, 1, 0, S->cs>>>(P.counts.p);
         SK(cudaGetLastError());
-        P.threads = 256;
+        P.threads = 64;   // block_size_for, engine.cu
         const int st = S->s.storage;
         // positions only (no curvature, volumes, constants, uplift, length abort, compensation):
         // the lean variant, with 2D loop borders, sphere coordinates and 1/256 filter weights where on
@@ -610,6 +613,13 @@ int run_window(gr_server *S, const std::vector<Req *> &adm, const std::vector<Re
         K.s1 = (int32_t)k1;
         P.fn<<<(unsigned)P.grid, P.threads, 0, S->cs>>>(K);
         SK(cudaGetLastError());
+        // the pass hands finished particles to their result slots and sorts admitted ones; in between,
+        // aborted particles only take up room, so it may wait
+        bool due = ++P.since >= kPassWindows;
+        for (const Req *r : finishing) due = due || r->integrator == p;
+        for (const Req *r : adm) due = due || r->integrator == p;
+        if (!due) continue;
+        P.since = 0;
         rc = compact_pool(S, P, (int32_t)k1);
         if (rc) return rc;
     }
