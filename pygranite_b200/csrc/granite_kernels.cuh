@@ -67,7 +67,7 @@ struct StepEntry {
     int32_t slot_back, slot_front;   // ring slots of the window's snapshots
     int32_t rec, crec, irec;
     int32_t pad[3];
-};
+};   // read as 16-byte words (advance_particle)
 
 struct KParams {
     // geometry (TrajectoryIntegrator.tpp:521-574)
@@ -272,7 +272,7 @@ __device__ __forceinline__ Cell3 make_cell3(const KParams &P, float ax, float ay
 // the cell is loaded: the x lerps of every later sample are then one paired FMA each, with the
 // difference lerp2_ would form (same instruction, same rounding).
 struct SampleCache {
-    int32_t base;      // 3D pairs: padded node index of the first corner
+    int32_t base;      // pairs in 3D and of Euler steps: padded node index of the first corner
     float2 nxy;        // else: minus the first corner; NaN: no cell, or one not to be kept
     float nz;
     float2 c2d[2][4];  // 2D: (u, v) of the back and of the front snapshot at corners 0, 2; differences 1 - 0, 3 - 2
@@ -554,29 +554,32 @@ __device__ __forceinline__ void load_cell(const KParams &P, float2 axy, float az
 }
 
 // The cell and fractions of every sample, clamped, and its padded node index for a key.
+template <int DIM>
 __device__ __forceinline__ PCell clamped_cell(const KParams &P, float2 axy, float az, float2 &f, float &fz) {
     axy.x = fminf(fmaxf(axy.x, -1.0f), P.fn[0]);
     axy.y = fminf(fmaxf(axy.y, -1.0f), P.fn[1]);
-    az = fminf(fmaxf(az, -1.0f), P.fn[2]);
-    const PCell c = make_pcell<3>(axy, az);
+    if (DIM == 3) az = fminf(fmaxf(az, -1.0f), P.fn[2]);
+    const PCell c = make_pcell<DIM>(axy, az);
     f = add2(axy, c.nxy);
-    fz = az + c.nz;
+    if (DIM == 3) fz = az + c.nz;
     return c;
 }
 
 // Wind at world position p, time weight t: interpolate() of TrajectoryIntegrator.icc:42-110.  The
 // cell's corners come from the sample cache, reloaded when the cell changes (wb: the window pair; or
 // wb, wf: the ring slots), interpolated in space, then in time.
-// 2D and ring slots: a sample lies in the cached cell when its coordinates minus the cell's first
+// 2D RK4 and ring slots: a sample lies in the cached cell when its coordinates minus the cell's first
 // corner are in [0, 1), one unsigned comparison of the bits each; those differences are then its
 // fractions (a - floor(a) bit for bit: the same subtraction), and nothing of the cell's search is
 // left on the way of such a sample.  (A fraction that rounds to 1 loads the same cell again.)
-// 3D pairs: some lane of nearly every warp loads a cell at nearly every sample, so the search is on
-// the warp's way in any case and goes before the test, where it costs no latency.  Measured, search
+// Other pairs: some lane of nearly every warp loads a cell at nearly every sample (of an Euler step the
+// only one), so the search is on the warp's way in any case and goes before the test, where it
+// costs no latency.  Measured, search
 // first against differences first: 1e6 particles x 300 steps 7.03 / 7.16 ms of step launches, 300,000 x 200
-// 2.30 / 2.33, 2D sphere 150,000 x 200 0.75 / 0.72, bf16 ring slots 777,777 x 100 2.66 / 2.61 ms.
+// 2.30 / 2.33, 10,000 x 1024 Euler steps in 2D 0.46 / 0.47, 10,000 x 1024 RK4 steps in 2D 0.80 / 0.75, 2D
+// sphere 150,000 x 200 0.75 / 0.72, bf16 ring slots 777,777 x 100 2.66 / 2.61 ms.
 // FT: the step kernel's feature set; lean variants run with filter_weights off (kernel_features).
-template <int DIM, typename W, int FT>
+template <int DIM, bool RK4, typename W, int FT>
 __device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf,
                                       SampleCache &cc) {
     constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
@@ -584,9 +587,9 @@ __device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, co
     const float az = DIM == 3 ? grid_z(P, p.z) : 0.f;
     float2 fr;
     float fz = 0.f;
-    if constexpr (IsPair<W>::value && DIM == 3) {
-        const PCell c = clamped_cell(P, axy, az, fr, fz);
-        const int32_t base = padded_index<3>(P, c);
+    if constexpr (IsPair<W>::value && (DIM == 3 || !RK4)) {
+        const PCell c = clamped_cell<DIM>(P, axy, az, fr, fz);
+        const int32_t base = padded_index<DIM>(P, c);
         if (base != cc.base) {
             cc.base = base;
             fill<DIM, W>(P, wb, wf, c, cc);
@@ -938,17 +941,20 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
     cc.reset();
     int slot = -1;   // ring layouts: back slot of the cached cell
     for (int s = P.s0; s < P.s1; ++s) {
-        // the step's time weights and flags; the rest of its entry where it is used, so that no register
-        // holds it over the step
+        // the step's time weights and flags; with registers to spare also its ring slots and record
+        // indices (a load at the record of every step of 10,000 particles in 2D: 0.56 ms instead of 0.48),
+        // in the 3D pair variants those where they are used, so that no register holds them over the step
+        constexpr bool whole = DIM == 2 || !IsPair<W>::value;
         const StepEntry *const entry = P.sched + s;
         const int4 head = __ldg(reinterpret_cast<const int4 *>(entry));
         struct {
             float t0, t1, t2;
             int flags;
         } const E{__int_as_float(head.x), __int_as_float(head.y), __int_as_float(head.z), head.w};
-        int2 slots = make_int2(0, 0);
-        if (!IsPair<W>::value && P.wind_dynamic) slots = __ldg(reinterpret_cast<const int2 *>(&entry->slot_back));
-        const int sb = slots.x, sf = slots.y;
+        int4 tail = make_int4(0, 0, 0, 0);   // slot_back, slot_front, rec, crec
+        if (whole) tail = __ldg(reinterpret_cast<const int4 *>(entry) + 1);
+        const int sb = !IsPair<W>::value && P.wind_dynamic ? tail.x : 0;
+        const int sf = !IsPair<W>::value && P.wind_dynamic ? tail.y : 0;
         const void *wb = IsPair<W>::value ? P.pair : reinterpret_cast<const char *>(P.wind) + (int64_t)sb * P.wind_stride;
         const void *wf = reinterpret_cast<const char *>(P.wind) + (int64_t)sf * P.wind_stride;
         // the cached cell belongs to the window's two snapshots
@@ -975,7 +981,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
 #pragma unroll kUnroll
                 for (int stage = 0; stage < 4; ++stage) {
                     const float tw = stage == 0 ? t0 : (stage == 3 ? E.t2 : E.t1);
-                    const V3 kc = wind_at<DIM, W, FT>(P, a, tw, wb, wf, cc);
+                    const V3 kc = wind_at<DIM, RK4, W, FT>(P, a, tw, wb, wf, cc);
                     const V3 k = sph ? sphere_(P, a.xy.y, kc) : kc;
                     if (stage == 0) {
                         acc = k;
@@ -992,7 +998,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
                 v = V3{mul2(acc.xy, P.sixth2), DIM == 3 ? acc.z * P.sixth : 0.f};
                 vc = sph ? V3{mul2(accc.xy, P.sixth2), 0.f} : v;
             } else {
-                vc = wind_at<DIM, W, FT>(P, p, t0, wb, wf, cc);
+                vc = wind_at<DIM, RK4, W, FT>(P, p, t0, wb, wf, cc);
                 v = sph ? sphere_(P, p.xy.y, vc) : vc;
             }
 
@@ -1003,7 +1009,8 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
             V3 dp{mul2(v.xy, P.h2), DIM == 3 ? v.z * P.h : 0.f};
             if (reverse) { dp.xy = make_float2(-dp.xy.x, -dp.xy.y); dp.z = -dp.z; }
             if (DIM == 3 && uplift_mode != 0) {
-                const int lb = uplift_mode == 2 ? __ldg(&entry->slot_back) : 0, lf = uplift_mode == 2 ? __ldg(&entry->slot_front) : 0;
+                const int lb = uplift_mode != 2 ? 0 : whole ? tail.x : __ldg(&entry->slot_back);
+                const int lf = uplift_mode != 2 ? 0 : whole ? tail.y : __ldg(&entry->slot_front);
                 const float *LB = P.lift + ((int64_t)lb * P.n_total + pid) * 3;
                 const float *LF = P.lift + ((int64_t)lf * P.n_total + pid) * 3;
                 if (uplift_mode == 1) {
@@ -1157,10 +1164,10 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
         }
 
         if (valid && (E.flags & SF_SAVE)) {
-            float *hp = P.hpos + ((int64_t)__ldg(&entry->rec) * P.n_total + pid) * DIM;
+            float *hp = P.hpos + ((int64_t)(whole ? tail.z : __ldg(&entry->rec)) * P.n_total + pid) * DIM;
             hp[0] = p.xy.x; hp[1] = p.xy.y;
             if (DIM == 3) hp[2] = p.z;
-            if (curvature_mode == 3 && (E.flags & SF_CURV_REC)) P.hcurv[(int64_t)__ldg(&entry->crec) * P.n_total + pid] = cv;
+            if (curvature_mode == 3 && (E.flags & SF_CURV_REC)) P.hcurv[(int64_t)(whole ? tail.w : __ldg(&entry->crec)) * P.n_total + pid] = cv;
             if constexpr ((FT & FT_DEFER) != 0) {
                 // the record's inputs: the position and the last moved step's (if any since the
                 // last evaluation)
@@ -1181,7 +1188,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
                     const float2 axy = grid_xy(P, p.xy);
                     const float az = grid_z(P, p.z);
                     if constexpr (IsPair<W>::value) {
-                        const PCell c = clamped_cell(P, axy, az, f, fz);
+                        const PCell c = clamped_cell<3>(P, axy, az, f, fz);
                         cc.base = padded_index<3>(P, c);
                         fill<3, W>(P, wb, wf, c, cc);
                     } else {
