@@ -71,7 +71,9 @@ typedef struct gr_settings {
     int32_t ring_slots;            /* device ring depth (>= 3); 0 = 3 */
     int32_t steps_per_launch;      /* steps fused into one launch; 0 = one snapshot window */
     int32_t sort_interval;         /* launches between Morton re-sorts / compactions; 0 = off; negative
-                                    * (the default): every 8 launches from 65,536 particles, else off */
+                                    * (the default): automatic from 65,536 particles, else off: the seeds
+                                    * before the first step, then every 8 windows (16 below 400,000
+                                    * particles without lifetimes) */
     int32_t block_size;            /* threads per block; 0 = autotuned default; capped at the step
                                       kernel's launch bound (128 for the float32 3D window-pair
                                       kernel, 256 for the others) */
