@@ -48,6 +48,7 @@
 #include "compact.cuh"
 #include "engine_graph.h"
 #include "host_util.h"
+#include "pack_kernels.cuh"
 #include "schedule.h"
 
 using namespace granite_b200;
@@ -140,6 +141,7 @@ struct gr_server {
     Schedule sched;
     DevBuf<StepEntry> d_sched;
     int64_t elem = 4;                  // bytes per stored value
+    bool wide = false;                 // wide_grid (advance.h): node-major slots, read without pairs
     bool resident = false;             // every snapshot has a slot of its own
     int64_t K = kRing;                 // slots
     std::vector<char> have;            // snapshots set
@@ -267,6 +269,16 @@ __global__ void planar_pack_kernel(const float *__restrict__ u, const float *__r
     }
 }
 
+// A snapshot's planes -> its slot.
+template <typename T>
+void pack_snapshot(gr_server *S, const float *const (&src)[3], void *out) {
+    const int threads = 256, blocks = grid_for(S->nodes, threads);
+    if (S->wide)
+        pack_wind_kernel<T><<<blocks, threads, 0, S->cs>>>(src[0], src[1], src[2], out, S->nodes, S->dim);
+    else
+        planar_pack_kernel<T><<<blocks, threads, 0, S->cs>>>(src[0], src[1], src[2], static_cast<T *>(out), S->nodes, S->dim);
+}
+
 // Two planar slots -> the window-pair layout the step kernel reads (granite_kernels.cuh,
 // Store<Pair<...>>): per node (u, v) of the back and of the front snapshot, then w: {u_b, v_b, u_f,
 // v_f, w_b, w_f, 0, 0} (3D) or {u_b, v_b, u_f, v_f} (2D), vector stores.  3D pairs carry the zero
@@ -333,12 +345,16 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx, int64_t field_budget
         S->inv_scale[d] = 1.0f / S->scale[d];
     }
     S->elem = s.storage == GR_STORE_F32 ? 4 : 2;
-    S->snap_bytes = S->nodes * S->dim * S->elem;                  // planar, unpadded
+    // planar, unpadded; node-major as the step kernel reads ring slots where pairs do not apply: their cell
+    // search (make_pcell) is exact below 2^22 only
+    S->wide = wide_grid(S->nx, S->ny, S->nz);
+    S->snap_bytes = S->nodes * (!S->wide ? S->dim : S->dim == 3 ? 4 : 2) * S->elem;
     S->slot_stride = ((S->snap_bytes + 255) / 256) * 256;
     // window pairs carry a border (padded_pair_nodes); the kernel indexes them with int32
     if (padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) > (int64_t(1) << 31) - 1)
         return SUSER("Invalid dataset was provided. Grid too large.");
-    const int64_t pair_bytes = ((padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) * (S->dim == 3 ? 8 : 4) * S->elem + 255) / 256) * 256;
+    const int64_t pair_bytes =
+        S->wide ? 0 : ((padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) * (S->dim == 3 ? 8 : 4) * S->elem + 255) / 256) * 256;
     // the whole field on the device where it fits the budget, with all its pairs if they fit too
     const int64_t field = S->slot_stride * S->n_snap;
     const char *env = std::getenv("GR_SERVE_RESIDENT");   // 0: host memory whatever fits
@@ -391,9 +407,9 @@ int allocate(gr_server *S, int64_t budget) {
         // the lean variant, with 2D loop borders, sphere coordinates and 1/256 filter weights where on
         const bool lean = !(S->dim == 2 && (S->s.border_mode != 0 || S->s.sphere_radius > 0.f)) &&
                           !S->s.filter_weights;
-        const int ft = lean ? FT_LEAN : FT_LEAN | FT_BORDER;
-        P.fn = st == GR_STORE_BF16 ? advance_bf16(S->dim, p == 1, true, ft)
-             : st == GR_STORE_F16 ? advance_f16(S->dim, p == 1, true, ft) : advance_f32(S->dim, p == 1, true, ft);
+        const int ft = lean && !S->wide ? FT_LEAN : FT_LEAN | FT_BORDER;
+        P.fn = st == GR_STORE_BF16 ? advance_bf16(S->dim, p == 1, !S->wide, ft)
+             : st == GR_STORE_F16 ? advance_f16(S->dim, p == 1, !S->wide, ft) : advance_f32(S->dim, p == 1, !S->wide, ft);
         cudaFuncAttributes fa{};
         SK(cudaFuncGetAttributes(&fa, reinterpret_cast<const void *>(P.fn)));
         P.threads = std::min(P.threads, fa.maxThreadsPerBlock);   // the kernel's launch bounds
@@ -426,10 +442,15 @@ KParams pool_params(gr_server *S, Pool &P) {
         K.scale[d] = S->scale[d];
     }
     K.nx = (int32_t)S->nx; K.ny = (int32_t)S->ny; K.nz = (int32_t)S->nz; K.dim = S->dim;
-    clamp_cells(K, true);
-    K.wind = S->ring.p;
-    K.wind_stride = S->slot_stride;
-    K.pair = pair_at(S, S->w);
+    K.wide = S->wide;
+    clamp_cells(K, !S->wide);
+    if (S->wide) {   // the window's two slots: the schedule's slots 0 and 1
+        const int64_t v = S->sweep * S->n_snap + S->w, back = v % S->K, front = (v + 1) % S->K;
+        K.wind = S->ring.p + back * S->slot_stride;
+        K.wind_stride = (front - back) * S->slot_stride;
+    } else {
+        K.pair = pair_at(S, S->w);
+    }
     K.pnx = (int32_t)(S->nx + 3); K.pnxy = (int32_t)((S->nx + 3) * (S->ny + 3));
     Pool::Arrays &A = P.st[P.cur];
     K.px = A.px.p; K.py = A.py.p; K.pz = A.pz.p;
@@ -503,7 +524,7 @@ int ensure_snapshot(gr_server *S, int64_t v) {
 }
 
 int pack_pair(gr_server *S, int64_t v) {
-    if (S->pair_stride > 0 && S->pair_built[S->w]) return GR_OK;
+    if (S->wide || (S->pair_stride > 0 && S->pair_built[S->w])) return GR_OK;
     S->pair_built[S->w] = 1;
     char *const out = pair_at(S, S->w);
     const char *back = S->ring.p + (v % S->K) * S->slot_stride;
@@ -892,6 +913,7 @@ int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t n
         StepEntry E{};
         E.t0 = h.t0; E.t1 = h.t1; E.t2 = h.t2;
         E.flags = h.time_pos ? SF_TIME_POS : 0;
+        E.slot_front = 1;   // of a wide grid's two slots (pool_params)
         hs[k] = E;
     }
     SK(S->d_sched.alloc(hs.size()));
@@ -931,18 +953,10 @@ int gr_server_set_snapshot(gr_server *S, int64_t snapshot, const float *const *c
     if (ncomp == 2) src[2] = src[1];
     // a resident snapshot is packed where it stays; else slot 0 is packing scratch until the start
     char *scratch = S->ring.p + (S->resident ? snapshot * S->slot_stride : 0);
-    const int threads = 256, blocks = grid_for(S->nodes, threads);
     switch (S->s.storage) {
-        case GR_STORE_BF16:
-            planar_pack_kernel<__nv_bfloat16><<<blocks, threads, 0, S->cs>>>(src[0], src[1], src[2], (__nv_bfloat16 *)scratch,
-                                                                             S->nodes, S->dim);
-            break;
-        case GR_STORE_F16:
-            planar_pack_kernel<__half><<<blocks, threads, 0, S->cs>>>(src[0], src[1], src[2], (__half *)scratch, S->nodes, S->dim);
-            break;
-        default:
-            planar_pack_kernel<float><<<blocks, threads, 0, S->cs>>>(src[0], src[1], src[2], (float *)scratch, S->nodes, S->dim);
-            break;
+        case GR_STORE_BF16: pack_snapshot<__nv_bfloat16>(S, src, scratch); break;
+        case GR_STORE_F16: pack_snapshot<__half>(S, src, scratch); break;
+        default: pack_snapshot<float>(S, src, scratch); break;
     }
     SK(cudaGetLastError());
     if (!S->resident) {
