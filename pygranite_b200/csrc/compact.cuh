@@ -252,7 +252,9 @@ static __global__ void morton_rank_kernel(int32_t *rank, int32_t nbx, int32_t nb
 struct Bricks {
     int bx = 4, by = 4, bz = 2, nbx = 0, nby = 0, nbz = 0, nbins = 0;
     DevBuf<int32_t> rank;
+    // nbins (0: not built) is set once the ranks are on their way: after an error the next call builds again.
     cudaError_t build(int dim, int64_t nx, int64_t ny, int64_t nz, cudaStream_t stream) {
+        nbins = 0;
         bx = 4; by = 4; bz = dim == 3 ? 2 : 1;
         for (;;) {
             nbx = (int)((nx + bx - 1) / bx);
@@ -261,11 +263,13 @@ struct Bricks {
             if ((int64_t)nbx * nby * nbz <= MAX_BINS && nbx <= 1024 && nby <= 1024 && nbz <= 1024) break;
             bx *= 2; by *= 2; if (dim == 3) bz *= 2;
         }
-        nbins = nbx * nby * nbz;
-        const cudaError_t e = rank.alloc((size_t)nbins);
+        const int n = nbx * nby * nbz;
+        cudaError_t e = rank.alloc((size_t)n);
         if (e != cudaSuccess) return e;
-        morton_rank_kernel<<<(nbins + 255) / 256, 256, 0, stream>>>(rank.p, nbx, nby, nbz);
-        return cudaGetLastError();
+        morton_rank_kernel<<<(n + 255) / 256, 256, 0, stream>>>(rank.p, nbx, nby, nbz);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) nbins = n;
+        return e;
     }
     void set(CompactParams &C) const {
         C.bx = bx; C.by = by; C.bz = bz;
@@ -278,8 +282,9 @@ struct Bricks {
 // Scratch of the passes: zeroed when it is allocated, left zero by every pass.
 struct CompactScratch {
     DevBuf<int32_t> hist, cursor, chunk, ticket;
+    bool ready = false;   // allocated and zeroed
     cudaError_t alloc(int nbins) {
-        if (ticket.p) return cudaSuccess;
+        if (ready) return cudaSuccess;
         const size_t chunks = ((size_t)nbins + SCAN_CHUNK) / SCAN_CHUNK, nb = chunks * SCAN_CHUNK;
         cudaError_t e = hist.alloc(nb);
         if (e == cudaSuccess) e = cursor.alloc(nb);
@@ -288,6 +293,7 @@ struct CompactScratch {
         if (e == cudaSuccess) e = ticket.alloc(1);
         if (e == cudaSuccess) e = cudaMemset(ticket.p, 0, sizeof(int32_t));
         if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // the runs' streams do not wait for it
+        ready = e == cudaSuccess;
         return e;
     }
     void set(CompactParams &C) const {
