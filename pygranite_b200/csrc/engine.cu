@@ -1158,6 +1158,8 @@ int run_prepare(gr_engine *e, RunPlan &R, bool graph) {
 
     rc = alloc_state(e);
     if (rc) return rc;
+    // a failed run returns with its passes still queued: their live counts land before this run sets its own
+    if (e->live_ready) CK(cudaEventSynchronize(e->live_ready));
     if (s.minimum_alive > 0) {
         rc = alloc_set(e, e->ck, false);
         if (rc) return rc;
