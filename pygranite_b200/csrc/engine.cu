@@ -543,9 +543,6 @@ extern "C" {
 constexpr int kAutoSortInterval = 8, kAutoSortSmall = 16;
 constexpr int64_t kAutoSortMin = 65536, kAutoSortLarge = 400000;
 
-// Launches and passes placed by the engine (no setting says where).
-bool auto_launches(const gr_engine *e) { return e->s.sort_interval < 0 && e->s.steps_per_launch <= 0; }
-
 int auto_sort_interval(const gr_engine *e) {
     return e->n >= kAutoSortLarge || e->has_life ? kAutoSortInterval : kAutoSortSmall;
 }
@@ -1186,11 +1183,8 @@ int run_prepare(gr_engine *e, RunPlan &R, bool graph) {
     R.small_set = small_set(e, R);
     e->use_pair = e->wind_dynamic && s.layout == 0 && !wide_grid(e->nx, e->ny, e->nz) && !R.small_set;
     R.spl = s.steps_per_launch > 0 ? s.steps_per_launch : (int64_t)1 << 40;
-    if (e->compacting && s.steps_per_launch <= 0 && R.nwin > 0) {
-        // compacting runs launch window by window, or from pass to pass
-        const int64_t windows = auto_launches(e) ? std::min<int64_t>(R.nwin, auto_sort_interval(e)) : 1;
-        R.spl = std::max<int64_t>(1, R.sched.window_begin[windows]);
-    }
+    if (e->compacting && s.sort_interval > 0 && s.steps_per_launch <= 0 && R.nwin > 0)
+        R.spl = std::max<int64_t>(1, R.sched.window_begin[1]);   // an interval of launches: window by window
     {
         const int rc = settle_pairs(e);
         if (rc) return rc;
@@ -1451,7 +1445,8 @@ struct RunCtx {
     int64_t grid = 0;          // graph runs: persistent grid of the step kernel
     size_t ev_used = 2;        // events 0 and 1 bracket the run
     int64_t executed = 0;      // steps enqueued
-    int64_t since_sort = 0;    // launches since the last compaction
+    int64_t since_sort = 0;    // launches since the last compaction (an interval from the settings)
+    int64_t sorted = 0;        // window of the first step after it (automatic passes)
     int64_t alive_known = -1;  // particles alive before the next step (-1: all of them)
     unsigned long long ps_known = 0;   // particle-steps counted before the next launch
     bool defer = false;        // volume / expression values by deferred_extras_kernel after each
@@ -1571,6 +1566,7 @@ int launch_deferred_extras(RunCtx &r, int64_t save_step, int64_t k_end, bool all
 int sort_now(RunCtx &r, int64_t k_end) {
     gr_engine *e = r.e;
     r.since_sort = 0;
+    r.sorted = r.R->sched.steps[k_end].window;
     const int q = compact_pass(e, r.R->rec_before[k_end], (int32_t)k_end, r.R->graph);
     if (q) return q;
     const int32_t gs = r.P.grid_stride;
@@ -1594,14 +1590,22 @@ int sort_seeds(RunCtx &r) {
     return sort_now(r, 0);
 }
 
-// After a launch of steps [k, k_end): maybe retire / re-sort (compact.cuh).
-int after_launch(RunCtx &r, int64_t k, int64_t k_end) {
+// Step before which the next automatic pass comes: no launch crosses it.  Windows, not launches, set it:
+// a window may take several launches (deferred values end one at every record) and a launch several
+// windows (ring slots).
+int64_t next_pass(const RunCtx &r) {
+    const gr_engine *e = r.e;
+    const RunPlan &R = *r.R;
+    if (!e->compacting || e->s.sort_interval > 0) return R.nsteps;
+    return R.sched.window_begin[std::min<int64_t>(R.nwin, r.sorted + auto_sort_interval(e))];
+}
+
+// After a launch that ended before step k_end: maybe retire / re-sort (compact.cuh).
+int after_launch(RunCtx &r, int64_t k_end) {
     gr_engine *e = r.e;
     const RunPlan &R = *r.R;
     if (!e->compacting || k_end >= R.nsteps) return 0;
-    // automatic passes count windows (a launch may span several), the settings' interval launches
-    r.since_sort += auto_launches(e) ? R.sched.steps[k_end - 1].window - R.sched.steps[k].window + 1 : 1;
-    if (r.since_sort < (e->s.sort_interval > 0 ? e->s.sort_interval : auto_sort_interval(e))) return 0;
+    if (e->s.sort_interval > 0 ? ++r.since_sort < e->s.sort_interval : k_end < next_pass(r)) return 0;
     if (r.defer) {   // retiring particles take their final values along
         const int q = launch_deferred_extras(r, -1, k_end, false);
         if (q) return q;
@@ -1622,7 +1626,7 @@ int launch_range(RunCtx &r, int64_t b, int64_t t) {
         for (int64_t k = b; k < t;) {
             const long long alive = r.alive_known < 0 ? e->n : r.alive_known;
             if (alive < minimum) return 1;
-            int64_t k1 = std::min({t, k + R.spl, k + kAliveSteps});
+            int64_t k1 = std::min({t, k + R.spl, k + kAliveSteps, next_pass(r)});
             const int64_t w = R.sched.steps[k].window;
             if (e->use_pair) k1 = std::min(k1, R.sched.window_begin[w + 1]);
             const int64_t L = k1 - k;
@@ -1664,14 +1668,14 @@ int launch_range(RunCtx &r, int64_t b, int64_t t) {
             r.alive_known = alive_after(L - 1);
             r.ps_known = e->h_counters[0];
             r.executed += L;
-            q = after_launch(r, k, k1);
+            q = after_launch(r, k1);
             if (q) return q;
             k = k1;
         }
         return 0;
     }
     for (int64_t k = b; k < t;) {
-        int64_t k1 = std::min(t, k + R.spl);
+        int64_t k1 = std::min({t, k + R.spl, next_pass(r)});
         const int64_t w = R.sched.steps[k].window;
         if (e->use_pair) k1 = std::min(k1, R.sched.window_begin[w + 1]);   // one window per launch
         if (r.defer && R.save_next[k] < R.nsteps)
@@ -1682,7 +1686,7 @@ int launch_range(RunCtx &r, int64_t b, int64_t t) {
             q = launch_deferred_extras(r, R.save_next[k], k1, false);
             if (q) return q;
         }
-        q = after_launch(r, k, k1);
+        q = after_launch(r, k1);
         if (q) return q;
         k = k1;
     }
