@@ -534,17 +534,22 @@ int ensure_particles(gr_engine *e) {
 
 extern "C" {
 
-// Automatic compaction (sort_interval < 0), from 65,536 particles: every 8 launches from 400,000
+// Automatic compaction (sort_interval < 0), from 65,536 particles: every 8 windows from 400,000
 // particles or with lifetimes (particles retire all the time), every 16 below, where a pass costs
-// more launches' worth of what it saves (1e6 x 300 steps: 8.38 ms every 8, 8.59 every 4, 8.76 sorted
-// once; 300,000 x 200 steps: 2.84, 2.91, 2.82; a batch of uneven lifetimes: 3.45, 3.53, 4.25 ms).
+// more windows' worth of what it saves (1e6 x 300 steps: 8.38 ms every 8, 8.59 every 4, 8.76 sorted
+// once; 150,000 x 250 steps: 1.81 ms every 8, 1.71 every 16; a batch of uneven lifetimes: 3.45, 3.53,
+// 4.25 ms).  Runs that end at a path length retire their particles within a few windows of one another:
+// every 8 from 80,000 particles (every option, 150 steps, most particles done after 60; ms every 8 / 16:
+// 120,000 on 24 x 24 x 16 nodes 1.39 / 1.62, on 192 x 192 x 64 1.95 / 1.99; 80,000 on 40 x 40 x 20
+// 1.19 / 1.22, 70,000 on 192 x 192 x 64 1.13 / 1.04).
 // Below 65,536 particles one wave of warps holds the whole set and a launch's time is that of
 // its slowest warp: passes cost more than they save (70,000 x 200 steps: 1.02 ms without, 1.20 with).
 constexpr int kAutoSortInterval = 8, kAutoSortSmall = 16;
-constexpr int64_t kAutoSortMin = 65536, kAutoSortLarge = 400000;
+constexpr int64_t kAutoSortMin = 65536, kAutoSortLarge = 400000, kAutoSortLengths = 80000;
 
 int auto_sort_interval(const gr_engine *e) {
-    return e->n >= kAutoSortLarge || e->has_life ? kAutoSortInterval : kAutoSortSmall;
+    const bool often = e->n >= kAutoSortLarge || e->has_life || (e->s.abort_mode != 0 && e->n >= kAutoSortLengths);
+    return often ? kAutoSortInterval : kAutoSortSmall;
 }
 
 void gr_settings_default(gr_settings *s) {
@@ -1582,11 +1587,16 @@ int sort_now(RunCtx &r, int64_t k_end) {
 // 1e6-particle plain configuration took 340 us each against 225 us).  What a pass saves grows with
 // the samples that follow and is four times as much in 3D; it breaks even at about 40 RK4 steps of
 // 100,000 particles in 3D, 100 in 2D, against the line's 50 and 200.
-constexpr int64_t kSortWork = 20000000;
+// An uplift is read by particle at every step, in order as long as the slots are: on a grid so small that
+// the gathers hit the caches anyway the sort then loses (every option, 120,000 x 150 steps, ms sorted /
+// not: 24 x 24 x 16 nodes 1.39 / 1.28, 40 x 40 x 20 1.45 / 1.40 but 80,000 there 1.19 / 1.24, 80 x 80 x 40
+// from 200,000 particles 2.04 / 2.12).
+constexpr int64_t kSortWork = 20000000, kSortNodes = 16384;
 int sort_seeds(RunCtx &r) {
     const gr_engine *e = r.e;
     const int64_t weight = (e->dim == 3 ? 4 : 1) * (e->s.integrator == 1 ? 4 : 1);
     if (!e->compacting || e->n * r.R->nsteps < 4 * kSortWork / weight) return 0;
+    if (e->s.uplift_mode != 0 && e->nodes < kSortNodes) return 0;
     return sort_now(r, 0);
 }
 
