@@ -1027,6 +1027,7 @@ std::vector<int32_t> rec_of_crec_table(const gr_engine *e, const RunPlan &R, int
 
 int ensure_pair(gr_engine *e, int64_t w);
 int settle_pairs(gr_engine *e);
+KParams make_params(gr_engine *e);
 
 int pair_elem(const gr_engine *e) {
     return e->s.storage == GR_STORE_F32 ? (e->dim == 3 ? 16 : 8) : (e->dim == 3 ? 8 : 4);
@@ -1047,13 +1048,20 @@ size_t pair_bytes(const gr_engine *e) {
 // particles and step (25 us with volumes or expressions, whose evaluation costs the deferred kernel
 // its lower register count).  Measured, ring against pair, ms of device time a run:
 // 192 x 192 x 64 nodes, 200 steps, 10 a window: positions of 70,000 particles 0.87 / 1.10, 150,000
-// 1.44 / 1.46, 300,000 2.18 / 2.01, with a volume, an expression and records 10,000 0.91 / 1.37, 70,000
-// 1.30 / 1.59, 150,000 2.29 / 2.03; 512 x 512 x 96 bf16, 777,777 x 100 steps 2.84 / 3.73; 24 x 24 x 16,
+// 1.44 / 1.46, 300,000 2.18 / 2.01; 512 x 512 x 96 bf16, 777,777 x 100 steps 2.84 / 3.73; 24 x 24 x 16,
 // 100 steps, 50,000 0.26 / 0.28, 150,000 0.61 / 0.52; 2D 1024 x 512 nodes, 200 steps, 150,000 0.58 /
 // 0.63, 400,000 1.16 / 1.08; 256 x 128, 10,000 x 1024 Euler steps, 128 a window, 0.58 / 0.42.  Where the
 // settings place the launches, only the pack is saved; in a graph a launch costs little, all the less
 // beside another engine's (the batch of 48 sets: 3.40 ms a replay with pairs, 3.63 without).
-bool small_set(const gr_engine *e, const RunPlan &R) {
+// RK4 in 3D with volumes or expressions that pairs would defer: the ring variant that evaluates them runs
+// at 128 registers and spills, so a record costs it 3 us and 11.5 ns a warp, a step 0.5 us and 0.34 ns a
+// warp (their slope follows the warps, of 16 lanes or 32 alike), against 13.5 us for a window's launch, 6.5 us
+// for a record's kernel and 0.8 of the pack.  Measured where more than one record a window already pays
+// for the launches: none was slower on the ring slots.  150 steps, a record a window, ring / pair: 24 x 24
+// x 16 nodes 6,000 0.43 / 0.48, 20,000 0.60 / 0.53, 25,000 0.51 / 0.52, 40,000 0.65 / 0.56; 80 x 80 x 40 25,000
+// 0.59 / 0.57, 40,000 0.74 / 0.62; 130 x 130 x 48 32,000 0.67 / 0.70, 60,000 0.89 / 0.79; 192 x 192 x 64 72,000
+// 1.05 / 1.17, 80,000 1.39 / 1.19.
+bool small_set(gr_engine *e, const RunPlan &R) {
     if (R.nsteps == 0 || !e->wind_dynamic) return false;
     const gr_settings &s = e->s;
     const bool extras = (s.volume_mode != 0 && e->nvol > 0) || e->nexpr > 0;
@@ -1061,7 +1069,15 @@ bool small_set(const gr_engine *e, const RunPlan &R) {
     const double pack = (double)e->nodes * 4 * pair_elem(e) / 5e6;   // us at 5 TB/s
     const double steps = (double)R.nsteps / (double)R.nwin;          // a window
     const double chain = e->dim == 3 ? 0.5 : 0.18, gathers = extras ? 25.0 : e->dim == 3 ? 8.6 : 3.0;
-    return steps * (chain + gathers * 1e-6 * (double)e->n) < launch + 0.5 * pack;
+    if (steps * (chain + gathers * 1e-6 * (double)e->n) >= launch + 0.5 * pack) return false;
+    const double records = (double)(R.rec_before[R.nsteps] - 1) / (double)R.nwin;   // a window
+    if (e->dim == 3 && s.integrator == 1 && records <= 1.0 && !R.graph &&
+        (kernel_features(make_params(e), true) & FT_DEFER) != 0) {
+        const int lanes = block_of_few(e->n);
+        const double warps = (double)e->n / (lanes > 0 ? lanes : 32);
+        return steps * (0.5 + 0.34e-3 * warps) + records * (3.0 + 11.5e-3 * warps) <= 13.5 + 6.5 * records + 0.8 * pack;
+    }
+    return true;
 }
 
 // Validation, schedule, device schedule and programs, state and history buffers.
