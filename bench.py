@@ -445,7 +445,7 @@ def run_batch(args, world, rank, local, pg_dist, storages=None):
                 r = e.tune(trial_steps=args.tune_steps)
                 tuned[f"{dim}d"] = {"layout": ["window-pair", "ring"][r.layout], "block_size": r.block_size,
                                     "sort_interval": r.sort_interval, "grid_waves": r.grid_waves,
-                                    "trials": r.trials, "trial_rate": r.particle_steps_per_s}
+                                    "kept_automatic": bool(r.kept), "trials": r.trials, "trial_rate": r.particle_steps_per_s}
         batch = capi.Batch([eb[d] for d in sorted(eb)])
         for _ in range(max(1, args.warmup)):
             batch.run()

@@ -320,14 +320,16 @@ void gr_batch_destroy(gr_batch *batch);
 int gr_batch_run(gr_batch *batch);
 int gr_batch_stats_get(const gr_batch *batch, gr_batch_stats *out);
 
-/* Autotuner: picks the wind layout, block size, sort interval and persistent-grid waves of an
- * engine by timing short runs (`trial_steps` steps each, resident snapshots, graph launch
- * shapes) and stores the fastest in its settings.  No counterpart in the reference.  Trials
- * overwrite the engine's results. */
+/* Autotuner: times short runs (`trial_steps` steps each, resident snapshots, graph launch shapes) of the
+ * engine's settings as they are and of explicit wind layouts, block sizes, sort intervals and
+ * persistent-grid waves, and stores the fastest explicit values in its settings if they beat the
+ * settings as they were (the automatic choices of an untuned engine) by 1%, in two trials; else it
+ * keeps those.  No counterpart in the reference.  Trials overwrite the engine's results. */
 typedef struct gr_tune_result {
-    int32_t layout, block_size, sort_interval, grid_waves;
-    double particle_steps_per_s;   /* of the chosen configuration */
+    int32_t layout, block_size, sort_interval, grid_waves;   /* fastest explicit values tried */
+    double particle_steps_per_s;   /* of the settings now stored */
     int32_t trials;
+    int32_t kept;                  /* 1: the settings are as they were */
 } gr_tune_result;
 int gr_tune(gr_engine *engine, int32_t trial_steps, gr_tune_result *out);
 

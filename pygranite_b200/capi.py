@@ -80,7 +80,8 @@ class BatchStats(ctypes.Structure):
 
 class TuneResult(ctypes.Structure):
     _fields_ = [("layout", ctypes.c_int32), ("block_size", ctypes.c_int32), ("sort_interval", ctypes.c_int32),
-                ("grid_waves", ctypes.c_int32), ("particle_steps_per_s", ctypes.c_double), ("trials", ctypes.c_int32)]
+                ("grid_waves", ctypes.c_int32), ("particle_steps_per_s", ctypes.c_double), ("trials", ctypes.c_int32),
+                ("kept", ctypes.c_int32)]
 
 
 class RequestInfo(ctypes.Structure):
@@ -415,6 +416,7 @@ class Engine:
         _check(lib().gr_update_settings(self.h, ctypes.byref(s)))
 
     def tune(self, trial_steps=40) -> TuneResult:
+        """gr_tune: the fastest explicit launch settings, stored unless the engine's own (`kept`) are as fast."""
         r = TuneResult()
         _check(lib().gr_tune(self.h, trial_steps, ctypes.byref(r)))
         return r

@@ -2412,14 +2412,21 @@ extern "C" int gr_tune(gr_engine *e, int32_t trial_steps, gr_tune_result *out) {
         return USER_ERR("MinimumAliveParticles needs host decisions between steps; it cannot run in a graph. >");
     const int32_t steps = trial_steps > 0 ? trial_steps : 40;
     const gr_settings base = e->s;
+    int trials = 0;
+    // what the engine runs untuned, first: automatic choices that depend on the set (lanes a warp, ring slots
+    // or pairs, when to sort) are none of the explicit values below
+    double asis = 0.0, best = 0.0;
+    int rc = tune_trial(e, base, steps, asis);
+    ++trials;
+    const bool pairs = e->use_pair;
     gr_settings cur = base;
     if (cur.block_size <= 0) cur.block_size = 256;
     if (cur.sort_interval <= 0) cur.sort_interval = 4;
     if (cur.grid_waves <= 0) cur.grid_waves = 1;
-    int trials = 0;
-    double best = 0.0;
-    int rc = tune_trial(e, cur, steps, best);
-    ++trials;
+    if (!rc) {
+        rc = tune_trial(e, cur, steps, best);
+        ++trials;
+    }
     // coordinate descent: layout, block size, sort interval, grid waves
     auto consider = [&](gr_settings c) -> int {
         double r = 0.0;
@@ -2432,7 +2439,7 @@ extern "C" int gr_tune(gr_engine *e, int32_t trial_steps, gr_tune_result *out) {
         }
         return 0;
     };
-    if (!rc && e->wind_dynamic) {
+    if (!rc && e->wind_dynamic && (cur.layout == 1 || pairs)) {   // (ring slots either way otherwise)
         gr_settings c = cur;
         c.layout = cur.layout == 0 ? 1 : 0;
         rc = consider(c);
@@ -2455,6 +2462,16 @@ extern "C" int gr_tune(gr_engine *e, int32_t trial_steps, gr_tune_result *out) {
             c.grid_waves = gw;
             rc = consider(c);
         }
+    // the explicit values replace the settings only where they win twice, by more than trials differ
+    bool kept = best <= asis * 1.01;
+    if (!rc && !kept) {
+        double r = 0.0;
+        rc = tune_trial(e, base, steps, r);
+        asis = std::max(asis, r);
+        if (!rc) rc = tune_trial(e, cur, steps, r);
+        trials += 2;
+        kept = std::min(best, r) <= asis * 1.01;
+    }
     e->step_cap = 0;
     ++e->gen;
     e->have_result = false;
@@ -2462,14 +2479,15 @@ extern "C" int gr_tune(gr_engine *e, int32_t trial_steps, gr_tune_result *out) {
         e->s = base;
         return rc;
     }
-    e->s = cur;
+    e->s = kept ? base : cur;
     if (out) {
         out->layout = cur.layout;
         out->block_size = cur.block_size;
         out->sort_interval = cur.sort_interval;
         out->grid_waves = cur.grid_waves;
-        out->particle_steps_per_s = best;
+        out->particle_steps_per_s = kept ? asis : best;
         out->trials = trials;
+        out->kept = kept ? 1 : 0;
     }
     return GR_OK;
 }

@@ -124,7 +124,7 @@ class BatchIntegrator:
         self._batch = None
 
     def tune(self, trial_steps=40):
-        """Autotunes layout, block size, sort interval and grid waves (gr_tune)."""
+        """Autotunes layout, block size, sort interval and grid waves; keeps the settings where none is faster (gr_tune)."""
         return self.engine.tune(trial_steps)
 
     def compute(self):
