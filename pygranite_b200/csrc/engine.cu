@@ -701,7 +701,7 @@ int gr_set_topography(gr_engine *e, const float *data, int64_t ny, int64_t nx) {
     int rc = set_device(e);
     if (rc) return rc;
     CK(e->topo.alloc((size_t)nx * ny));
-    CK(cudaMemcpy(e->topo.p, data, (size_t)nx * ny * sizeof(float), cudaMemcpyHostToDevice));
+    CK(copy_in(e->topo.p, data, (size_t)nx * ny * sizeof(float)));
     e->has_topo = e->dim == 3;   // 2D variants never use the topography (Macros.hpp:71)
     return GR_OK;
 }
@@ -799,8 +799,8 @@ static int set_seeds(gr_engine *e, const float *pos, int64_t n, int32_t dim, boo
     if (rc) return rc;
     e->n = n;
     CK(e->seeds.alloc((size_t)n * dim));
-    CK(cudaMemcpy(e->seeds.p, pos, (size_t)n * dim * sizeof(float),
-                  device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
+    CK(copy_in(e->seeds.p, pos, (size_t)n * dim * sizeof(float),
+               device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
     if (!device_src) e->stats.h2d_bytes += n * dim * (int64_t)sizeof(float);
     return GR_OK;
 }
@@ -826,7 +826,7 @@ int gr_set_lifetimes(gr_engine *e, const int32_t *steps, int64_t n) {
     int rc = set_device(e);
     if (rc) return rc;
     CK(e->life_src.alloc((size_t)n));
-    CK(cudaMemcpy(e->life_src.p, steps, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice));
+    CK(copy_in(e->life_src.p, steps, (size_t)n * sizeof(int32_t)));
     e->stats.h2d_bytes += n * (int64_t)sizeof(int32_t);
     e->has_life = true;
     e->life_n = n;

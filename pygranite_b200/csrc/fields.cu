@@ -249,11 +249,11 @@ int gr_field_fourier(int32_t dim, const int64_t *shape, const double *spacing, i
     const size_t cm = (size_t)dim * n_modes;
     FK(f->k.alloc(cm * dim)); FK(f->amp.alloc(cm)); FK(f->phase.alloc(cm)); FK(f->om.alloc(cm));
     FK(f->scale.alloc((size_t)dim));
-    FK(cudaMemcpy(f->k.p, k, cm * dim * sizeof(double), cudaMemcpyHostToDevice));
-    FK(cudaMemcpy(f->amp.p, amp, cm * sizeof(double), cudaMemcpyHostToDevice));
-    FK(cudaMemcpy(f->phase.p, phase, cm * sizeof(double), cudaMemcpyHostToDevice));
-    FK(cudaMemcpy(f->om.p, omega, cm * sizeof(double), cudaMemcpyHostToDevice));
-    FK(cudaMemcpy(f->scale.p, scale, (size_t)dim * sizeof(double), cudaMemcpyHostToDevice));
+    FK(copy_in(f->k.p, k, cm * dim * sizeof(double)));
+    FK(copy_in(f->amp.p, amp, cm * sizeof(double)));
+    FK(copy_in(f->phase.p, phase, cm * sizeof(double)));
+    FK(copy_in(f->om.p, omega, cm * sizeof(double)));
+    FK(copy_in(f->scale.p, scale, (size_t)dim * sizeof(double)));
     // the per-axis factors of every mode (time-independent)
     FK(f->coef.alloc(cm));
     FK(f->fac_x.alloc(cm * (size_t)f->nx));

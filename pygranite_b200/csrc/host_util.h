@@ -28,6 +28,14 @@ size_t dev_pool_idle_bytes();
 cudaError_t stream_take(cudaStream_t *out);
 void stream_give(cudaStream_t st, int dev);
 
+// A copy to the device for kernels on the library's streams, which do not wait for the legacy stream: a
+// cudaMemcpy from pageable memory or on the device may return before the data is there (seeds of 100,000
+// particles were read by a graph launched right after it while their last part was still on the way).
+inline cudaError_t copy_in(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind = cudaMemcpyHostToDevice) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, kind);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 inline int grid_for(int64_t n, int threads) {
     int64_t b = (n + threads - 1) / threads;
     if (b < 1) b = 1;

@@ -924,7 +924,7 @@ int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t n
         hs[k] = E;
     }
     SK(S->d_sched.alloc(hs.size()));
-    SK(cudaMemcpy(S->d_sched.p, hs.data(), hs.size() * sizeof(StepEntry), cudaMemcpyHostToDevice));
+    SK(copy_in(S->d_sched.p, hs.data(), hs.size() * sizeof(StepEntry)));
     rc = allocate(S.get(), hbm_budget_bytes > 0 ? hbm_budget_bytes : quarter);
     if (rc) return rc;
     // pinned result staging: a quarter of the arena (at most 256 MB), never less than one full
@@ -953,7 +953,7 @@ int gr_server_set_snapshot(gr_server *S, int64_t snapshot, const float *const *c
         if (device_src) {
             src[c] = comps[c];
         } else {
-            SK(cudaMemcpy(S->raw.p + c * plane, comps[c], plane * sizeof(float), cudaMemcpyHostToDevice));
+            SK(copy_in(S->raw.p + c * plane, comps[c], plane * sizeof(float)));
             src[c] = S->raw.p + c * plane;
         }
     }
