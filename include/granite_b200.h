@@ -338,8 +338,10 @@ int gr_tune(gr_engine *engine, int32_t trial_steps, gr_tune_result *out);
  *
  * The field (n_snapshots snapshots of nz x ny x nx nodes, DataTimeDistance apart, stored as
  * settings->storage) is packed once by gr_server_set_snapshot: into device memory where the
- * whole field fits a quarter of what is free at creation, else into pinned host memory.  A
- * worker thread sweeps it window by window, the field in host memory through a 4-slot device ring.
+ * whole field and one window pair fit a quarter of what is free at creation (all pairs are kept where
+ * they fit as well), else into pinned host memory.  This memory comes on top of `hbm_budget_bytes`, which
+ * is for the particles; gr_server_create_limited sets a limit of its own for it.  A
+ * worker thread sweeps the field window by window, one in host memory through a 4-slot device ring.
  * A request is a seed set, a start time (seconds on the field's clock, rounded down to the
  * step grid DeltaT), a step count and an integrator (0 Euler, 1 RK4); it runs from its start step
  * until the step count, an abort, or the end of the field, whichever comes first.  Requests
@@ -379,6 +381,10 @@ typedef struct gr_server_stats {
 } gr_server_stats;
 int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t nz, int64_t ny, int64_t nx,
                      int64_t hbm_budget_bytes, gr_server **out);
+/* The same with a limit for the field on the device, in bytes: 0 = host memory behind the ring (4 slots and
+ * one pair on the device), negative = as gr_server_create.  For callers that share the GPU. */
+int gr_server_create_limited(const gr_settings *settings, int64_t n_snapshots, int64_t nz, int64_t ny, int64_t nx,
+                             int64_t hbm_budget_bytes, int64_t field_bytes, gr_server **out);
 /* Snapshot k as float32 planes (z, y, x) / (y, x); device_src = 1 for device pointers. */
 int gr_server_set_snapshot(gr_server *server, int64_t snapshot, const float *const *components,
                            int32_t n_components, int32_t device_src);

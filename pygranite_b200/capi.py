@@ -26,7 +26,7 @@ EXPORTS = [
     "gr_fetch_volume_info", "gr_fetch_compute_info", "gr_load_windfield_device",
     "gr_set_seeds_device", "gr_plan", "gr_advance_noalloc", "gr_update_settings", "gr_settings_get",
     "gr_set_lifetimes", "gr_batch_create", "gr_batch_destroy", "gr_batch_run", "gr_batch_stats_get", "gr_tune",
-    "gr_fetch_final_positions", "gr_server_create", "gr_server_set_snapshot", "gr_server_start",
+    "gr_fetch_final_positions", "gr_server_create", "gr_server_create_limited", "gr_server_set_snapshot", "gr_server_start",
     "gr_server_submit", "gr_server_wait", "gr_server_result", "gr_server_release", "gr_server_cancel",
     "gr_server_stats_get", "gr_server_destroy", "gr_field_double_gyre", "gr_field_fourier", "gr_field_load",
     "gr_field_loader", "gr_field_snapshot", "gr_field_destroy", "gr_host_alloc", "gr_host_free",
@@ -160,6 +160,8 @@ def lib():
             "gr_tune": (ctypes.c_int, [P, I32, ctypes.POINTER(TuneResult)]),
             "gr_fetch_final_positions": (ctypes.c_int, [P, FP, I64]),
             "gr_server_create": (ctypes.c_int, [ctypes.POINTER(Settings), I64, I64, I64, I64, I64, ctypes.POINTER(P)]),
+            "gr_server_create_limited": (ctypes.c_int, [ctypes.POINTER(Settings), I64, I64, I64, I64, I64, I64,
+                                                        ctypes.POINTER(P)]),
             "gr_server_set_snapshot": (ctypes.c_int, [P, I64, ctypes.POINTER(P), I32, I32]),
             "gr_server_start": (ctypes.c_int, [P]),
             "gr_server_submit": (ctypes.c_int, [P, FP, I64, I32, ctypes.c_double, I32, I32,
@@ -548,12 +550,18 @@ class Batch:
 class Server:
     """gr_server: trajectory requests served with continuous batching over one field."""
 
-    def __init__(self, settings: Settings, n_snapshots, shape, hbm_budget=0):
+    def __init__(self, settings: Settings, n_snapshots, shape, hbm_budget=0, field_budget=None):
+        """hbm_budget: bytes for the particles; field_budget: bytes for the field on the device (0: host memory;
+        None: a quarter of what is free, on top of hbm_budget)."""
         nz, ny, nx = shape if len(shape) == 3 else (1,) + tuple(shape)
         self.dim = 3 if settings.space == 0 else 2
         self.h = ctypes.c_void_p()
-        _check(lib().gr_server_create(ctypes.byref(settings), n_snapshots, nz, ny, nx, hbm_budget,
-                                      ctypes.byref(self.h)))
+        if field_budget is None:
+            _check(lib().gr_server_create(ctypes.byref(settings), n_snapshots, nz, ny, nx, hbm_budget,
+                                          ctypes.byref(self.h)))
+        else:
+            _check(lib().gr_server_create_limited(ctypes.byref(settings), n_snapshots, nz, ny, nx, hbm_budget,
+                                                  field_budget, ctypes.byref(self.h)))
 
     def set_snapshot(self, k, planes):
         """Host float32 planes (numpy)."""

@@ -3,7 +3,7 @@
 // No counterpart in the reference, which integrates one seed set per TrajectoryIntegrator.
 // Requests (a seed set, a start time, a step count, Euler or RK4) arrive at any time from
 // any thread.  One worker thread sweeps the field window by window.  A field that fits a quarter of
-// the free device memory stays there, packed, and so does every window's pair once it has been built;
+// the free device memory, or what the caller allows it (gr_server_create_limited), stays there, packed, and so does every window's pair once it has been built;
 // a larger one is kept in pinned host memory and a 4-slot device ring holds the snapshots of the
 // current window and the next ones, refilled on a copy stream while the current window integrates.
 // All requests share the field's global step clock (start times are rounded down to the step grid), so
@@ -11,7 +11,7 @@
 //
 //   per window, on the compute stream:
 //     admit   requests whose start step falls in the window, while their state fits the
-//             HBM budget: seeds -> the tail of the integrator's particle pool;
+//             budget for particles: seeds -> the tail of the integrator's particle pool;
 //     pack    the window-pair buffer from the two slots (planar, unpadded: 25% less upload
 //             than padded 3D nodes), unless it is there already;
 //     advance one persistent grid-stride launch per pool over the window's steps (a
@@ -357,8 +357,7 @@ int setup(gr_server *S, int64_t nz, int64_t ny, int64_t nx, int64_t field_budget
         S->wide ? 0 : ((padded_pair_nodes(S->dim, S->nx, S->ny, S->nz) * (S->dim == 3 ? 8 : 4) * S->elem + 255) / 256) * 256;
     // the whole field on the device where it fits the budget, with all its pairs if they fit too
     const int64_t field = S->slot_stride * S->n_snap;
-    const char *env = std::getenv("GR_SERVE_RESIDENT");   // 0: host memory whatever fits
-    S->resident = !(env && env[0] == '0') && field + pair_bytes <= field_budget;
+    S->resident = field + pair_bytes <= field_budget;
     if (S->resident && field + pair_bytes * (S->n_snap - 1) <= field_budget) S->pair_stride = pair_bytes;
     if (S->resident && (S->ring.alloc((size_t)field) != cudaSuccess ||
                         S->pair.alloc((size_t)(S->pair_stride > 0 ? S->pair_stride * (S->n_snap - 1) : pair_bytes)) !=
@@ -865,6 +864,12 @@ extern "C" {
 
 int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t nz, int64_t ny, int64_t nx,
                      int64_t hbm_budget_bytes, gr_server **out) {
+    const char *env = std::getenv("GR_SERVE_RESIDENT");   // 0: host memory whatever fits
+    return gr_server_create_limited(settings, n_snapshots, nz, ny, nx, hbm_budget_bytes, env && env[0] == '0' ? 0 : -1, out);
+}
+
+int gr_server_create_limited(const gr_settings *settings, int64_t n_snapshots, int64_t nz, int64_t ny, int64_t nx,
+                             int64_t hbm_budget_bytes, int64_t field_bytes, gr_server **out) {
     if (!settings || !out) return SUSER("null argument");
     *out = nullptr;
     const gr_settings &s = *settings;
@@ -896,7 +901,7 @@ int gr_server_create(const gr_settings *settings, int64_t n_snapshots, int64_t n
     size_t fr = 0, tot = 0;
     SK(cudaMemGetInfo(&fr, &tot));
     const int64_t quarter = (int64_t)((fr + dev_pool_idle_bytes()) / 4);   // the pool's idle memory is ours to use
-    int rc = setup(S.get(), S->dim == 3 ? nz : 1, ny, nx, quarter);
+    int rc = setup(S.get(), S->dim == 3 ? nz : 1, ny, nx, field_bytes < 0 ? quarter : field_bytes);
     if (rc) return rc;
     // the field's global step clock: the reference's float32 schedule over all windows
     ScheduleInput si;

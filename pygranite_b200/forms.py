@@ -152,13 +152,15 @@ class BatchIntegrator:
 
 class TrajectoryServer:
     """Trajectory requests served with continuous batching over the loader's whole field (every
-    snapshot it delivers, kept packed in pinned host memory and streamed through a 4-slot device
-    ring).  Positions only: no curvature, volumes, constants, uplift or length abort."""
+    snapshot it delivers, packed: in device memory where it fits `field_budget` bytes, a quarter of
+    what is free if None, else in pinned host memory behind a 4-slot device ring).  `hbm_budget` bytes
+    hold the particles.  Positions only: no curvature, volumes, constants, uplift or length abort."""
 
-    def __init__(self, settings, loader, hbm_budget=0, max_snapshots=None):
+    def __init__(self, settings, loader, hbm_budget=0, max_snapshots=None, field_budget=None):
         self.settings = settings
         wind, _ = _pull_snapshots(loader, max_snapshots or (1 << 62))
-        self.server = capi.Server(c_settings(settings), len(wind), np.shape(wind[0][0]), hbm_budget=hbm_budget)
+        self.server = capi.Server(c_settings(settings), len(wind), np.shape(wind[0][0]), hbm_budget=hbm_budget,
+                                  field_budget=field_budget)
         for k, w in enumerate(wind):
             self.server.set_snapshot(k, w)
         self.server.start()
