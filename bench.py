@@ -64,6 +64,7 @@ def parse():
     p.add_argument("--ref-steps", type=int, default=20, help="reference arm: steps of the workload's prefix")
     p.add_argument("--parity-sample", type=int, default=2000,
                    help="particles of the timed run checked against the float32 / float64 oracle (0 = off)")
+    p.add_argument("--detail", default="", help="plain workload: file for the whole record (repetitions, accuracy, forms)")
     p.add_argument("--no-forms", action="store_true", help="plain workload: skip the batch / serve / precision forms")
     p.add_argument("--workload", default="plain", choices=["plain", "batch", "serve", "precision"],
                    help="plain: the 3D RK4 configuration; batch: 512 seed sets of uneven size and lifetime; "
@@ -798,6 +799,7 @@ def run_serve(args, world, rank, local, pg_dist):
         pg_dist.barrier()
     if rank != 0:
         return None
+    streamed = s1.h2d_bytes - s0.h2d_bytes > 2 * 24 * nparts   # more than seeds and their 12 bytes a particle
     lat, queue = np.array(lat), np.array(queue)
     pct = lambda a, q: float(np.percentile(a, q)) if a.size else None  # noqa: E731
     accuracy = serve_accuracy(w, acc_out, host_snaps, args.serve_storage) if acc_out else None
@@ -806,7 +808,8 @@ def run_serve(args, world, rank, local, pg_dist):
         "steps": 1, "warmup": 3, "ms_per_step": t_max, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": args.serve_storage,
         "data": "synthetic (seeded Fourier-mode field, Poisson request stream)",
-        "config": {"workload": SERVE_WORKLOAD, "grid": [nx, ny, nz], "snapshots": w.n_snapshots, "ring_slots": 4,
+        "config": {"workload": SERVE_WORKLOAD, "grid": [nx, ny, nz], "snapshots": w.n_snapshots,
+                   "field": "host memory, 4-slot ring" if streamed else "device memory",
                    "rate_per_s": args.serve_rate, "arrival_seconds": args.serve_seconds,
                    "requests": len(ids), "completed": int(lat.size), "particles": int(nparts),
                    "storage": args.serve_storage, "parallelism": f"replicas{world}",
@@ -968,6 +971,58 @@ def run_forms(args, world, rank, local):
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
     return forms
+
+
+LINE_LIMIT = 2400
+
+
+def headline(line, limit=LINE_LIMIT):
+    """The plain workload's record as the one line that is printed: every figure of it that stands for a phase, without
+    repetitions, per-sample accuracy and the other workloads' own records (--detail writes those to a file).  Readers
+    keep the last few thousand characters of the output, so a longer line is not a line to them."""
+    def short(x):
+        if isinstance(x, dict):
+            return {k: short(v) for k, v in x.items()}
+        if isinstance(x, (list, tuple)):
+            return [short(v) for v in x]
+        return float(f"{x:.6g}") if isinstance(x, float) else x
+
+    def pick(d, *keys):
+        return {k: short(d[k]) for k in keys if k in d} if isinstance(d, dict) else d
+
+    out = {k: v for k, v in line.items() if k not in ("parity", "e2e", "native_loader", "roofline", "cpu_baseline", "forms")}
+    e2e = line.get("e2e")
+    if e2e:
+        out["e2e"] = dict(pick(e2e, "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "steps", "ms_per_step"),
+                          value=e2e["value"])
+        if e2e.get("parity"):
+            out["e2e"]["f32_bitexact"] = e2e["parity"]["f32_bitexact"]
+        if e2e.get("pageable"):
+            out["e2e"]["pageable"] = pick(e2e["pageable"], "value", "ms_per_step")
+    else:
+        out["e2e"] = e2e
+    if line.get("parity"):
+        out["parity"] = pick(line["parity"], "f32_bitexact", "sample", "records", "mismatched_particles")
+        last = list(line["parity"].get("f64", {}).items())[:1]
+        out["parity"].update({f"cell_rms_{k}": short(v["cell_rms"]) for k, v in last})
+    out["native_loader"] = pick(line.get("native_loader"), "value", "run_ms")
+    out["roofline"] = pick(line.get("roofline"), "bound", "achieved", "peak", "unit", "frac", "traffic", "peak_source",
+                           "bytes_per_particle_step", "kernel", "avg_launch_ms", "particle_steps_per_launch", "dram_gbs",
+                           "issue_frac", "active_bound")
+    out["cpu_baseline"] = pick(line.get("cpu_baseline"), "value", "unit", "cores", "kind", "sample")
+    if line.get("forms"):
+        out["forms"] = {name: pick(f, "value", "error", "phase_s") for name, f in line["forms"].items()}
+    # over the limit the least needed goes first
+    for key, sub in (("forms", None), ("native_loader", None), ("wall_s", None), ("run", None), ("parity", None),
+                     ("e2e", "pageable"), ("roofline", "active_bound"), ("roofline", "dram_gbs"), ("roofline", "issue_frac"),
+                     ("roofline", "particle_steps_per_launch"), ("cpu_baseline", "sample")):
+        if len(json.dumps(out)) <= limit:
+            break
+        if sub is None:
+            out.pop(key, None)
+        elif isinstance(out.get(key), dict):
+            out[key].pop(sub, None)
+    return out
 
 
 def main():
@@ -1237,7 +1292,10 @@ def main():
         "parity": parity, "e2e": e2e, "native_loader": native, "roofline": roofline, "cpu_baseline": cpu,
         "clocks": clocks, "gpu_launches": int(launches + aux), "wall_s": wall, "forms": forms,
     }
-    print(json.dumps(line), flush=True)
+    if args.detail:
+        with open(args.detail, "w") as f:
+            json.dump(line, f)
+    print(json.dumps(headline(line)), flush=True)
     if pg_dist:
         pg_dist.destroy_process_group()
     return 0
