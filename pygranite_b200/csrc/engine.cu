@@ -1053,7 +1053,7 @@ size_t pair_bytes(const gr_engine *e) {
 // 0.63, 400,000 1.16 / 1.08; 256 x 128, 10,000 x 1024 Euler steps, 128 a window, 0.58 / 0.42.  Where the
 // settings place the launches, only the pack is saved; in a graph a launch costs little, all the less
 // beside another engine's (the batch of 48 sets: 3.40 ms a replay with pairs, 3.63 without).
-// RK4 in 3D with volumes or expressions that pairs would defer: the ring variant that evaluates them runs
+// RK4 in 3D with volumes or expressions that pairs would defer (pairs, so not where the layout is given): the ring variant that evaluates them runs
 // at 128 registers and spills, so a record costs it 3 us and 11.5 ns a warp, a step 0.5 us and 0.34 ns a
 // warp (their slope follows the warps, of 16 lanes or 32 alike), against 13.5 us for a window's launch, 6.5 us
 // for a record's kernel and 0.8 of the pack.  Measured where more than one record a window already pays
@@ -1071,7 +1071,7 @@ bool small_set(gr_engine *e, const RunPlan &R) {
     const double chain = e->dim == 3 ? 0.5 : 0.18, gathers = extras ? 25.0 : e->dim == 3 ? 8.6 : 3.0;
     if (steps * (chain + gathers * 1e-6 * (double)e->n) >= launch + 0.5 * pack) return false;
     const double records = (double)(R.rec_before[R.nsteps] - 1) / (double)R.nwin;   // a window
-    if (e->dim == 3 && s.integrator == 1 && records <= 1.0 && !R.graph &&
+    if (e->dim == 3 && s.integrator == 1 && s.layout == 0 && records <= 1.0 && !R.graph &&
         (kernel_features(make_params(e), true) & FT_DEFER) != 0) {
         const int lanes = block_of_few(e->n);
         const double warps = (double)e->n / (lanes > 0 ? lanes : 32);
