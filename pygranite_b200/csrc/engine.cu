@@ -1053,14 +1053,14 @@ size_t pair_bytes(const gr_engine *e) {
 // 0.63, 400,000 1.16 / 1.08; 256 x 128, 10,000 x 1024 Euler steps, 128 a window, 0.58 / 0.42.  Where the
 // settings place the launches, only the pack is saved; in a graph a launch costs little, all the less
 // beside another engine's (the batch of 48 sets: 3.40 ms a replay with pairs, 3.63 without).
-// RK4 in 3D with volumes or expressions that pairs would defer (pairs, so not where the layout is given): the ring variant that evaluates them runs
-// at 128 registers and spills, so a record costs it 3 us and 11.5 ns a warp, a step 0.5 us and 0.34 ns a
-// warp (their slope follows the warps, of 16 lanes or 32 alike), against 13.5 us for a window's launch, 6.5 us
-// for a record's kernel and 0.8 of the pack.  Measured where more than one record a window already pays
-// for the launches: none was slower on the ring slots.  150 steps, a record a window, ring / pair: 24 x 24
-// x 16 nodes 6,000 0.43 / 0.48, 20,000 0.60 / 0.53, 25,000 0.51 / 0.52, 40,000 0.65 / 0.56; 80 x 80 x 40 25,000
-// 0.59 / 0.57, 40,000 0.74 / 0.62; 130 x 130 x 48 32,000 0.67 / 0.70, 60,000 0.89 / 0.79; 192 x 192 x 64 72,000
-// 1.05 / 1.17, 80,000 1.39 / 1.19.
+// RK4 in 3D with volumes or expressions that pairs would defer (pairs, so not where the layout is
+// given): the ring variant that evaluates them runs at 128 registers and spills, so a record costs it 3 us
+// and 11.5 ns a warp, a step 0.5 us and 0.34 ns a warp (their slope follows the warps, of 16 lanes or 32
+// alike), against 13.5 us for a window's launch, 6.5 us for a record's kernel and 0.8 of the pack.  More
+// than one record a window pays for the launches already: none measured was slower on the ring slots.
+// 150 steps, a record a window, ring / pair: 24 x 24 x 16 nodes 6,000 0.43 / 0.48, 20,000 0.60 / 0.53, 25,000
+// 0.51 / 0.52, 40,000 0.65 / 0.56; 80 x 80 x 40 25,000 0.59 / 0.57, 40,000 0.74 / 0.62; 130 x 130 x 48 32,000
+// 0.67 / 0.70, 60,000 0.89 / 0.79; 192 x 192 x 64 72,000 1.05 / 1.17, 80,000 1.39 / 1.19.
 bool small_set(gr_engine *e, const RunPlan &R) {
     if (R.nsteps == 0 || !e->wind_dynamic) return false;
     const gr_settings &s = e->s;

@@ -1200,8 +1200,13 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
                 dirty = false;
                 // refill the sample cache for the next step's first sample (at p): the cached
                 // nodes are then dead while the values above are evaluated, which frees their
-                // registers there
-                if constexpr (DIM == 3) {
+                // registers there.  RK4 steps on ring slots drop the cell instead: a second copy of the 16
+                // loads in the loop costs them more (a record every 5 steps, 50,000 particles x 143 steps,
+                // refilled / dropped: a volume and an expression 0.97 / 0.86 ms, every option 1.05 / 0.99;
+                // Euler steps, records every 20 and 30: every option 0.33 / 0.36, a volume 0.40 / 0.46).
+                if constexpr (DIM == 3 && RK4 && !IsPair<W>::value) {
+                    cc.reset();
+                } else if constexpr (DIM == 3) {
                     float2 f;
                     float fz;
                     const float2 axy = grid_xy(P, p.xy);
@@ -1211,8 +1216,7 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
                         cc.base = padded_index<3>(P, c);
                         fill<3, W>(P, wb, wf, c, cc);
                     } else {
-                        constexpr bool options = !(FT & FT_LEAN) || (FT & FT_BORDER);
-                        load_cell<3, W>(P, axy, az, options && P.wide, wb, wf, f, fz, cc);
+                        load_cell<3, W>(P, axy, az, !LEAN && P.wide, wb, wf, f, fz, cc);
                     }
                 }
             }
