@@ -171,6 +171,8 @@ int gr_batch_run(gr_batch *b) {
         const int rc = capture(b);
         if (rc) return rc;
     }
+    for (gr_engine *e : b->engines)
+        if (cudaEvent_t ev = engine_inputs(e)) BK(cudaStreamWaitEvent(b->stream, ev, 0));
     BK(cudaEventRecord(b->t0, b->stream));
     BK(cudaGraphLaunch(b->exec, b->stream));
     BK(cudaEventRecord(b->t1, b->stream));

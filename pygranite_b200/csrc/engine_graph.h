@@ -18,6 +18,9 @@ int graph_enqueue(gr_engine *e);
 // After the enqueued run finished: counters and result sizes.
 int graph_collect(gr_engine *e);
 cudaStream_t engine_stream(gr_engine *e);
+// Event after the last copy of seeds, lifetimes or topography (null: none): what replays the run on another
+// stream waits for it.
+cudaEvent_t engine_inputs(const gr_engine *e);
 int engine_device(const gr_engine *e);
 uint64_t engine_generation(const gr_engine *e);
 int64_t engine_launches(const gr_engine *e, int64_t *aux);
