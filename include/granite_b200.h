@@ -69,14 +69,17 @@ typedef struct gr_settings {
                                       keeps; 1: from a float64 accumulator */
     int32_t compensated;           /* 1: Kahan-compensated float32 position update */
     int32_t ring_slots;            /* device ring depth (>= 3); 0 = 3 */
-    int32_t steps_per_launch;      /* steps fused into one launch; 0 = one snapshot window */
+    int32_t steps_per_launch;      /* steps fused into one launch; 0 = automatic: a snapshot window; on ring
+                                      slots all resident windows up to the next compaction; at most up to a
+                                      record where volume / expression values are deferred */
     int32_t sort_interval;         /* launches between Morton re-sorts / compactions; 0 = off; negative
                                     * (the default): automatic from 65,536 particles, else off: the seeds
                                     * before the first step, then every 8 windows (16 below 400,000
-                                    * particles without lifetimes) */
-    int32_t block_size;            /* threads per block; 0 = autotuned default; capped at the step
-                                      kernel's launch bound (128 for the float32 3D window-pair
-                                      kernel, 256 for the others) */
+                                    * particles without lifetimes; with a length abort below 80,000) */
+    int32_t block_size;            /* threads per block; 0 = automatic: 64, fewer for few particles; capped
+                                      at the step kernel's launch bound (128 for the float32 3D kernels and
+                                      the 16-bit 3D ones with total curvature or deferred values, 256 for the
+                                      others) */
     int32_t device;                /* CUDA device ordinal */
     int32_t layout;                /* wind layout read by the step kernel: 0 = automatic: window pairs
                                       when the windfield is dynamic (one load returns the back and
@@ -445,12 +448,12 @@ void gr_field_destroy(gr_field *field);
  * border modes, sphere coordinates, ReferenceFilter; no curvature, volumes, constants, uplift,
  * topography, length abort, MinimumAliveParticles, constant wind, 16-bit storage, Kahan
  * positions or float64 time weights (GR_ERR_USER otherwise).
- * Its scratch (the per-step time weights and two counters, GR_NOALLOC_SCRATCH_BYTES) is one
+ * Its scratch (the per-step time weights and a counter, GR_NOALLOC_SCRATCH_BYTES) is one
  * file-scope device array that every GPU loading the library holds until the process exits;
  * steps beyond GR_NOALLOC_MAX_STEPS are rejected.  The first call on a device looks up that
  * array's device address (cudaGetSymbolAddress) and keeps it for the life of the process, so
  * make that first call before any stream capture; a cudaDeviceReset between calls is not
- * supported.  Each call rebuilds the weights and clears the counters on `stream` before its
+ * supported.  Each call rebuilds the weights and clears the counter on `stream` before its
  * step kernel.  All calls share the array: calls whose work overlaps on the GPU (different
  * streams, no ordering between them) race. */
 #define GR_NOALLOC_MAX_STEPS 4096

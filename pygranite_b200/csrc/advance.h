@@ -54,7 +54,7 @@ inline void derive_params(KParams &P, float h) {
     P.inv2 = make_float2(P.inv_scale[0], P.inv_scale[1]);
 }
 
-// Grids that the fast cell arithmetic does not cover (pcell1 needs coordinates below 2^22).
+// Grids that the fast cell arithmetic does not cover (make_pcell needs coordinates below 2^22).
 inline bool wide_grid(int64_t nx, int64_t ny, int64_t nz) {
     return nx >= (1 << 22) - 2 || ny >= (1 << 22) - 2 || nz >= (1 << 22) - 2;
 }

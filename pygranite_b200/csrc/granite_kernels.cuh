@@ -44,9 +44,10 @@ constexpr int GR_MAX_EXPR = 4;
 constexpr int GR_MAX_CON = 4;
 
 // Compile-time feature sets of the step kernel.  FT_GENERIC honours every runtime option.  A
-// lean variant (FT_LEAN) is picked by the host (kernel_features in advance.h) when the launch has
-// no uplift, length abort, topography, sphere coordinates, loop borders, per-step alive counts
-// or 1/256 filter weights, and curvature Off or Total; FT_CURV / FT_EXTRAS say whether it keeps total curvature and volume
+// lean variant (FT_LEAN) is picked by the host (kernel_features in advance.h) when the launch has a
+// dynamic windfield, no uplift, length abort, topography or per-step alive counts, and curvature
+// Off or Total; without FT_BORDER also no sphere coordinates, loop borders, 1/256 filter weights or wide
+// grid.  FT_CURV / FT_EXTRAS say whether it keeps total curvature and volume
 // / expression values, FT_COMP Kahan-compensated positions (instantiated without extras: the
 // precision form).  FT_DEFER (with FT_LEAN, instead of FT_EXTRAS) leaves the volume / expression
 // values to deferred_extras_kernel after the launch: the step kernel only stores each moved step's
@@ -75,7 +76,7 @@ struct KParams {
     int32_t nx, ny, nz, dim;
     float fn[3], flo;             // clamp of a sample's grid coordinates: [flo, fn] (clamp_cells)
     int32_t below;                // cells -below .. n + below - 1 are read as they are
-    int32_t wide;                 // 1: a grid too large for pcell1 or the cell index (ring layouts only)
+    int32_t wide;                 // 1: a grid too large for make_pcell or the cell index (ring layouts only)
     // operand pairs of the paired instructions and -off: world position -> grid is
     // (p + noff) * inv_scale
     float2 noff2, inv2, h2, hh2, sixth2, i2h2, ihh2;
@@ -197,7 +198,7 @@ template <> struct Store<float> {
 // at once and (w_b, w_f) likewise, and the horizontal wind leaves the sample as a pair, so the time
 // interpolation, the stage positions, the coordinates and the curvature differences are paired
 // operations on (x, y) too.  Built per window from the ring (pack_kernels.cuh), with a border
-// (make_pcell, bil2p_padded).
+// (clamped_cell, fill_padded, fill_edge2).
 template <typename W> struct Pair {};
 
 template <typename W> struct IsPair { static constexpr bool value = false; };
@@ -578,7 +579,7 @@ __device__ __forceinline__ PCell clamped_cell(const KParams &P, float2 axy, floa
 // first against differences first: 1e6 particles x 300 steps 7.03 / 7.16 ms of step launches, 300,000 x 200
 // 2.30 / 2.33, 10,000 x 1024 Euler steps in 2D 0.46 / 0.47, 10,000 x 1024 RK4 steps in 2D 0.80 / 0.75, 2D
 // sphere 150,000 x 200 0.75 / 0.72, bf16 ring slots 777,777 x 100 2.66 / 2.61 ms.
-// FT: the step kernel's feature set; lean variants run with filter_weights off (kernel_features).
+// FT: the step kernel's feature set; lean variants but FT_BORDER run with filter_weights off (kernel_features).
 template <int DIM, bool RK4, typename W, int FT>
 __device__ __forceinline__ V3 wind_at(const KParams &P, const V3 &p, float t, const void *wb, const void *wf,
                                       SampleCache &cc) {
@@ -1253,8 +1254,10 @@ __device__ __forceinline__ void advance_particle(const KParams &P, const int32_t
 // Launch bounds: 256 threads, 2 blocks per SM (128 registers).  The float32 3D kernels keep 48
 // cached floats in 128-thread blocks: 4 per SM (128 registers) in the generic variant and the lean
 // ones with volume / expression values or with both Kahan positions and curvature, 5 per SM (96
-// registers, 20 warps) in the other lean ones on window pairs, whose state fits there without spills;
-// the extra warps hide more of the sampling and curvature latency.  Ring slots stay at 4 blocks: with 16
+// registers, 20 warps) in the other lean ones on window pairs, whose state fits there, but for 24 bytes of
+// spill stores and 12 of loads in the RK4 variants with total curvature (0.65e6 of the 142e6 warp
+// instructions of a 10-step launch of 1e6 particles); the extra warps hide more of the sampling and
+// curvature latency.  Ring slots stay at 4 blocks: with 16
 // loads in flight 96 registers spill in the step loop (gr_advance_noalloc, 500,001 particles x 20
 // steps, 0.49 ms against 0.44).  16-bit 3D kernels: 128 x 5 for the lean variants
 // with curvature or deferred values (measured 5-6% faster than 256 x 2 on the 3D benchmark

@@ -5,7 +5,7 @@
 // real-time loops that forbid allocation after start-up (an allocation may synchronise the
 // device or take an unbounded time).  This entry point gives them the plain integrator (Euler
 // or RK4 between two snapshots, the border checks and abort codes) on buffers they own.  Its
-// only scratch, the per-step time weights and two counters, is the file-scope array below:
+// only scratch, the per-step time weights and a counter, is the file-scope array below:
 // every GPU that loads the library keeps these GR_NOALLOC_SCRATCH_BYTES until the process
 // exits, and every call shares them.
 #include <cuda_runtime.h>
@@ -28,7 +28,7 @@ namespace {
 
 struct NoAllocScratch {
     StepEntry sched[GR_NOALLOC_MAX_STEPS];
-    unsigned long long counters[2];   // [0] particle-steps, [1] alive after the call
+    unsigned long long counters[2];   // [0] particle-steps, [1] unused (GR_NOALLOC_SCRATCH_BYTES counts it)
 };
 
 static_assert(sizeof(NoAllocScratch) == GR_NOALLOC_SCRATCH_BYTES, "scratch size stated in granite_b200.h");
@@ -56,8 +56,7 @@ __global__ void __launch_bounds__(256) noalloc_schedule_kernel(NoAllocScratch *S
             S->sched[k].t0 = T;
             T = T + h;
         }
-        S->counters[0] = 0ull;   // the counters keep the previous call's values: clear them
-        S->counters[1] = 0ull;
+        S->counters[0] = 0ull;   // it keeps the previous call's value: clear it
     }
     __syncthreads();
     for (int k = threadIdx.x; k < steps; k += blockDim.x) {
@@ -110,7 +109,7 @@ extern "C" int gr_advance_noalloc(const gr_settings *s, int64_t nz, int64_t ny, 
     NoAllocScratch *S = g_scratch_ptr[s->device];
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    // the step schedule and cleared counters, built on the device in stream order
+    // the step schedule and the cleared counter, built on the device in stream order
     noalloc_schedule_kernel<<<1, 256, 0, st>>>(S, time_back, time_front, time_start, s->delta_t, steps);
     if (cudaGetLastError() != cudaSuccess) return err(GR_ERR_RUNTIME, "ERROR < RUNTIME | schedule launch failed >");
     const float h = s->delta_t;
