@@ -2,6 +2,7 @@
 with one pair, the field with all pairs.  Results are the float32 oracle's in each, and the device memory held stays
 within the limit and what a server with limit 0 holds."""
 import ctypes
+import gc
 
 import numpy as np
 import pytest
@@ -42,6 +43,7 @@ def problem():
 def serve(problem, limit):
     """Device bytes of the server, bytes copied to the device by two rounds of requests."""
     base, wind, reqs = problem
+    gc.collect()          # what earlier tests left is not to be given back in between
     before = used()
     srv = capi.Server(capi.settings_from_reference(base), SNAPSHOTS, SHAPE, hbm_budget=4 << 20, field_budget=limit)
     held = used() - before

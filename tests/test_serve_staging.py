@@ -1,6 +1,7 @@
 """Admission staging of the request server (GPU): as large as the requests at hand, from the library's host cache, and grown
 by larger ones; results stay those of the float32 oracle."""
 import ctypes
+import gc
 
 import numpy as np
 import pytest
@@ -28,6 +29,7 @@ def test_staging_grows_with_the_requests(dim):
     for k, s in enumerate(wind):
         srv.set_snapshot(k, s)
     srv.start()
+    gc.collect()          # what earlier tests left is not to be given back in between
     live, made, held = cache().live_bytes, cache().allocations + cache().reuses, []
     for n in (1, 87_382, 104_857, 104_858, 350_000, 7):     # around 2 MB and 8 MB blocks
         seeds = rng.uniform(0, shape[::-1], (n, dim)).astype(np.float32)
